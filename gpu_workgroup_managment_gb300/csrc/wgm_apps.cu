@@ -72,8 +72,8 @@ static bool wgm_needs_weights(int kind) {
   return kind == WGM_APP_LONESTAR_SSSP || kind == WGM_APP_PANNOTIA_SSSP;
 }
 static bool wgm_uses_static_hubs(int kind) {
-  return kind == WGM_APP_PANNOTIA_COLOR || kind == WGM_APP_PANNOTIA_MIS ||
-         kind == WGM_APP_PANNOTIA_SSSP || kind == WGM_APP_PAGERANK;
+  return kind == WGM_APP_PANNOTIA_COLOR || kind == WGM_APP_PANNOTIA_SSSP ||
+         kind == WGM_APP_PAGERANK;
 }
 
 /* Reject graphs the kernels cannot walk safely.  The Lonestar loader quirk
@@ -141,8 +141,8 @@ static void wgm_build_hubs(const wgm_graph_desc *g, int T, std::vector<int> &ids
 static void wgm_app_free_buffers(wgm_app *a) {
   void *ptrs[] = {a->d_row,     a->d_col,       a->d_wt,      a->d_node_value, a->d_out,
                   a->d_wl_start, a->d_wl_cnt,   a->d_wl_u,
-                  a->d_cnt,       a->d_stamp,   a->d_stop,       a->d_hub_acc,
-                  a->d_status,  a->d_contrib,   a->d_dang,    a->d_hub_sum,    a->d_rounds,
+                  a->d_cnt,       a->d_stamp,   a->d_stop,
+                  a->d_mis_word, a->d_mis_mask, a->d_mis_wide, a->d_contrib,   a->d_dang,    a->d_hub_sum,    a->d_rounds,
                   a->hubs.ids,  a->hubs.prefix, a->hubs.wmap, a->d_trow, a->d_tcol,
                   a->d_oct_input, a->d_oct_second, a->d_oct_pools, a->d_oct_tree,
                   a->d_oct_ctr, a->d_oct_locks, a->d_oct_heads,
@@ -152,6 +152,15 @@ static void wgm_app_free_buffers(wgm_app *a) {
   for (void *p : ptrs)
     if (p) cudaFree(p);
   a->hubs = wgm_dev_hubs();
+}
+
+/* Independent set: the edges of one vertex that a single warp looks at, and
+ * room for every vertex that has more (wgm_phase_mis). */
+static int wgm_mis_scan_edges(const wgm_app *a) {
+  return (int)std::min<int64_t>(2LL * a->hub_threshold, INT32_MAX / 2);
+}
+static size_t wgm_mis_wide_cap(const wgm_app *a) {
+  return (size_t)(a->E / wgm_mis_scan_edges(a)) + 1;
 }
 
 template <class T>
@@ -185,16 +194,10 @@ static int wgm_upload_hubs(wgm_app *a, const wgm_graph_desc *g) {
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   a->hubs.H = (int)ids.size();
   a->hubs.total = prefix.back();
-  if (a->kind == WGM_APP_PANNOTIA_COLOR || a->kind == WGM_APP_PANNOTIA_MIS ||
-      a->kind == WGM_APP_PAGERANK) {
-    if (a->d_hub_acc) cudaFree(a->d_hub_acc);
+  if (a->kind == WGM_APP_PAGERANK) {
     if (a->d_hub_sum) cudaFree(a->d_hub_sum);
-    a->d_hub_acc = nullptr;
     a->d_hub_sum = nullptr;
-    if (a->kind == WGM_APP_PAGERANK)
-      e = wgm_dmalloc(&a->d_hub_sum, (size_t)a->hubs.H);
-    else
-      e = wgm_dmalloc(&a->d_hub_acc, (size_t)a->hubs.H * 2);
+    e = wgm_dmalloc(&a->d_hub_sum, (size_t)a->hubs.H);
     if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   }
   return WGM_OK;
@@ -313,7 +316,8 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
       a->out_bytes = V * 4;
       if (e == cudaSuccess) e = cudaMalloc(&a->d_out, a->out_bytes);
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_node_value, V);
-      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_stop, 3 * WGM_LINE);
+      if (e == cudaSuccess && kind == WGM_APP_PANNOTIA_MIS)
+        e = wgm_dmalloc(&a->d_stop, 3 * WGM_LINE);
       if (e == cudaSuccess && kind == WGM_APP_PANNOTIA_COLOR) {
         /* frontier pieces of in-edges; every vertex is coloured once, so a
          * round never holds more than V + E/piece pieces */
@@ -327,7 +331,12 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
         if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cnt, 3 * WGM_LINE);
         if (e == cudaSuccess) e = wgm_dmalloc(&a->d_tcv, E); /* in-edges with values */
       }
-      if (e == cudaSuccess && kind == WGM_APP_PANNOTIA_MIS) e = wgm_dmalloc(&a->d_status, V);
+      if (kind == WGM_APP_PANNOTIA_MIS) {
+        if (e == cudaSuccess) e = wgm_dmalloc(&a->d_mis_word, V);
+        if (e == cudaSuccess) e = wgm_dmalloc(&a->d_stamp, V); /* resume edges */
+        if (e == cudaSuccess) e = wgm_dmalloc(&a->d_mis_mask, (V + 31) / 32);
+        if (e == cudaSuccess) e = wgm_dmalloc(&a->d_mis_wide, wgm_mis_wide_cap(a));
+      }
       break;
     case WGM_APP_PANNOTIA_SSSP:
       a->out_bytes = V * 4;
@@ -584,8 +593,6 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.col = a->d_col;
       x.node_value = a->d_node_value;
       x.color = (int *)a->d_out;
-      x.stop = a->d_stop;
-      x.hub_acc = a->d_hub_acc;
       x.hubs = wgm_hubs_view(a);
       x.hub_threshold = a->hub_threshold;
       x.rounds_out = a->d_rounds;
@@ -608,11 +615,13 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.col = a->d_col;
       x.node_value = a->d_node_value;
       x.s_array = (int *)a->d_out;
-      x.status = a->d_status;
+      x.word = a->d_mis_word;
+      x.ptr = a->d_stamp;
+      x.mask = a->d_mis_mask;
       x.stop = a->d_stop;
-      x.hub_acc = a->d_hub_acc;
-      x.hubs = wgm_hubs_view(a);
-      x.hub_threshold = a->hub_threshold;
+      x.wide = a->d_mis_wide;
+      x.wide_cap = (int)wgm_mis_wide_cap(a);
+      x.scan = wgm_mis_scan_edges(a);
       x.rounds_out = a->d_rounds;
       return WGM_OK;
     }
@@ -761,6 +770,13 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
       (a->kind == WGM_APP_LONESTAR_BFS || a->kind == WGM_APP_LONESTAR_SSSP)) {
     const long long sms = a->rt->prop.multiProcessorCount;
     const long long want = ((long long)a->E / 8192 + sms - 1) / sms * sms;
+    *grid = (int)std::min<long long>(hw, std::max(sms, want));
+  }
+  /* Independent set by default: a thread per vertex, in whole CTAs per SM.
+   * More only lengthen the barrier that every round ends with. */
+  if (num_wgs <= 0 && a->kind == WGM_APP_PANNOTIA_MIS) {
+    const long long sms = a->rt->prop.multiProcessorCount, b = std::max(block, 1);
+    const long long want = ((long long)a->V / b + sms - 1) / sms * sms;
     *grid = (int)std::min<long long>(hw, std::max(sms, want));
   }
   /* Pannotia SSSP by default: 1024 threads per SM (four 256-thread CTAs of

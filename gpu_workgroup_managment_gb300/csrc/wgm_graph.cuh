@@ -692,8 +692,6 @@ struct wgm_color_args {
   const int *tcol;
   const float *node_value;
   int *color;    /* [V] output: 1-based colours */
-  int *stop;     /* unused (kept for the argument layout of older callers) */
-  int *hub_acc;  /* unused */
   wgm_hubs hubs; /* static layout of out-degree > hub_threshold vertices */
   int hub_threshold;
   int *rounds_out;
@@ -1253,12 +1251,15 @@ struct wgm_mis_args {
   const int *row;
   const int *col;
   const float *node_value;
-  int *s_array; /* [V] output: 2 = member, 0 = not */
-  int *status;  /* [V]: -1 active, 2r removed in round r, 2r+1 joined in r */
-  int *stop;    /* [3 lines] */
-  int *hub_acc; /* [2][H] running min (float bits), by round parity */
-  wgm_hubs hubs;
-  int hub_threshold;
+  int *s_array;   /* [V] output: 2 = member, 0 = not */
+  int2 *word;     /* [V] {status, value bits}; status: -1 active, 2r removed in
+                     round r, 2r+1 joined in r */
+  int *ptr;       /* [V] first edge that can still hold a blocker */
+  unsigned *mask; /* [ceil(V/32)] bit: the vertex may still be active */
+  int *stop;      /* [3 lines] by round mod 3: word 0 any active, word 1 wide entries */
+  int4 *wide;     /* [wide_cap] this round's {vertex, first edge, first blocker, 0} */
+  int wide_cap;   /* >= vertices of more than `scan` edges */
+  int scan;       /* edges of one vertex that a single warp looks at */
   int *rounds_out;
 };
 
@@ -1273,58 +1274,236 @@ __device__ __forceinline__ bool wgm_active_at(int st, int r) {
   return st == -1 || (st >> 1) == r;
 }
 
-/* Phases: (0) init; (1,r) mis1+mis2 for non-hub vertices and hub minima over
- * the grid; (2,r) mis2 for hubs.  (1,r) first applies the reference's exit
- * test to round r-1 (mis.cl:106-108). */
+/* Is edge target j a blocker of a vertex of value v in round r? */
+__device__ __forceinline__ bool wgm_mis_blocks(const wgm_mis_args &a, int j, float v, int r) {
+  const int2 w = __ldca(&a.word[j]);
+  return __int_as_float(w.y) < v && wgm_active_at(w.x, r);
+}
+
+/* Remove the active targets of the lanes' edges start .. start + deg
+ * (warp-collective, four 32-edge windows in flight; mis.cl:86-93). */
+__device__ __forceinline__ void wgm_mis_mark(const wgm_mis_args &a, int r, int start, int deg) {
+  const int lane = wgm_lane();
+  const int incl = wgm_warp_incl_scan(deg);
+  const int total = __shfl_sync(WGM_FULL, incl, 31);
+  const int off = incl - deg, base = start - off;
+  for (int w = 0; w < total; w += 128) {
+    int j[4], st[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int sl = w + 32 * q + lane;
+      const int o = wgm_owner_of(off, min(sl, total - 1));
+      const int e = __shfl_sync(WGM_FULL, base, o) + sl;
+      j[q] = sl < total ? __ldg(&a.col[e]) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) st[q] = j[q] >= 0 ? __ldcg(&a.word[j[q]].x) : 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (st[q] == -1) a.word[j[q]].x = 2 * r; /* once: a hub has many joining neighbours */
+  }
+}
+
+/* First blocker among the edges of the 128-edge steps e0, e0 + stride, ...
+ * below `end` (warp-collective, a step's four windows in flight); INT_MAX if
+ * none. */
+__device__ __forceinline__ int wgm_mis_scan(const wgm_mis_args &a, long long e0, int end,
+                                            int stride, float v, int r) {
+  const int lane = wgm_lane();
+  for (long long x = e0; x < end; x += stride) {
+    const int e = (int)x;
+    int j[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) j[q] = 32 * q + lane < end - e ? __ldg(&a.col[e + 32 * q + lane]) : -1;
+    bool hit[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) hit[q] = j[q] >= 0 && wgm_mis_blocks(a, j[q], v, r);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const unsigned m = __ballot_sync(WGM_FULL, hit[q]);
+      if (m) return e + 32 * q + __ffs(m) - 1;
+    }
+  }
+  return INT_MAX;
+}
+
+/* Round r of the lanes' vertices i (act: the lane has one that may still be
+ * active; cleared when it is not).  Returns whether the vertex stays. */
+__device__ __forceinline__ bool wgm_mis_visit(const wgm_launch &Lc, const wgm_mis_args &a, int r,
+                                              int i, bool &act, int *tab) {
+  const int lane = wgm_lane();
+  const float BIG = (float)WGM_PANNOTIA_BIG;
+  int e = 0, start = 0, end = 0;
+  float v = 0.f;
+  if (act) {
+    const int2 w = __ldcg(&a.word[i]);
+    act = wgm_active_at(w.x, r);
+    v = __int_as_float(w.y);
+    start = __ldg(&a.row[i]);
+    end = __ldg(&a.row[i + 1]);
+    e = r == 1 ? start : __ldcg(&a.ptr[i]);
+  }
+  const int e0 = e;
+  bool blocked = false;
+  if (act) {
+    int j[4];
+    bool hit[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) j[q] = q < end - e ? __ldg(&a.col[e + q]) : -1;
+#pragma unroll
+    for (int q = 0; q < 4; q++) hit[q] = j[q] >= 0 && wgm_mis_blocks(a, j[q], v, r);
+#pragma unroll
+    for (int q = 3; q >= 0; q--)
+      if (hit[q]) {
+        blocked = true;
+        e = e0 + q;
+      }
+    if (!blocked) e += min(4, end - e);
+  }
+  /* the rest of the longer rows, by the whole warp: a step looks at 128
+   * edges, shared evenly among the vertices still open */
+  bool wide = false;
+  const int elim = end - e > a.scan ? e + a.scan : end;
+  unsigned open = __ballot_sync(WGM_FULL, act && !blocked && e < end);
+  while (open) {
+    const int nopen = __popc(open);
+    const int ql = 31 - __clz(128 / nopen), quota = 1 << ql; /* 4 ... 128 */
+    const bool mine = (open >> lane) & 1u;
+    const int rank = __popc(open & wgm_lanemask_lt());
+    if (mine) tab[rank] = lane;
+    __syncwarp();
+    int j[4], own[4];
+    unsigned hit[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int sl = 32 * q + lane, oi = sl >> ql;
+      own[q] = oi < nopen ? tab[oi] : 0;
+      const int oe = __shfl_sync(WGM_FULL, e, own[q]), x = sl & (quota - 1);
+      const int lim = __shfl_sync(WGM_FULL, elim, own[q]);
+      j[q] = oi < nopen && x < lim - oe ? __ldg(&a.col[oe + x]) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float ov = __shfl_sync(WGM_FULL, v, own[q]);
+      hit[q] = __ballot_sync(WGM_FULL, j[q] >= 0 && wgm_mis_blocks(a, j[q], ov, r));
+    }
+    if (mine) {
+      /* this vertex's slots are [rank * quota, (rank + 1) * quota) */
+      const int s0 = rank << ql, w0 = s0 >> 5;
+      unsigned h = w0 == 0 ? hit[0] : w0 == 1 ? hit[1] : w0 == 2 ? hit[2] : hit[3];
+      int f = -1;
+      if (ql < 5) h = (h >> (s0 & 31)) & ((1u << quota) - 1u);
+      if (h) f = __ffs(h) - 1;
+      if (ql >= 6 && f < 0) { /* 64 or 128 slots */
+        const unsigned h1 = w0 == 0 ? hit[1] : hit[3];
+        if (h1) f = 31 + __ffs(h1);
+        if (ql == 7 && f < 0 && hit[2]) f = 63 + __ffs(hit[2]);
+        if (ql == 7 && f < 0 && hit[3]) f = 95 + __ffs(hit[3]);
+      }
+      blocked = f >= 0;
+      e = blocked ? e + f : e + min(quota, elim - e);
+      wide = !blocked && e == elim && elim < end;
+    }
+    __syncwarp();
+    open = __ballot_sync(WGM_FULL, mine && !blocked && e < elim);
+  }
+  bool join = act && !blocked && !wide && v < BIG;
+  if (join) {
+    a.s_array[i] = 2;
+    a.word[i].x = 2 * r + 1;
+    wide = end - start > a.scan; /* its marks are the grid's */
+  }
+  if (wide) {
+    const int b = atomicAdd(&a.stop[(r % 3) * WGM_LINE + 1], 1);
+    if (b < a.wide_cap)
+      a.wide[b] = make_int4(i, e, INT_MAX, 0);
+    else
+      wgm_fail(Lc, WGM_DEV_OVERFLOW, WGM_SITE_QUEUE, r);
+  }
+  if (__any_sync(WGM_FULL, join && !wide))
+    wgm_mis_mark(a, r, start, join && !wide ? end - start : 0);
+  if (act && !join && (e != e0 || r == 1)) a.ptr[i] = e;
+  return act && !join;
+}
+
+/* A vertex joins when no active out-neighbour has a smaller value
+ * (mis.cl:68-75: value < the minimum over active neighbours), so a look
+ * stops at the first such neighbour - its blocker - and the next round goes
+ * on from there: a neighbour that did not block (larger, or gone) never will
+ * again, statuses only leave "active".  Over all rounds every edge is looked
+ * at about once at most instead of once per round: on RMAT-20 (31.4 M edges,
+ * 8 rounds) 5.1 M looks and 2.6 M marks against ~100 M looks, 1.37 ms ->
+ * 0.23 ms.  What bounds it now is one round's chain of dependent round trips
+ * (mask, status and row, column, neighbour, then the marks and the barrier:
+ * 8 us for a round with a handful of vertices, 54 us for the first, which
+ * touches every row).  Two details that cost more than the looks did: a
+ * removed mark is stored only over "active" (a hub has tens of thousands of
+ * joining neighbours; storing it each time made round 1 take 328 us), and
+ * the looks read through L1 - a status read stale within a round reads as
+ * the same "active at its start".
+ *
+ * The vertices that may still be active are kept as one mask word per 32; a
+ * warp owns every NW-th word and packs the vertices left in them 32 at a
+ * time, so a late round's few do not take a pass per word.  Each lane first
+ * looks at four edges of its own vertex (enough for nine in ten on RMAT
+ * graphs), then the warp shares the longer rows, 128 edges a step.  A vertex
+ * with more than `scan` edges left to look at, or to mark, would hold one
+ * warp for long: it goes to a short list that the whole grid works off in
+ * two extra phases, which run only in rounds that list one.
+ * Phases: (0) init; (1,r) looks, joins and marks; (2,r) looks at the listed
+ * vertices, or round r+1 at once when none was listed; (3,r) their joins.
+ * (1,r) first applies the reference's exit test to round r-1
+ * (mis.cl:106-108). */
 static __device__ int wgm_phase_mis(const wgm_launch &Lc, wgm_cta *c, const wgm_mis_args &a,
                                     wgm_warp_smem *sm, wgm_step cur, wgm_step *nxt) {
   const wgm_split s(c);
-  const int V = a.V;
-  const int BIG = __float_as_int((float)WGM_PANNOTIA_BIG);
+  __shared__ int s_pend[WGM_MAX_WARPS][64];
+  const int V = a.V, lane = s.lane, nchunk = (V + 31) >> 5;
+  const float BIG = (float)WGM_PANNOTIA_BIG;
+  int *tab = sm->tab[s.warp];
   if (cur.target == 0) {
     for (int i = s.tid; i < V; i += s.nth) {
       a.s_array[i] = 0; /* mis.h:58-92 */
-      a.status[i] = -1;
+      a.word[i] = make_int2(-1, __float_as_int(__ldg(&a.node_value[i])));
     }
-    for (int h = s.tid; h < 2 * a.hubs.H; h += s.nth) a.hub_acc[h] = BIG;
-    if (c->id == 0 && threadIdx.x == 0)
-      for (int k = 0; k < 3; k++) a.stop[k * WGM_LINE] = 0;
+    for (int k = s.tid; k < nchunk; k += s.nth)
+      a.mask[k] = V - 32 * k >= 32 ? WGM_FULL : (1u << (V & 31)) - 1u;
+    if (c->id == 0 && threadIdx.x < 3) {
+      a.stop[threadIdx.x * WGM_LINE] = 0;
+      a.stop[threadIdx.x * WGM_LINE + 1] = 0;
+    }
     *nxt = {1, 1};
     return WGM_PHASE_NEXT;
   }
-  const int r = cur.round;
-  int *hacc = a.hub_acc + (size_t)(r & 1) * a.hubs.H;
-  const int nwin = (a.hubs.total + 31) >> 5;
-  if (cur.target == 2) {
-    /* mis2 for hubs.  The join test is a pure function of the final hub
-     * minimum and the round-start status (a joined hub reads 2r+1, still
-     * "active at r"), so every warp re-derives it while marking neighbours
-     * and one thread per hub records the join.  The other parity's minima
-     * are reset here for the next round. */
-    int *hnext = a.hub_acc + (size_t)((r + 1) & 1) * a.hubs.H;
-    for (int h = s.tid; h < a.hubs.H; h += s.nth) {
-      int v = __ldg(&a.hubs.ids[h]);
-      if (__ldcg(&a.status[v]) == -1 &&
-          __ldg(&a.node_value[v]) < __int_as_float(__ldcg(&hacc[h]))) {
-        a.s_array[v] = 2;
-        a.status[v] = 2 * r + 1;
-      }
-      hnext[h] = BIG;
-    }
-    for (int k = s.gw; k < nwin; k += s.NW) {
-      wgm_hub_window(a.hubs, a.row, k, [&](bool valid, int h, int e) {
-        if (!valid) return;
-        int v = __ldg(&a.hubs.ids[h]);
-        int stv = __ldcg(&a.status[v]);
-        if (wgm_active_at(stv, r) && stv != 2 * r &&
-            __ldg(&a.node_value[v]) < __int_as_float(__ldcg(&hacc[h]))) {
-          int j = __ldg(&a.col[e]);
-          if (wgm_active_at(__ldcg(&a.status[j]), r) && j != v) a.status[j] = 2 * r;
+  int r = cur.round;
+  if (cur.target >= 2) {
+    const int n = __ldcg(&a.stop[(r % 3) * WGM_LINE + 1]);
+    if (n == 0) {
+      r++; /* nothing listed: this phase is round r+1's first */
+    } else {
+      /* S warps share a listed vertex, each taking every S-th step of 128 edges */
+      const int S = max(1, s.NW / n), sub = s.gw % S, per = s.NW / S;
+      for (int b = s.gw / S; b < n && s.gw < per * S; b += per) {
+        const int4 w = __ldcg(&a.wide[b]);
+        const int row0 = __ldg(&a.row[w.x]), end = __ldg(&a.row[w.x + 1]);
+        const float v = __ldg(&a.node_value[w.x]);
+        if (cur.target == 2) {
+          const int e = wgm_mis_scan(a, w.y + 128LL * sub, end, S * 128, v, r);
+          if (lane == 0 && e != INT_MAX) atomicMin(&a.wide[b].z, e);
+        } else if (w.z != INT_MAX) {
+          if (lane == 0 && sub == 0) a.ptr[w.x] = w.z;
+        } else if (v < BIG) {
+          if (lane == 0 && sub == 0) {
+            a.s_array[w.x] = 2;
+            a.word[w.x].x = 2 * r + 1;
+          }
+          for (long long e = row0 + 128LL * sub; e < end; e += 128LL * S)
+            wgm_mis_mark(a, r, (int)e, lane == 0 ? (int)min(128LL, end - e) : 0);
         }
-      });
+      }
+      *nxt = cur.target == 2 ? wgm_step{3, r} : wgm_step{1, r + 1};
+      return WGM_PHASE_NEXT;
     }
-    *nxt = {1, r + 1};
-    return WGM_PHASE_NEXT;
   }
   if (r > 1 && __ldcg(&a.stop[((r - 1) % 3) * WGM_LINE]) == 0) {
     if (c->id == 0 && threadIdx.x == 0 && a.rounds_out) *a.rounds_out = r - 1;
@@ -1334,80 +1513,40 @@ static __device__ int wgm_phase_mis(const wgm_launch &Lc, wgm_cta *c, const wgm_
     wgm_fail(Lc, WGM_DEV_BAD_INPUT, WGM_SITE_QUEUE, r);
     return WGM_PHASE_DONE;
   }
-  if (c->id == 0 && threadIdx.x == 0) a.stop[((r + 1) % 3) * WGM_LINE] = 0;
+  if (c->id == 0 && threadIdx.x < 2) a.stop[((r + 1) % 3) * WGM_LINE + threadIdx.x] = 0;
   bool any = false;
-  const int lane = s.lane, warp = s.warp;
-  for (int b = s.gw * 32; b < V; b += s.NW * 32) {
-    int i = b + lane;
-    int deg = 0, start = 0;
-    bool act = false;
-    if (i < V) {
-      act = __ldcg(&a.status[i]) == -1; /* active: nothing else can stamp it yet */
-      start = __ldg(&a.row[i]);
-      int d = __ldg(&a.row[i + 1]) - start;
-      if (act) any = true; /* mis.cl:33 */
-      if (d > a.hub_threshold)
-        act = false;
-      else if (act)
-        deg = d;
-    }
-    sm->acc[warp][lane] = BIG;
-    int incl = wgm_warp_incl_scan(deg);
-    int total = __shfl_sync(WGM_FULL, incl, 31);
-    int off = incl - deg;
-    __syncwarp();
-    /* mis1: min over neighbours active at round start (mis.cl:44-51).  (A
-     * four-window version of this walk measured slower here: 8.6 against
-     * 6.9 ms on RMAT-22, the status gathers of idle windows cost more than
-     * the latency they hide.) */
-    wgm_for_each_edge(off, deg, start - off, total, 0, 32, sm->tab[warp],
-                      [&](bool valid, int e, int owner) {
-                        if (valid) {
-                          int j = __ldg(&a.col[e]);
-                          if (wgm_active_at(__ldcg(&a.status[j]), r))
-                            atomicMin(&sm->acc[warp][owner],
-                                      __float_as_int(__ldg(&a.node_value[j])));
-                        }
-                      });
-    __syncwarp();
-    /* mis2: join, then mark the neighbours removed (mis.cl:68-95). */
-    bool join = act && __ldg(&a.node_value[i]) < __int_as_float(sm->acc[warp][lane]);
-    if (join) {
-      a.s_array[i] = 2;
-      a.status[i] = 2 * r + 1;
-    }
-    int jdeg = join ? deg : 0;
-    int jincl = wgm_warp_incl_scan(jdeg);
-    int jtotal = __shfl_sync(WGM_FULL, jincl, 31);
-    int joff = jincl - jdeg;
-    wgm_for_each_edge(joff, jdeg, start - joff, jtotal, 0, 32, sm->tab[warp],
-                      [&](bool valid, int e, int owner) {
-                        if (valid) {
-                          int j = __ldg(&a.col[e]);
-                          if (wgm_active_at(__ldcg(&a.status[j]), r)) a.status[j] = 2 * r;
-                        }
-                      });
-  }
-  /* Hub minima across the grid (mis1 for hubs). */
-  for (int k = s.gw; k < nwin; k += s.NW) {
-    wgm_hub_window(a.hubs, a.row, k, [&](bool valid, int h, int e) {
-      int h0 = __shfl_sync(WGM_FULL, h, 0);
-      int val = INT_MAX;
-      if (valid && wgm_active_at(__ldcg(&a.status[__ldg(&a.hubs.ids[h])]), r)) {
-        int j = __ldg(&a.col[e]);
-        if (wgm_active_at(__ldcg(&a.status[j]), r)) val = __float_as_int(__ldg(&a.node_value[j]));
+  /* this warp's chunks are gw, gw + NW, ...: 32 of their masks in one load */
+  int *pend = s_pend[s.warp];
+  for (long long k0 = s.gw; k0 < nchunk; k0 += 32LL * s.NW) {
+    const long long kl = k0 + (long long)lane * s.NW;
+    const unsigned ml = kl < nchunk ? __ldcg(&a.mask[kl]) : 0u;
+    unsigned todo = __ballot_sync(WGM_FULL, ml != 0u);
+    int n = 0;
+    while (todo || n) {
+      /* gather up to 32 vertices: later rounds leave few in a chunk */
+      while (todo && n < 32) {
+        const int kc = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const unsigned m = __shfl_sync(WGM_FULL, ml, kc);
+        if ((m >> lane) & 1u)
+          pend[n + __popc(m & wgm_lanemask_lt())] = (int)(k0 + (long long)kc * s.NW) * 32 + lane;
+        n += __popc(m);
       }
-      int m0, m1;
-      float f0, f1;
-      wgm_two_seg_reduce(h == h0, val, 0.f, 1, &m0, &m1, &f0, &f1);
-      if (lane == 0) {
-        if (m0 != INT_MAX) atomicMin(&hacc[h0], m0);
-        if (m1 != INT_MAX && h0 + 1 < a.hubs.H) atomicMin(&hacc[h0 + 1], m1);
-      }
-    });
+      __syncwarp();
+      bool act = lane < n;
+      const bool had = act;
+      const int i = act ? pend[lane] : 0;
+      const int rest = lane + 32 < n ? pend[lane + 32] : 0;
+      __syncwarp();
+      if (lane + 32 < n) pend[lane] = rest;
+      n = max(n - 32, 0);
+      const bool left = wgm_mis_visit(Lc, a, r, i, act, tab);
+      any |= act; /* mis.cl:33 */
+      if (had && !left) atomicAnd(&a.mask[i >> 5], ~(1u << (i & 31)));
+    }
   }
   if (__any_sync(WGM_FULL, any) && lane == 0) a.stop[(r % 3) * WGM_LINE] = 1;
-  *nxt = (a.hubs.H > 0) ? wgm_step{2, r} : wgm_step{1, r + 1};
+  *nxt = {2, r};
   return WGM_PHASE_NEXT;
 }
 

@@ -53,7 +53,9 @@ struct wgm_app {
   int *d_wl_start = nullptr, *d_wl_cnt = nullptr, *d_wl_u = nullptr; /* Lonestar pieces */
   int wl_cap = 0, piece = 32;
   int *d_cnt = nullptr, *d_stamp = nullptr, *d_stop = nullptr;
-  int *d_hub_acc = nullptr, *d_status = nullptr;
+  int2 *d_mis_word = nullptr; /* independent set: {status, value bits} */
+  unsigned *d_mis_mask = nullptr;
+  int4 *d_mis_wide = nullptr;
   float *d_contrib = nullptr, *d_dang = nullptr, *d_hub_sum = nullptr;
   int *d_rounds = nullptr;
   /* colour: in-edge CSR when the graph is not symmetric (else the graph) */
