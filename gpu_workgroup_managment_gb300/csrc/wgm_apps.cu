@@ -71,9 +71,9 @@ static bool wgm_is_lonestar(int kind) {
 static bool wgm_needs_weights(int kind) {
   return kind == WGM_APP_LONESTAR_SSSP || kind == WGM_APP_PANNOTIA_SSSP;
 }
+/* (colour's hubs follow its priorities: wgm_color_layout) */
 static bool wgm_uses_static_hubs(int kind) {
-  return kind == WGM_APP_PANNOTIA_COLOR || kind == WGM_APP_PANNOTIA_SSSP ||
-         kind == WGM_APP_PAGERANK;
+  return kind == WGM_APP_PANNOTIA_SSSP || kind == WGM_APP_PAGERANK;
 }
 
 /* Reject graphs the kernels cannot walk safely.  The Lonestar loader quirk
@@ -108,14 +108,17 @@ static int wgm_validate_graph(int kind, const wgm_graph_desc *g) {
   return WGM_OK;
 }
 
-/* Hub layout for the static-frontier apps (see wgm_hubs in wgm_graph.cuh). */
-static void wgm_build_hubs(const wgm_graph_desc *g, int T, std::vector<int> &ids,
-                           std::vector<int> &prefix, std::vector<int> &wmap) {
+/* Hub layout for the static-frontier apps (see wgm_hubs in wgm_graph.cuh);
+ * hubs in the order of `order` (vertex order when null). */
+static void wgm_build_hubs(int V, const int32_t *row_ptr, const int *order, int T,
+                           std::vector<int> &ids, std::vector<int> &prefix,
+                           std::vector<int> &wmap) {
   ids.clear();
   prefix.assign(1, 0);
   wmap.clear();
-  for (int v = 0; v < g->num_nodes; v++) {
-    int d = g->row_ptr[v + 1] - g->row_ptr[v];
+  for (int k = 0; k < V; k++) {
+    const int v = order ? order[k] : k;
+    int d = row_ptr[v + 1] - row_ptr[v];
     if (d > T) {
       ids.push_back(v);
       prefix.push_back(prefix.back() + d);
@@ -132,9 +135,9 @@ static void wgm_build_hubs(const wgm_graph_desc *g, int T, std::vector<int> &ids
     while (prefix[h + 1] <= k * 32) h++;
     const int split = h + 1 < H ? std::min(32, prefix[h + 1] - k * 32) : 32;
     wmap[4 * (size_t)k + 0] = h;
-    wmap[4 * (size_t)k + 1] = g->row_ptr[ids[h]] + (k * 32 - prefix[h]);
+    wmap[4 * (size_t)k + 1] = row_ptr[ids[h]] + (k * 32 - prefix[h]);
     wmap[4 * (size_t)k + 2] = split;
-    wmap[4 * (size_t)k + 3] = split < 32 ? g->row_ptr[ids[h + 1]] : 0;
+    wmap[4 * (size_t)k + 3] = split < 32 ? row_ptr[ids[h + 1]] : 0;
   }
 }
 
@@ -147,7 +150,8 @@ static void wgm_app_free_buffers(wgm_app *a) {
                   a->d_oct_input, a->d_oct_second, a->d_oct_pools, a->d_oct_tree,
                   a->d_oct_ctr, a->d_oct_locks, a->d_oct_heads,
                   a->d_c4_board, a->d_c4_nodes, a->d_c4_pool, a->d_c4_locks,
-                  a->d_c4_heads, a->d_c4_ctr, a->d_tcv, a->d_tcv4, a->d_cmax, a->d_cq,
+                  a->d_c4_heads, a->d_c4_ctr, a->d_cb_ord, a->d_cb_colour,
+                  a->d_cb_crank, a->d_cb_list, a->d_cb_hub, a->d_cb_cnt, a->d_hub_rank, a->d_hub_max, a->d_tcv, a->d_tcv4, a->d_cmax, a->d_cq,
                   a->d_cqctl};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -168,9 +172,9 @@ static cudaError_t wgm_dmalloc(T **p, size_t count) {
   return cudaMalloc((void **)p, std::max<size_t>(count, 1) * sizeof(T));
 }
 
-static int wgm_upload_hubs(wgm_app *a, const wgm_graph_desc *g) {
+static int wgm_upload_hubs(wgm_app *a, const int32_t *row_ptr, const int *order) {
   std::vector<int> ids, prefix, wmap;
-  wgm_build_hubs(g, a->hub_threshold, ids, prefix, wmap);
+  wgm_build_hubs(a->V, row_ptr, order, a->hub_threshold, ids, prefix, wmap);
   cudaStream_t s = a->rt->stream;
   cudaError_t e = cudaSuccess;
   if (a->hubs.ids) {
@@ -237,6 +241,184 @@ static int wgm_upload_transpose(wgm_app *a, const wgm_graph_desc *g) {
   return WGM_OK;
 }
 
+/* Vertices by descending value (values are finite and >= 0, so their bits
+ * sort like the floats): a stable radix sort, 11 bits a pass.  False when two
+ * values are equal. */
+static bool wgm_priority_order(const float *nv, int V, std::vector<int> &order) {
+  struct rec {
+    uint32_t key;
+    int v;
+  };
+  std::vector<rec> x((size_t)V), y((size_t)V);
+  for (int i = 0; i < V; i++) {
+    const float f = nv[i] + 0.0f; /* -0 -> +0 */
+    uint32_t b;
+    std::memcpy(&b, &f, 4);
+    x[i] = {~b, i};
+  }
+  for (int pass = 0; pass < 3; pass++) {
+    const int sh = 11 * pass;
+    std::vector<int> at(2049, 0);
+    for (const rec &r : x) at[((r.key >> sh) & 2047u) + 1]++;
+    for (int k = 0; k < 2048; k++) at[k + 1] += at[k];
+    for (const rec &r : x) y[at[(r.key >> sh) & 2047u]++] = r;
+    x.swap(y);
+  }
+  order.resize((size_t)V);
+  for (int i = 0; i < V; i++) {
+    if (i && x[i].key == x[i - 1].key) return false;
+    order[i] = x[i].v;
+  }
+  return true;
+}
+
+static int wgm_block_size(const wgm_runtime *rt) {
+  int b = rt->cfg.threads_per_wg;
+  if (b < 32 || b > 1024 || b % 32) b = 256;
+  return b;
+}
+
+/* About how many colours independent priorities give.  A chain of falling
+ * priorities inside n vertices of average degree d among themselves gets to
+ * about e d links (n d^k / k! chains of k links are expected to fall all the
+ * way, at least one while k < e d), and the densest part of the graph sets
+ * it: here the best of the subgraphs of vertices of degree at least t, t by
+ * half octaves.  RMAT-20: 2194 against 1629 colours, RMAT-14 477 against
+ * 288, grids 11 against 12-13, a star 5 against 2. */
+static double wgm_color_estimate(const std::vector<int> &row, const unsigned long long *edges) {
+  long long vertices[WGM_DEGREE_BUCKETS] = {};
+  for (size_t v = 0; v + 1 < row.size(); v++) vertices[wgm_degree_bucket(row[v + 1] - row[v])]++;
+  double best = 1.0, n = 0.0, e = 0.0;
+  for (int t = WGM_DEGREE_BUCKETS - 1; t > 0; t--) {
+    n += (double)vertices[t];
+    e += (double)edges[t];
+    if (n > 0.0) best = std::max(best, std::min(2.718 * e / n, n));
+  }
+  return best;
+}
+
+/* Colour's layout, which follows its priorities: hubs in rank order and the
+ * blocks of wgm_k_color_blocks.  NB = sqrt(E / WGM_CB_TARGET) keeps a
+ * block's list (about 1.5 E / NB^2 edges when values are independent of the
+ * graph) near 2900 edges: 128 blocks on RMAT-20.  A block's
+ * vertices also have to fit in shared memory twice, beside as many CTAs per
+ * SM as colour runs on (512 threads).  The lists are counted on the device.
+ * The graph keeps the rounds where
+ *   - a list is too long even with twice the blocks;
+ *   - all lists together are four times what independent values give: the
+ *     values follow the edges, as on a grid numbered row by row, and chains
+ *     run inside every block;
+ *   - the colours it can be expected to take are fewer than 1.5 NB: a block
+ *     costs about 6 us, a round about 5 us, so grids of random priorities
+ *     (a dozen rounds) stay with the rounds once they have 8 blocks. */
+#define WGM_CB_TARGET 1933.0
+static int wgm_color_layout(wgm_app *a) {
+  const int V = a->V;
+  a->cb_blocks = 0;
+  if ((int)a->order.size() != V || (int)a->h_row.size() != V + 1) return WGM_OK;
+  int s = wgm_upload_hubs(a, a->h_row.data(), a->order.data());
+  if (s) return s;
+  std::vector<int> hub_of((size_t)V, -1), hub_rank;
+  for (int k = 0; k < V; k++)
+    if (a->h_row[a->order[k] + 1] - a->h_row[a->order[k]] > a->hub_threshold) {
+      hub_of[k] = (int)hub_rank.size();
+      hub_rank.push_back(k);
+    }
+  const double E = (double)a->E;
+  const int ctas = std::max(1, 512 / wgm_block_size(a->rt));
+  /* 1 KB reserved and 9 KB static per CTA */
+  const long long room =
+      ((long long)a->rt->prop.sharedMemPerMultiprocessor / ctas - 10 * 1024) / 4;
+  const int maxB = (int)std::min<long long>(WGM_CB_MAX_B, room / 2) & ~3;
+  if (maxB < 256) return WGM_OK;
+  int NB = std::max((int)std::ceil(std::sqrt(E / WGM_CB_TARGET)), (V + maxB - 1) / maxB);
+  NB = std::min(std::max(NB, 1), V);
+  const size_t max_blocks = (size_t)std::min<long long>(2LL * NB, V) + 1;
+  cudaStream_t st = a->rt->stream;
+  cudaError_t e = cudaSuccess;
+  for (int **p : {&a->d_cb_hub, &a->d_hub_rank, &a->d_hub_max}) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+  e = wgm_dmalloc(&a->d_cb_hub, max_blocks);
+  if (e == cudaSuccess) e = wgm_dmalloc(&a->d_hub_rank, hub_rank.size());
+  if (e == cudaSuccess) e = wgm_dmalloc(&a->d_hub_max, hub_rank.size());
+  if (e == cudaSuccess && !a->d_cb_ord) {
+    e = wgm_dmalloc(&a->d_cb_ord, (size_t)V);
+    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cb_colour, (size_t)V + 4);
+    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cb_crank, (size_t)a->E);
+    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cb_list, 2 * (size_t)WGM_CB_LISTS);
+    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cb_cnt, 3 * (size_t)WGM_LINE);
+  }
+  if (e == cudaSuccess && !hub_rank.empty())
+    e = cudaMemcpyAsync(a->d_hub_rank, hub_rank.data(), hub_rank.size() * 4,
+                        cudaMemcpyHostToDevice, st);
+  int *tmp = nullptr, *cnt = nullptr; /* order, hub_of, rank; the counts */
+  unsigned long long *hist = nullptr, edges[WGM_DEGREE_BUCKETS] = {};
+  if (e == cudaSuccess) e = wgm_dmalloc(&tmp, 3 * (size_t)V);
+  if (e == cudaSuccess) e = wgm_dmalloc(&cnt, 2 * max_blocks);
+  if (e == cudaSuccess) e = wgm_dmalloc(&hist, WGM_DEGREE_BUCKETS);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(tmp, a->order.data(), (size_t)V * 4, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(tmp + V, hub_of.data(), (size_t)V * 4, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = wgm_launch_color_order(V, (int)a->E, a->d_row, a->d_col, tmp, tmp + V, a->d_cb_ord,
+                               tmp + 2 * (size_t)V, a->d_cb_crank, st);
+  for (int tries = 0; e == cudaSuccess && tries < 2; tries++) {
+    /* whole 16-byte lines of colours, in memory and in shared memory */
+    const int B = std::min(maxB, (int)((((long long)V + NB - 1) / NB + 3) & ~3LL));
+    NB = (V + B - 1) / B;
+    std::vector<int> n(2 * (size_t)NB);
+    e = cudaMemsetAsync(cnt, 0, n.size() * 4, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, sizeof(edges), st);
+    if (e == cudaSuccess)
+      e = wgm_launch_color_count(V, a->d_cb_crank, a->d_cb_ord, B, cnt, hist, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(edges, hist, sizeof(edges), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(n.data(), cnt, n.size() * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) break;
+    long long all = 0;
+    int late = 0, inner = 0;
+    for (int b = 0; b < NB; b++) {
+      all += n[2 * b] + n[2 * b + 1];
+      late = std::max(late, n[2 * b]);
+      inner = std::max(inner, n[2 * b + 1]);
+    }
+    if (late <= WGM_CB_LATE && inner <= WGM_CB_INNER) {
+      if ((double)all <= 6.0 * E / NB + 64.0 * NB &&
+          wgm_color_estimate(a->h_row, edges) > 1.5 * NB) {
+        a->cb_blocks = NB;
+        a->cb_size = B;
+      }
+      break;
+    }
+    NB = (int)std::min<long long>(2LL * NB, V);
+  }
+  if (e == cudaSuccess && a->cb_blocks) {
+    std::vector<int> bh((size_t)a->cb_blocks + 1);
+    size_t h = 0;
+    for (int b = 0; b <= a->cb_blocks; b++) {
+      while (h < hub_rank.size() && hub_rank[h] < (long long)b * a->cb_size) h++;
+      bh[b] = (int)h;
+    }
+    e = cudaMemcpyAsync(a->d_cb_hub, bh.data(), bh.size() * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  const cudaError_t e2 = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = e2;
+  if (tmp) cudaFree(tmp);
+  if (cnt) cudaFree(cnt);
+  if (hist) cudaFree(hist);
+  if (e != cudaSuccess) {
+    a->cb_blocks = 0;
+    return wgm_cuda_fail(a->rt, e);
+  }
+  return WGM_OK;
+}
+
 extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
   if (!a || a->kind == WGM_APP_OCTREE || a->kind == WGM_APP_CONNECT_FOUR ||
       a->kind == WGM_APP_PLUGIN)
@@ -254,7 +436,12 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
     e = cudaMemcpyAsync(a->d_wt, g->weights, (size_t)a->E * 4, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   if (wgm_uses_static_hubs(a->kind)) {
-    s = wgm_upload_hubs(a, g);
+    s = wgm_upload_hubs(a, g->row_ptr, nullptr);
+    if (s) return s;
+  }
+  if (a->kind == WGM_APP_PANNOTIA_COLOR) {
+    a->h_row.assign(g->row_ptr, g->row_ptr + a->V + 1);
+    s = wgm_color_layout(a); /* nothing to do before the first priorities */
     if (s) return s;
   }
   if (a->kind == WGM_APP_PANNOTIA_COLOR || a->kind == WGM_APP_PANNOTIA_BC) {
@@ -398,20 +585,20 @@ extern "C" int wgm_app_set_node_values(wgm_app *a, const float *nv) {
   if (!a || !nv || !a->d_node_value) return WGM_ERR_INVALID;
   for (int i = 0; i < a->V; i++)
     if (!(nv[i] >= 0.0f && nv[i] < 1.0e30f)) return WGM_ERR_INVALID; /* finite, >= 0 */
-  {
-    /* Equal priorities on adjacent vertices stall colour and MIS forever (in
-     * the reference too): require distinct values. */
-    std::vector<float> sorted(nv, nv + a->V);
-    std::sort(sorted.begin(), sorted.end());
-    for (int i = 1; i < a->V; i++)
-      if (sorted[i] == sorted[i - 1]) return WGM_ERR_INVALID;
-  }
+  /* Equal priorities on adjacent vertices stall colour and MIS forever (in
+   * the reference too): require distinct values. */
+  std::vector<int> order;
+  if (!wgm_priority_order(nv, a->V, order)) return WGM_ERR_INVALID;
   cudaSetDevice(a->rt->device);
   cudaError_t e = cudaMemcpyAsync(a->d_node_value, nv, (size_t)a->V * 4, cudaMemcpyHostToDevice,
                                   a->rt->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(a->rt->stream);
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   a->has_node_values = true;
+  if (a->kind == WGM_APP_PANNOTIA_COLOR) {
+    a->order.swap(order);
+    return wgm_color_layout(a);
+  }
   return WGM_OK;
 }
 
@@ -684,6 +871,26 @@ static wgm_color_async_args wgm_color_async_view(const wgm_app *a) {
   return q;
 }
 
+/* The default of standalone runs where the layout allows it. */
+static bool wgm_color_blocks_on(const wgm_app *a) {
+  return a->kind == WGM_APP_PANNOTIA_COLOR && a->color_mode == 0 && a->cb_blocks > 0;
+}
+
+static wgm_color_blocks_args wgm_color_blocks_view(const wgm_app *a) {
+  wgm_color_blocks_args q;
+  q.ord = a->d_cb_ord;
+  q.crank = a->d_cb_crank;
+  q.colour = a->d_cb_colour;
+  q.blk_hub = a->d_cb_hub;
+  q.hub_rank = a->d_hub_rank;
+  q.list = a->d_cb_list;
+  q.cnt = a->d_cb_cnt;
+  q.hub_max = a->d_hub_max;
+  q.NB = a->cb_blocks;
+  q.B = a->cb_size;
+  return q;
+}
+
 static bool wgm_color_async_on(const wgm_app *a) {
   return a->kind == WGM_APP_PANNOTIA_COLOR && a->color_mode == 1;
 }
@@ -709,6 +916,8 @@ static cudaError_t wgm_app_enqueue(wgm_app *a, const wgm_launch &L, int grid, in
         if (e != cudaSuccess) return e;
         return wgm_launch_color_async(L, A.color, wgm_color_async_view(a), grid, block, stream);
       }
+      if (wgm_color_blocks_on(a))
+        return wgm_launch_color_blocks(L, A.color, wgm_color_blocks_view(a), grid, block, stream);
       return wgm_launch_color(L, A.color, grid, block, stream);
     case WGM_APP_PANNOTIA_MIS:
       return wgm_launch_mis(L, A.mis, grid, block, stream);
@@ -744,6 +953,11 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
   } else if (wgm_color_async_on(a)) {
     int per_sm = 0;
     cudaError_t e = wgm_color_async_per_sm(block, &per_sm);
+    if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
+    hw = std::min(per_sm * a->rt->prop.multiProcessorCount, WGM_MAX_GROUPS);
+  } else if (wgm_color_blocks_on(a)) {
+    int per_sm = 0;
+    cudaError_t e = wgm_color_blocks_per_sm(block, a->cb_size, &per_sm);
     if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
     hw = std::min(per_sm * a->rt->prop.multiProcessorCount, WGM_MAX_GROUPS);
   } else {
@@ -790,12 +1004,6 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
     *grid = (int)std::min<long long>(hw, std::max(base, byE));
   }
   return WGM_OK;
-}
-
-static int wgm_block_size(const wgm_runtime *rt) {
-  int b = rt->cfg.threads_per_wg;
-  if (b < 32 || b > 1024 || b % 32) b = 256;
-  return b;
 }
 
 extern "C" int wgm_launch_persistent(wgm_runtime *rt, wgm_app *a, int num_wgs, void *stream) {

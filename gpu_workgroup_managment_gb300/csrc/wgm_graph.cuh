@@ -990,6 +990,319 @@ static __device__ int wgm_phase_color(const wgm_launch &Lc, wgm_cta *c, const wg
 }
 
 /* ------------------------------------------------------------------------ */
+/* Pannotia colour in priority blocks (standalone runs)                      */
+/* ------------------------------------------------------------------------ */
+
+/* colour(v) = 1 + the largest colour among v's larger out-neighbours (1 if
+ * none; degree-1 vertices 1), the recurrence wgm_phase_color computes a
+ * round - a grid barrier and six dependent round trips - per colour.  Here
+ * the vertices are taken by rank (descending value), NB blocks of B: every
+ * larger out-neighbour of a vertex is in its own block or an earlier one.
+ *   - The grid looks at every edge of block b once (stage A): an edge to a
+ *     block before b - 1, whose colours are final, raises the vertex's
+ *     colour so far; an edge inside block b or to block b - 1 goes to a
+ *     short list.
+ *   - One CTA finishes the block (stage B) with the colours of blocks b - 1
+ *     and b in shared memory: listed edges from block b - 1 raise their
+ *     target, the inner ones (a few hundred) are relaxed all at once until a
+ *     sweep changes nothing - as many sweeps as the longest chain inside
+ *     the block.
+ * Stage B of block b - 1 runs beside stage A of block b, so a block costs
+ * one grid barrier, and a link of a colour chain a sweep of shared memory
+ * instead of a round.  Colours, columns and the list all go by rank, so
+ * stage B touches memory in whole lines only: one CTA gathers about 0.3
+ * words a cycle, and with vertex ids it spent 10 us a block on 5700 gathers.
+ * RMAT-20 (about 1650 colours): 128 blocks, 8.6 ms in rounds -> 1.6 ms.  A
+ * block takes 12.5 us, and stage B sets it: 2 us to fetch the block's
+ * colours and lists, 1.5 us for the late edges, 4 us for the inner ones
+ * (14 links a block), 1 us to write back, and 3.5 us for a barrier that
+ * waits for those writes; stage A takes 2-5 us beside it. */
+#define WGM_CB_LATE 6144  /* edges listed from a block to the one before it */
+#define WGM_CB_INNER 3072 /* edges listed inside a block */
+#define WGM_CB_LISTS (WGM_CB_LATE + WGM_CB_INNER)
+#define WGM_CB_MAX_B 8192 /* vertices of a block (a list entry packs 13 + 13 bits) */
+struct wgm_color_blocks_args {
+  const int4 *ord;     /* [V] by rank: {vertex, first edge, out-degree, hub index or -1} */
+  const int *crank;    /* [E] col[] as ranks */
+  int *colour;         /* [V] by rank: colour so far, then the colour */
+  const int *blk_hub;  /* [NB+1] first hub of each block (hubs in rank order) */
+  const int *hub_rank; /* [H] */
+  unsigned *list;      /* [2][WGM_CB_LISTS] by block parity: late edges, then inner
+                          ones, each target << 16 | source, ranks in their blocks */
+  int *cnt;            /* [3 lines] by block mod 3: late edges, inner edges; word 2 of
+                          line 0: largest colour */
+  int *hub_max;        /* [H] largest final colour seen by a hub */
+  int NB, B;
+};
+
+extern __shared__ int wgm_cb_dyn[]; /* group 0: the colours of two blocks, 2 x B; a 0 */
+
+/* Append the lanes' edges of four windows to the block's lists: target k,
+ * source rank j; late when lo2 <= j < lo, inner when lo <= j < lo + k. */
+__device__ __forceinline__ bool wgm_cb_emit(const int (&k)[4], const int (&j)[4], int lo, int lo2,
+                                            int *counter, unsigned *list) {
+  const int lane = wgm_lane();
+  unsigned ml[4], mi[4];
+  int nl = 0, ni = 0;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    ml[q] = __ballot_sync(WGM_FULL, j[q] >= lo2 && j[q] < lo);
+    mi[q] = __ballot_sync(WGM_FULL, j[q] >= lo && j[q] < lo + k[q]);
+    nl += __popc(ml[q]);
+    ni += __popc(mi[q]);
+  }
+  if ((nl | ni) == 0) return true;
+  int base = 0; /* both counters at once */
+  if (lane < 2 && (lane ? ni : nl)) base = atomicAdd(counter + lane, lane ? ni : nl);
+  int bl = __shfl_sync(WGM_FULL, base, 0), bi = __shfl_sync(WGM_FULL, base, 1);
+  if (bl + nl > WGM_CB_LATE || bi + ni > WGM_CB_INNER) return false;
+  bi += WGM_CB_LATE;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    if ((ml[q] >> lane) & 1u)
+      list[bl + __popc(ml[q] & wgm_lanemask_lt())] = (unsigned)k[q] << 16 | (unsigned)(j[q] - lo2);
+    if ((mi[q] >> lane) & 1u)
+      list[bi + __popc(mi[q] & wgm_lanemask_lt())] = (unsigned)k[q] << 16 | (unsigned)(j[q] - lo);
+    bl += __popc(ml[q]);
+    bi += __popc(mi[q]);
+  }
+  return true;
+}
+
+/* What a warp's first step of stage A reads and no barrier orders: its
+ * vertices' records and the targets of their first 128 edges. */
+struct wgm_cb_first {
+  int4 o;
+  int own[4], j[4];
+};
+
+/* Vertices per warp of stage A: few, so that a block's edges spread over
+ * every warp. */
+__device__ __forceinline__ int wgm_cb_per(int n, int NW) {
+  return max(1, min(32, (n + NW - 1) / NW));
+}
+
+/* Owner lane and target rank of the edge slots w .. w + 127. */
+__device__ __forceinline__ void wgm_cb_load(const int *crank, int off, int base, int total, int w,
+                                            int (&own)[4], int (&j)[4]) {
+#pragma unroll
+  for (int p = 0; p < 4; p++) {
+    const int sl = w + 32 * p + wgm_lane();
+    own[p] = wgm_owner_of(off, min(sl, total - 1));
+    const int e = __shfl_sync(WGM_FULL, base, own[p]) + sl;
+    j[p] = sl < total ? __ldg(&crank[e]) : INT_MAX;
+  }
+}
+
+/* Degree as stage A walks it: hubs go by windows, a degree-1 vertex skips
+ * its neighbour (color.cl:46). */
+__device__ __forceinline__ int wgm_cb_degree(const int4 &o) {
+  return o.w >= 0 || o.z == 1 ? 0 : o.z;
+}
+
+__device__ __forceinline__ wgm_cb_first wgm_cb_prefetch(const wgm_color_args &a,
+                                                        const wgm_color_blocks_args &q, int b,
+                                                        int gw, int NW) {
+  const int lane = wgm_lane(), lo = b * q.B, n = min(q.B, a.V - lo);
+  const int per = wgm_cb_per(n, NW), k = gw * per + lane;
+  wgm_cb_first F;
+  F.o = lane < per && k < n ? __ldg(&q.ord[lo + k]) : make_int4(0, 0, 0, -1);
+  const int deg = wgm_cb_degree(F.o), incl = wgm_warp_incl_scan(deg);
+  const int total = __shfl_sync(WGM_FULL, incl, 31), off = incl - deg;
+  wgm_cb_load(q.crank, off, F.o.y - off, total, 0, F.own, F.j);
+  return F;
+}
+
+/* Stage A of block b on warp gw of NW.  Returns false on a full list. */
+__device__ __forceinline__ bool wgm_cb_look(const wgm_color_args &a,
+                                            const wgm_color_blocks_args &q, int b, int gw, int NW,
+                                            wgm_cb_first &F, wgm_warp_smem *sm) {
+  const int lane = wgm_lane(), warp = threadIdx.x >> 5;
+  const int lo = b * q.B, n = min(q.B, a.V - lo), lo2 = lo - q.B; /* < 0 for block 0 */
+  int *cnt = &q.cnt[(b % 3) * WGM_LINE];
+  unsigned *list = q.list + (size_t)(b & 1) * WGM_CB_LISTS;
+  int *acc = sm->acc[warp];
+  bool ok = true;
+  const int per = wgm_cb_per(n, NW);
+  for (int k0 = gw * per; k0 < n; k0 += NW * per) {
+    const bool mine = lane < per && k0 + lane < n, first = k0 == gw * per;
+    if (!first) F.o = mine ? __ldg(&q.ord[lo + k0 + lane]) : make_int4(0, 0, 0, -1);
+    const int4 o = F.o;
+    const int deg = wgm_cb_degree(o);
+    acc[lane] = 0;
+    const int incl = wgm_warp_incl_scan(deg);
+    const int total = __shfl_sync(WGM_FULL, incl, 31);
+    const int off = incl - deg;
+    __syncwarp();
+    for (int w = 0; w < total; w += 128) {
+      int c[4], k[4];
+      if (!first || w) wgm_cb_load(q.crank, off, o.y - off, total, w, F.own, F.j);
+#pragma unroll
+      for (int p = 0; p < 4; p++) c[p] = F.j[p] < lo2 ? __ldca(&q.colour[F.j[p]]) : 0;
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        k[p] = k0 + F.own[p];
+        if (c[p] > 0) atomicMax(&acc[F.own[p]], c[p]);
+      }
+      ok &= wgm_cb_emit(k, F.j, lo, lo2, cnt, list);
+    }
+    __syncwarp();
+    if (mine) q.colour[lo + k0 + lane] = acc[lane] + 1;
+    __syncwarp();
+  }
+  /* the block's hubs, a window of 32 edges at a time, last warps first */
+  const int h0 = __ldg(&q.blk_hub[b]), h1 = __ldg(&q.blk_hub[b + 1]);
+  if (h0 < h1) {
+    const int w0 = __ldg(&a.hubs.prefix[h0]) >> 5, w1 = (__ldg(&a.hubs.prefix[h1]) + 31) >> 5;
+    const int4 *wrec = reinterpret_cast<const int4 *>(a.hubs.wmap);
+    for (int k0 = w0 + (NW - 1 - gw) * 4; k0 < w1; k0 += NW * 4) {
+      int4 w[4];
+      int j[4], c[4], k[4];
+#pragma unroll
+      for (int p = 0; p < 4; p++) w[p] = __ldg(wrec + min(k0 + p, w1 - 1));
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        int h, e;
+        wgm_hub_slot(w[p], lane, &h, &e);
+        const bool in =
+            k0 + p < w1 && (k0 + p) * 32 + lane < a.hubs.total && h >= h0 && h < h1;
+        j[p] = in ? __ldg(&q.crank[e]) : INT_MAX;
+        k[p] = in ? __ldg(&q.hub_rank[h]) - lo : 0;
+      }
+#pragma unroll
+      for (int p = 0; p < 4; p++) c[p] = j[p] < lo2 ? __ldca(&q.colour[j[p]]) : 0;
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const bool first = lane < w[p].z;
+        const int m0 = __reduce_max_sync(WGM_FULL, first ? c[p] : 0);
+        const int m1 = __reduce_max_sync(WGM_FULL, first ? 0 : c[p]);
+        if (lane == 0 && m0 > 0) atomicMax(&q.hub_max[w[p].x], m0);
+        if (lane == 0 && m1 > 0) atomicMax(&q.hub_max[w[p].x + 1], m1);
+      }
+      ok &= wgm_cb_emit(k, j, lo, lo2, cnt, list);
+    }
+  }
+  return ok;
+}
+
+/* Stage B of block b on this CTA (every thread): returns the thread's
+ * largest colour.  A function of its own: its registers and those of the
+ * prefetched step of stage A never live at once. */
+static __device__ __noinline__ int wgm_cb_finish(int V, int B, int b, int *colour,
+                                                 const unsigned *lists, int *cnts,
+                                                 const int *blk_hub, const int *hub_rank,
+                                                 const int *hub_max) {
+  const int T = blockDim.x, lo = b * B, nv = min(B, V - lo);
+  const unsigned *list = lists + (size_t)(b & 1) * WGM_CB_LISTS;
+  int *cnt = cnts + (b % 3) * WGM_LINE;
+  int *cur = wgm_cb_dyn + (b & 1) * B;
+  const int *prev = wgm_cb_dyn + ((b + 1) & 1) * B;
+  /* everything a thread reads is in flight before it waits: the lists' first
+   * entries beside their lengths, the block's colours */
+  constexpr int KL = 8, KI = 4;
+  unsigned late[KL], in[KI];
+  const int2 n2 = __ldcg(reinterpret_cast<const int2 *>(cnt));
+#pragma unroll
+  for (int p = 0; p < KI; p++) {
+    const int e = threadIdx.x + p * T;
+    in[p] = e < WGM_CB_INNER ? __ldcg(&list[WGM_CB_LATE + e]) : 0u;
+  }
+#pragma unroll
+  for (int p = 0; p < KL; p++) {
+    const int e = threadIdx.x + p * T;
+    late[p] = e < WGM_CB_LATE ? __ldcg(&list[e]) : 0u;
+  }
+  const int h0 = __ldg(&blk_hub[b]), h1 = __ldg(&blk_hub[b + 1]);
+  for (int k0 = 4 * threadIdx.x; k0 < nv; k0 += 16 * T) { /* lo is a multiple of 4 */
+    int4 c[4];
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+      if (k0 + 4 * p * T < nv)
+        c[p] = __ldcg(reinterpret_cast<const int4 *>(&colour[lo + k0 + 4 * p * T]));
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+      if (k0 + 4 * p * T < nv) *reinterpret_cast<int4 *>(&cur[k0 + 4 * p * T]) = c[p];
+  }
+  const int nl = min(n2.x, WGM_CB_LATE), ni = min(n2.y, WGM_CB_INNER);
+  if (threadIdx.x == 0) wgm_cb_dyn[2 * B] = 0;
+  __syncthreads();
+  for (int h = h0 + threadIdx.x; h < h1; h += T)
+    atomicMax(&cur[__ldg(&hub_rank[h]) - lo], __ldcg(&hub_max[h]) + 1);
+  for (int e0 = threadIdx.x; e0 < nl; e0 += KL * T) {
+    if (e0 >= KL * T) {
+#pragma unroll
+      for (int p = 0; p < KL; p++) late[p] = e0 + p * T < nl ? __ldcg(&list[e0 + p * T]) : 0u;
+    }
+    /* few exceed what earlier blocks gave their target */
+    int c[KL], d[KL];
+#pragma unroll
+    for (int p = 0; p < KL; p++) {
+      const bool have = e0 + p * T < nl;
+      c[p] = have ? prev[late[p] & 0xffffu] : 0;
+      d[p] = have ? cur[late[p] >> 16] : 1;
+    }
+#pragma unroll
+    for (int p = 0; p < KL; p++)
+      if (c[p] >= d[p]) atomicMax(&cur[late[p] >> 16], c[p] + 1);
+  }
+  __syncthreads();
+  /* Inner edges, all at once until a sweep changes nothing.  A look at four edges takes about 200 cycles and a CTA
+   * barrier with its vote 260, so a sweep looks three times (13 links: 4600
+   * cycles, against 6750 with one look).  A chain inside the block has fewer
+   * than nv links; an absent edge reads a word that stays 0.  Plain stores
+   * do: of two that meet, the smaller may stay, but its loser is still
+   * violated at the next look, and no value ever passes the true colour. */
+  volatile int *col = cur;
+  int src[KI], dst[KI];
+#pragma unroll
+  for (int p = 0; p < KI; p++) {
+    const bool have = (int)threadIdx.x + p * T < ni;
+    src[p] = have ? (int)(in[p] & 0xffffu) : (2 - (b & 1)) * B;
+    dst[p] = have ? (int)(in[p] >> 16) : 0;
+  }
+  for (int sweep = 0; sweep <= nv; sweep++) {
+    bool changed = false;
+#pragma unroll 1
+    for (int look = 0; look < 3; look++) {
+      int c[KI], d[KI];
+#pragma unroll
+      for (int p = 0; p < KI; p++) {
+        c[p] = col[src[p]];
+        d[p] = col[dst[p]];
+      }
+#pragma unroll
+      for (int p = 0; p < KI; p++)
+        if (c[p] >= d[p]) {
+          col[dst[p]] = c[p] + 1;
+          changed = true;
+        }
+    }
+    for (int e = threadIdx.x + KI * T; e < ni; e += T) { /* dense blocks */
+      const unsigned y = __ldcg(&list[WGM_CB_LATE + e]);
+      const int c = col[y & 0xffffu] + 1;
+      if (c > col[y >> 16]) {
+        col[y >> 16] = c;
+        changed = true;
+      }
+    }
+    if (!__syncthreads_or(changed)) break;
+  }
+  int m = 0;
+  for (int k = 4 * threadIdx.x; k < nv; k += 4 * T) {
+    const int4 c = *reinterpret_cast<const int4 *>(&cur[k]);
+    *reinterpret_cast<int4 *>(&colour[lo + k]) = c;
+    m = max(m, c.x);
+    if (k + 1 < nv) m = max(m, c.y);
+    if (k + 2 < nv) m = max(m, c.z);
+    if (k + 3 < nv) m = max(m, c.w);
+  }
+  /* this line counts block b + 3 next; its pushes begin two barriers on */
+  if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
+  __syncthreads();
+  return m;
+}
+
+/* ------------------------------------------------------------------------ */
 /* Pannotia colour without rounds (standalone runs)                          */
 /* ------------------------------------------------------------------------ */
 

@@ -65,6 +65,14 @@ struct wgm_app {
    * first such run */
   int color_mode = 0;
   int bfs_mode = -1; /* Lonestar BFS: -1 automatic, 0 grid, 1 one CTA */
+  /* colour in priority blocks (wgm_color_layout): order and row pointers on
+   * the host, cb_blocks 0 when the graph is left to the rounds */
+  std::vector<int> h_row, order;
+  int4 *d_cb_ord = nullptr;
+  unsigned *d_cb_list = nullptr;
+  int *d_cb_colour = nullptr, *d_cb_crank = nullptr, *d_cb_hub = nullptr, *d_cb_cnt = nullptr;
+  int *d_hub_rank = nullptr, *d_hub_max = nullptr;
+  int cb_blocks = 0, cb_size = 0;
   int4 *d_tcv4 = nullptr;
   int *d_cmax = nullptr, *d_cq = nullptr, *d_cqctl = nullptr;
   int cq_cap = 0;

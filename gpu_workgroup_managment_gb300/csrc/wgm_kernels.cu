@@ -4,6 +4,8 @@
  */
 #include "wgm_kernels.cuh"
 
+#include <algorithm>
+
 #define WGM_PERSISTENT_PROLOGUE                                  \
   __shared__ wgm_cta c;                                          \
   __shared__ wgm_warp_smem sm;                                   \
@@ -63,6 +65,124 @@ __global__ void __maxnreg__(48) wgm_k_mis(wgm_launch L, wgm_mis_args a) {
   WGM_PERSISTENT_PROLOGUE
   WGM_DRIVE(wgm_phase_mis(L, &c, a, &sm, cur, nxt));
   WGM_PERSISTENT_EPILOGUE
+}
+
+/* Pannotia colour in priority blocks (wgm_cb_look, wgm_cb_finish).  Dynamic
+ * shared memory: wgm_color_blocks_smem_bytes (group 0 uses it). */
+__global__ void __launch_bounds__(1024) wgm_k_color_blocks(wgm_launch L, wgm_color_args a,
+                                                           wgm_color_blocks_args q) {
+  WGM_PERSISTENT_PROLOGUE
+  const wgm_split s(&c);
+  int mx = 0;
+  bool ok = true;
+  for (int h = s.tid; h < a.hubs.H; h += s.nth) q.hub_max[h] = 0;
+  if (c.id == 0 && threadIdx.x < 3)
+    for (int k = 0; k < 3; k++) q.cnt[threadIdx.x * WGM_LINE + k] = 0;
+  /* group 0 finishes blocks, the others look; a single group does both */
+  const bool both = c.ngroups == 1;
+  const int nw = blockDim.x >> 5;
+  const int gw = both ? s.gw : s.gw - nw, NW = both ? nw : s.NW - nw;
+  bool live = true;
+  for (int b = 0; b <= q.NB; b++) {
+    const bool look = b < q.NB && (both || c.id > 0);
+    wgm_cb_first F;
+    if (look) F = wgm_cb_prefetch(a, q, b, gw, NW);
+    live = wgm_barrier(L, &c);
+    if (!live) break;
+    if (b > 0 && c.id == 0)
+      mx = max(mx, wgm_cb_finish(a.V, q.B, b - 1, q.colour, q.list, q.cnt, q.blk_hub, q.hub_rank,
+                                 q.hub_max));
+    if (look) ok &= wgm_cb_look(a, q, b, gw, NW, F, &sm);
+  }
+  /* the largest colour is the reference's round count */
+  if (c.id == 0) {
+    mx = __reduce_max_sync(WGM_FULL, mx);
+    if (s.lane == 0) atomicMax(&q.cnt[2], mx);
+  }
+  if (!__all_sync(WGM_FULL, ok) && s.lane == 0) wgm_fail(L, WGM_DEV_OVERFLOW, WGM_SITE_QUEUE, 0);
+  if (live && wgm_barrier(L, &c)) {
+    for (int k = s.tid; k < a.V; k += s.nth) a.color[__ldg(&q.ord[k]).x] = __ldcg(&q.colour[k]);
+    if (c.id == 0 && threadIdx.x == 0 && a.rounds_out) *a.rounds_out = __ldcg(&q.cnt[2]);
+  }
+  WGM_PERSISTENT_EPILOGUE
+}
+
+size_t wgm_color_blocks_smem_bytes(int B) { return (2 * (size_t)B + 4) * 4; }
+
+/* CTAs per SM of a launch with blocks of B vertices. */
+cudaError_t wgm_color_blocks_per_sm(int block, int B, int *per_sm) {
+  /* the limit is the kernel's, whoever launches it next: always the most */
+  cudaError_t e = cudaFuncSetAttribute(wgm_k_color_blocks,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)wgm_color_blocks_smem_bytes(WGM_CB_MAX_B));
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, wgm_k_color_blocks, block,
+                                                       wgm_color_blocks_smem_bytes(B));
+}
+
+cudaError_t wgm_launch_color_blocks(const wgm_launch &L, const wgm_color_args &a,
+                                    const wgm_color_blocks_args &q, int grid, int block,
+                                    cudaStream_t s) {
+  wgm_k_color_blocks<<<grid, block, wgm_color_blocks_smem_bytes(q.B), s>>>(L, a, q);
+  return cudaGetLastError();
+}
+
+/* Layout of the priority blocks: the rank order's vertex records, the
+ * columns as ranks, how many late (cnt[2b]) and inner edges (cnt[2b+1])
+ * each block would list, and the edges by the smaller degree of their ends
+ * (hist, by wgm_degree_bucket). */
+__global__ void __launch_bounds__(256) wgm_k_color_order(int V, const int *row, const int *order,
+                                                         const int *hub_of, int4 *ord, int *rank) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < V; k += gridDim.x * blockDim.x) {
+    const int v = order[k], s = row[v];
+    ord[k] = make_int4(v, s, row[v + 1] - s, hub_of[k]);
+    rank[v] = k;
+  }
+}
+__global__ void __launch_bounds__(256) wgm_k_color_rank(int E, const int *col, const int *rank,
+                                                        int *crank) {
+  for (long long e = blockIdx.x * 256LL + threadIdx.x; e < E; e += gridDim.x * 256LL)
+    crank[e] = __ldg(&rank[col[e]]);
+}
+__global__ void __launch_bounds__(256) wgm_k_color_count(int V, const int *crank, const int4 *ord,
+                                                         int B, int *cnt,
+                                                         unsigned long long *hist) {
+  const int nw = gridDim.x * (blockDim.x >> 5), lane = wgm_lane();
+  __shared__ int h[WGM_DEGREE_BUCKETS];
+  if (threadIdx.x < WGM_DEGREE_BUCKETS) h[threadIdx.x] = 0;
+  __syncthreads();
+  for (int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < V; k += nw) {
+    const int4 o = ord[k];
+    const int b = k / B, lo = b * B;
+    int n = 0, inner = 0;
+    for (int x = lane; x < o.z && o.z != 1; x += 32) {
+      const int r = crank[o.y + x];
+      n += r < lo && r >= lo - B;
+      inner += r < k && r >= lo;
+      atomicAdd(&h[wgm_degree_bucket(min(o.z, __ldg(&ord[r].z)))], 1);
+    }
+    n = __reduce_add_sync(WGM_FULL, n);
+    inner = __reduce_add_sync(WGM_FULL, inner);
+    if (lane == 0 && n) atomicAdd(&cnt[2 * b], n);
+    if (lane == 0 && inner) atomicAdd(&cnt[2 * b + 1], inner);
+  }
+  __syncthreads();
+  if (threadIdx.x < WGM_DEGREE_BUCKETS && h[threadIdx.x])
+    atomicAdd(&hist[threadIdx.x], (unsigned long long)h[threadIdx.x]);
+}
+
+cudaError_t wgm_launch_color_order(int V, int E, const int *row, const int *col, const int *order,
+                                   const int *hub_of, int4 *ord, int *rank, int *crank,
+                                   cudaStream_t s) {
+  wgm_k_color_order<<<std::min((V + 255) / 256, 1216), 256, 0, s>>>(V, row, order, hub_of, ord,
+                                                                    rank);
+  wgm_k_color_rank<<<1216, 256, 0, s>>>(E, col, rank, crank);
+  return cudaGetLastError();
+}
+cudaError_t wgm_launch_color_count(int V, const int *crank, const int4 *ord, int B, int *cnt,
+                                   unsigned long long *hist, cudaStream_t s) {
+  wgm_k_color_count<<<std::min((V + 7) / 8, 1216), 256, 0, s>>>(V, crank, ord, B, cnt, hist);
+  return cudaGetLastError();
 }
 
 /* Pannotia colour without rounds (wgm_color_async_run): the counts of

@@ -37,12 +37,29 @@ struct wgm_barrier_bench_args {
   unsigned long long *t_last;  /* %globaltimer after the last barrier */
 };
 
+/* Half octaves of a degree: 0, 1, 2, 3, 4-5, 6-7, 8-11, ... */
+#define WGM_DEGREE_BUCKETS 64
+__host__ __device__ inline int wgm_degree_bucket(int d) {
+  int l = 0;
+  for (int x = d; x > 1; x >>= 1) l++;
+  return d < 2 ? d : 2 * l + ((d >> (l - 1)) & 1);
+}
+
 /* Host helpers (wgm_kernels.cu). */
 const void *wgm_kernel_fn(int kid);
 cudaError_t wgm_launch_lonestar(bool sssp, const wgm_launch &L, const wgm_lonestar_args &a,
                                 int grid, int block, cudaStream_t s);
 cudaError_t wgm_launch_color(const wgm_launch &L, const wgm_color_args &a, int grid, int block,
                              cudaStream_t s);
+cudaError_t wgm_launch_color_blocks(const wgm_launch &L, const wgm_color_args &a,
+                                    const wgm_color_blocks_args &q, int grid, int block,
+                                    cudaStream_t s);
+cudaError_t wgm_color_blocks_per_sm(int block, int B, int *per_sm);
+cudaError_t wgm_launch_color_order(int V, int E, const int *row, const int *col, const int *order,
+                                   const int *hub_of, int4 *ord, int *rank, int *crank,
+                                   cudaStream_t s);
+cudaError_t wgm_launch_color_count(int V, const int *crank, const int4 *ord, int B, int *cnt,
+                                   unsigned long long *hist, cudaStream_t s);
 cudaError_t wgm_launch_mis(const wgm_launch &L, const wgm_mis_args &a, int grid, int block,
                            cudaStream_t s);
 size_t wgm_bfs_cta_smem_bytes(int V, int F);
