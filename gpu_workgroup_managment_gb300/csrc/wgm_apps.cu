@@ -150,7 +150,7 @@ static void wgm_app_free_buffers(wgm_app *a) {
                   a->d_oct_input, a->d_oct_second, a->d_oct_pools, a->d_oct_tree,
                   a->d_oct_ctr, a->d_oct_locks, a->d_oct_heads,
                   a->d_c4_board, a->d_c4_nodes, a->d_c4_pool, a->d_c4_locks,
-                  a->d_c4_heads, a->d_c4_ctr, a->d_cb_ord, a->d_cb_colour,
+                  a->d_c4_heads, a->d_c4_ctr, a->d_ell, a->d_cb_ord, a->d_cb_colour,
                   a->d_cb_crank, a->d_cb_list, a->d_cb_hub, a->d_cb_cnt, a->d_hub_rank, a->d_hub_max, a->d_tcv, a->d_tcv4, a->d_cmax, a->d_cq,
                   a->d_cqctl};
   for (void *p : ptrs)
@@ -419,6 +419,39 @@ static int wgm_color_layout(wgm_app *a) {
   return WGM_OK;
 }
 
+/* Lonestar BFS on one CTA (wgm_bfs_cta): chosen by default for graphs of
+ * at most WGM_BFS_CTA_AUTO_V vertices and average degree at most 8, whose
+ * levels carry little work each; possible up to WGM_BFS_CTA_MAX_V vertices
+ * (the visited bits in shared memory). */
+#define WGM_BFS_CTA_AUTO_V 65536
+#define WGM_BFS_CTA_MAX_V (1 << 20)
+#define WGM_BFS_CTA_FRONT 8192
+#define WGM_BFS_CTA_THREADS 1024
+static bool wgm_bfs_cta_on(const wgm_app *a) {
+  if (a->kind != WGM_APP_LONESTAR_BFS || a->V > WGM_BFS_CTA_MAX_V) return false;
+  if (a->bfs_mode >= 0) return a->bfs_mode == 1;
+  return a->V <= WGM_BFS_CTA_AUTO_V && a->E <= 8LL * a->V;
+}
+
+/* The one-CTA BFS's W columns per vertex, where the automatic mode takes it
+ * and every row has at most 8. */
+static int wgm_bfs_ell_layout(wgm_app *a, const int32_t *row_ptr) {
+  a->ell_w = 0;
+  if (a->V > WGM_BFS_CTA_AUTO_V || a->E > 8LL * a->V) return WGM_OK;
+  int most = 0;
+  for (int v = 0; v < a->V; v++) most = std::max(most, row_ptr[v + 1] - row_ptr[v]);
+  if (most > 8) return WGM_OK;
+  const int W = most > 4 ? 8 : 4;
+  if (!a->d_ell) {
+    cudaError_t e = wgm_dmalloc(&a->d_ell, 8 * (size_t)a->V);
+    if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
+  }
+  cudaError_t e = wgm_launch_bfs_ell(W, a->V, a->d_row, a->d_col, a->d_ell, a->rt->stream);
+  if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
+  a->ell_w = W;
+  return WGM_OK;
+}
+
 extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
   if (!a || a->kind == WGM_APP_OCTREE || a->kind == WGM_APP_CONNECT_FOUR ||
       a->kind == WGM_APP_PLUGIN)
@@ -437,6 +470,10 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   if (wgm_uses_static_hubs(a->kind)) {
     s = wgm_upload_hubs(a, g->row_ptr, nullptr);
+    if (s) return s;
+  }
+  if (a->kind == WGM_APP_LONESTAR_BFS) {
+    s = wgm_bfs_ell_layout(a, g->row_ptr);
     if (s) return s;
   }
   if (a->kind == WGM_APP_PANNOTIA_COLOR) {
@@ -624,31 +661,20 @@ static int wgm_bc_cta_launch(wgm_runtime *rt, wgm_app *a, cudaStream_t s) {
   return WGM_OK;
 }
 
-/* Lonestar BFS on one CTA (wgm_bfs_cta): chosen by default for graphs of
- * at most WGM_BFS_CTA_AUTO_V vertices and average degree at most 8, whose
- * levels carry little work each; possible up to WGM_BFS_CTA_MAX_V vertices
- * (the visited bits in shared memory). */
-#define WGM_BFS_CTA_AUTO_V 65536
-#define WGM_BFS_CTA_MAX_V (1 << 20)
-static bool wgm_bfs_cta_on(const wgm_app *a) {
-  if (a->kind != WGM_APP_LONESTAR_BFS || a->V > WGM_BFS_CTA_MAX_V) return false;
-  if (a->bfs_mode >= 0) return a->bfs_mode == 1;
-  return a->V <= WGM_BFS_CTA_AUTO_V && a->E <= 8LL * a->V;
-}
-
 static int wgm_bfs_cta_launch(wgm_runtime *rt, wgm_app *a, cudaStream_t s) {
   wgm_mega_args A;
   std::memset(&A, 0, sizeof(A));
   int st = wgm_app_fill_mega(a, &A);
   if (st) return st;
-  /* the frontier buffers take what shared memory the visited bits leave */
+  /* two frontier buffers beside the visited bits: 64 KB, and the rest of the
+   * SM's 256 KB stays L1 */
   const long long avail = (long long)rt->prop.sharedMemPerBlockOptin - 1024 -
                           (long long)((a->V + 31) / 32) * 4;
-  const int F = (int)std::min<long long>(1 << 16, avail / 8);
+  const int F = (int)std::min<long long>(WGM_BFS_CTA_FRONT, avail / 8);
   if (F < 256) return WGM_ERR_INVALID;
   if (rt->cfg.host_handshake) return WGM_ERR_INVALID; /* no discovery, no handshake */
-  cudaError_t e = wgm_launch_bfs_cta(A.ls, a->d_wl_start, a->wl_cap, F, &rt->hf_dev->status,
-                                     1024, s);
+  cudaError_t e = wgm_launch_bfs_cta(A.ls, a->ell_w, a->d_ell, a->d_wl_start, a->wl_cap, F,
+                                     &rt->hf_dev->status, WGM_BFS_CTA_THREADS, s);
   if (e != cudaSuccess) return wgm_cuda_fail(rt, e);
   return WGM_OK;
 }

@@ -547,77 +547,127 @@ __device__ __forceinline__ bool wgm_ls_level(const wgm_launch &Lc, wgm_cta *c,
  * traversal lives in one CTA: visited bits in shared memory, claimed with a
  * shared-memory atomicOr; the frontier in shared memory (vertices past its
  * capacity spill to global memory); level counters triple-buffered in shared
- * memory, so a level is one __syncthreads and two global round trips (row
- * pointers, then columns).  Same levels as the Lonestar kernel: the source
+ * memory, so a level is one __syncthreads and the round trips of its
+ * adjacency.  Same levels as the Lonestar kernel: the source
  * is level 0, a vertex first reached while level L runs gets L, out-of-range
  * columns are skipped (bfs.cl:116), the loader quirk's negative last degree
  * walks nothing, and the level count is the first level whose frontier
- * walks no edge (the grid form never queues a vertex without edges). */
-struct wgm_bfs_cta_smem {
-  unsigned *bits; /* [ceil(V/32)] visited */
-  int *front;     /* [2][F] frontier buffers */
-  int F;
-};
+ * walks no edge (the grid form never queues a vertex without edges).
+ *
+ * The adjacency: graphs of out-degree at most W = 4 or 8 keep a second copy
+ * of their columns as W per vertex (wgm_k_bfs_ell; WGM_BFS_PAD fills up), so
+ * one round trip brings a vertex's whole row.  W = 0 walks the CSR, four
+ * columns a round trip.
+ * The frontier is kept short of shared memory's size, for the L1 is what
+ * serves the neighbouring rows.  256x256 grid: 1.86 us a level with one
+ * column per round trip (four in a row) -> 0.94 us; 1024 threads 0.344,
+ * 512 0.341, 256 0.37 ms.  Measured and left out: prefetching a found
+ * vertex's row (3 % slower), a warp's reservation by ballots instead of one
+ * per lane (11 % slower), skewed bit words (no change). */
+#define WGM_BFS_PAD INT_MIN
+extern __shared__ int wgm_bfs_dyn[]; /* [ceil(V/32)] visited bits, then 2 x F frontier */
 
-__device__ __forceinline__ void wgm_bfs_cta(const wgm_lonestar_args &a, int *spill, int spill_cap,
-                                            const wgm_bfs_cta_smem &S, int *s_cnt) {
-  const int V = a.V, nw = (V + 31) >> 5;
-  for (int i = threadIdx.x; i < nw; i += blockDim.x) S.bits[i] = 0u;
-  for (int i = threadIdx.x; i < V; i += blockDim.x)
-    a.dist[i] = (i == a.source) ? 0u : WGM_LONESTAR_INF;
+template <int W>
+__device__ __forceinline__ void wgm_bfs_cta(const wgm_lonestar_args &a, const int4 *ell, int *spill,
+                                            int spill_cap, int F, int *s_cnt) {
+  const int V = a.V, nw = (V + 31) >> 5, T = blockDim.x;
+  unsigned *bits = reinterpret_cast<unsigned *>(wgm_bfs_dyn);
+  for (int i = threadIdx.x; i < nw; i += T) bits[i] = 0u;
+  for (int i = threadIdx.x; i < V; i += T) a.dist[i] = (i == a.source) ? 0u : WGM_LONESTAR_INF;
+  if (threadIdx.x < 8) s_cnt[threadIdx.x] = threadIdx.x == 1; /* 0-2: level sizes by L mod 3,
+                                                                 3: overflow, 4-6: the level
+                                                                 walked an edge, by L mod 3 */
+  __syncthreads();
+  /* level 1 reads buffer 1 */
+  int in = nw + F, out = nw, in_sp = spill_cap, out_sp = 0;
   if (threadIdx.x == 0) {
-    s_cnt[0] = 0;
-    s_cnt[1] = 1;
-    s_cnt[2] = 0;
-    s_cnt[3] = 0; /* overflow */
-    for (int k = 4; k < 7; k++) s_cnt[k] = 0; /* the level walked an edge, by L mod 3 */
+    bits[a.source >> 5] = 1u << (a.source & 31);
+    wgm_bfs_dyn[in] = a.source;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    S.bits[a.source >> 5] = 1u << (a.source & 31);
-    S.front[S.F] = a.source; /* level 1 reads buffer 1 */
-  }
-  __syncthreads();
-  int L = 1;
+  int L = 1, c0 = 1, c1 = 2, c2 = 0; /* L, L + 1, L + 2 mod 3 */
   for (;;) {
-    const int n = s_cnt[L % 3];
-    if (n == 0) break;
-    if (L > V + 1) break;
-    const int *in = S.front + (size_t)(L & 1) * S.F;
-    int *out = S.front + (size_t)((L + 1) & 1) * S.F;
-    const int *in_sp = spill + (size_t)(L & 1) * spill_cap;
-    int *out_sp = spill + (size_t)((L + 1) & 1) * spill_cap;
-    int *oc = &s_cnt[(L + 1) % 3];
+    const int n = s_cnt[c0];
+    if (n == 0 || L > V + 1) break;
     if (threadIdx.x == 0) {
-      s_cnt[(L + 2) % 3] = 0;
-      s_cnt[4 + (L + 2) % 3] = 0;
+      s_cnt[c2] = 0;
+      s_cnt[4 + c2] = 0;
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const int v = i < S.F ? in[i] : __ldcg(&in_sp[i - S.F]);
-      const int s = __ldg(&a.row[v]);
-      const int e = s + max(__ldg(&a.row[v + 1]) - s, 0);
-      if (e > s) s_cnt[4 + L % 3] = 1;
-      for (int j = s; j < e; j++) {
-        const int u = __ldg(&a.col[j]);
-        if ((unsigned)u >= (unsigned)V) continue;
-        const unsigned bit = 1u << (u & 31);
-        if (S.bits[u >> 5] & bit) continue;
-        if (atomicOr(&S.bits[u >> 5], bit) & bit) continue;
-        a.dist[u] = (unsigned)L;
-        const int k = atomicAdd(oc, 1);
-        if (k < S.F)
-          out[k] = u;
-        else if (k - S.F < spill_cap)
-          out_sp[k - S.F] = u;
+    /* Claim N neighbours for level L and queue the new ones: N bit words
+     * read together, N claims together, one reservation. */
+    auto reach = [&](auto &u) {
+      constexpr int N = sizeof(u) / sizeof(u[0]);
+      unsigned w[N];
+      int found = 0;
+#pragma unroll
+      for (int q = 0; q < N; q++)
+        w[q] = (unsigned)u[q] < (unsigned)V ? bits[u[q] >> 5] : 0xffffffffu;
+#pragma unroll
+      for (int q = 0; q < N; q++) {
+        const unsigned bit = 1u << (u[q] & 31);
+        if (!(w[q] & bit)) w[q] = atomicOr(&bits[u[q] >> 5], bit);
+      }
+#pragma unroll
+      for (int q = 0; q < N; q++) {
+        w[q] = ~w[q] >> (u[q] & 31) & 1u; /* now: claimed here */
+        found += w[q];
+      }
+      if (found == 0) return;
+      int k = atomicAdd(&s_cnt[c1], found);
+#pragma unroll
+      for (int q = 0; q < N; q++) {
+        if (!w[q]) continue;
+        a.dist[u[q]] = (unsigned)L;
+        if (k < F)
+          wgm_bfs_dyn[out + k] = u[q];
+        else if (k - F < spill_cap)
+          spill[out_sp + k - F] = u[q];
         else
           s_cnt[3] = 1;
+        k++;
+      }
+    };
+    for (int i = threadIdx.x; i < n; i += T) {
+      const int v = i < F ? wgm_bfs_dyn[in + i] : __ldcg(&spill[in_sp + i - F]);
+      if (W) {
+        int u[W ? W : 1];
+#pragma unroll
+        for (int q = 0; q < W / 4; q++) {
+          const int4 r = __ldg(&ell[v * (W / 4) + q]);
+          u[4 * q] = r.x;
+          u[4 * q + 1] = r.y;
+          u[4 * q + 2] = r.z;
+          u[4 * q + 3] = r.w;
+        }
+        if (u[0] != WGM_BFS_PAD) s_cnt[4 + c0] = 1;
+        reach(u);
+      } else {
+        const int s = __ldg(&a.row[v]);
+        const int d = max(__ldg(&a.row[v + 1]) - s, 0);
+        if (d > 0) s_cnt[4 + c0] = 1;
+        for (int j = 0; j < d; j += 4) {
+          int u[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) u[q] = j + q < d ? __ldg(&a.col[s + j + q]) : -1;
+          reach(u);
+        }
       }
     }
     __syncthreads();
     /* the grid form queues no vertex without edges (it has no pieces): a
      * level that walked no edge is where its frontier was empty */
-    if (!s_cnt[4 + L % 3]) break;
+    if (!s_cnt[4 + c0]) break;
     L++;
+    int t = c0;
+    c0 = c1;
+    c1 = c2;
+    c2 = t;
+    t = in;
+    in = out;
+    out = t;
+    t = in_sp;
+    in_sp = out_sp;
+    out_sp = t;
   }
   if (threadIdx.x == 0 && a.levels_out) *a.levels_out = L;
 }

@@ -65,6 +65,8 @@ struct wgm_app {
    * first such run */
   int color_mode = 0;
   int bfs_mode = -1; /* Lonestar BFS: -1 automatic, 0 grid, 1 one CTA */
+  int *d_ell = nullptr; /* one-CTA BFS: ell_w columns per vertex (0: none) */
+  int ell_w = 0;
   /* colour in priority blocks (wgm_color_layout): order and row pointers on
    * the host, cb_blocks 0 when the graph is left to the rounds */
   std::vector<int> h_row, order;

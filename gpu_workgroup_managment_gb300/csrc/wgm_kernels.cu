@@ -229,29 +229,59 @@ cudaError_t wgm_launch_color_async(const wgm_launch &L, const wgm_color_args &a,
 /* Lonestar BFS on one CTA (wgm_bfs_cta): a plain one-CTA launch, no
  * discovery and no grid barrier.  Dynamic shared memory: the visited bits,
  * then the two frontier buffers of F vertices each. */
-__global__ void __launch_bounds__(1024) wgm_k_bfs_cta(wgm_lonestar_args a, int *spill,
-                                                      int spill_cap, int F, int *status) {
-  extern __shared__ unsigned wgm_bfs_cta_dyn[];
+template <int W>
+__global__ void __launch_bounds__(1024) wgm_k_bfs_cta(wgm_lonestar_args a, const int4 *ell,
+                                                      int *spill, int spill_cap, int F,
+                                                      int *status) {
   __shared__ int s_cnt[8];
-  wgm_bfs_cta_smem S;
-  S.bits = wgm_bfs_cta_dyn;
-  S.front = reinterpret_cast<int *>(wgm_bfs_cta_dyn + ((a.V + 31) >> 5));
-  S.F = F;
-  wgm_bfs_cta(a, spill, spill_cap, S, s_cnt);
+  wgm_bfs_cta<W>(a, ell, spill, spill_cap, F, s_cnt);
   if (threadIdx.x == 0 && s_cnt[3] && status) *status = WGM_DEV_OVERFLOW;
+}
+
+/* The columns as W per vertex (wgm_bfs_cta): a column equal to the padding is
+ * out of range and becomes another that is. */
+template <int W>
+__global__ void __launch_bounds__(256) wgm_k_bfs_ell(int V, const int *row, const int *col,
+                                                     int *ell) {
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < (long long)V * W;
+       i += gridDim.x * 256LL) {
+    const int v = (int)(i / W), q = (int)(i % W), s = row[v];
+    int u = WGM_BFS_PAD;
+    if (q < row[v + 1] - s) {
+      u = col[s + q];
+      if (u == WGM_BFS_PAD) u = -1;
+    }
+    ell[i] = u;
+  }
+}
+
+cudaError_t wgm_launch_bfs_ell(int W, int V, const int *row, const int *col, int *ell,
+                               cudaStream_t s) {
+  const int grid = (int)std::min<long long>(((long long)V * W + 255) / 256, 1216);
+  if (W == 4)
+    wgm_k_bfs_ell<4><<<grid, 256, 0, s>>>(V, row, col, ell);
+  else
+    wgm_k_bfs_ell<8><<<grid, 256, 0, s>>>(V, row, col, ell);
+  return cudaGetLastError();
 }
 
 size_t wgm_bfs_cta_smem_bytes(int V, int F) {
   return (size_t)((V + 31) / 32) * 4 + (size_t)2 * F * 4;
 }
 
-cudaError_t wgm_launch_bfs_cta(const wgm_lonestar_args &a, int *spill, int spill_cap, int F,
-                               int *status, int block, cudaStream_t s) {
-  const size_t smem = wgm_bfs_cta_smem_bytes(a.V, F);
-  cudaError_t e = cudaFuncSetAttribute(wgm_k_bfs_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+cudaError_t wgm_launch_bfs_cta(const wgm_lonestar_args &a, int W, const int *ell, int *spill,
+                               int spill_cap, int F, int *status, int block, cudaStream_t s) {
+  auto *k = W == 4 ? wgm_k_bfs_cta<4> : W == 8 ? wgm_k_bfs_cta<8> : wgm_k_bfs_cta<0>;
+  /* the limit is the kernel's, whoever launches it next: always the most */
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - 1024);
   if (e != cudaSuccess) return e;
-  wgm_k_bfs_cta<<<1, block, smem, s>>>(a, spill, spill_cap, F, status);
+  k<<<1, block, wgm_bfs_cta_smem_bytes(a.V, F), s>>>(a, reinterpret_cast<const int4 *>(ell), spill,
+                                                     spill_cap, F, status);
   return cudaGetLastError();
 }
 
