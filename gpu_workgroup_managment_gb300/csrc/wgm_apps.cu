@@ -150,7 +150,7 @@ static void wgm_app_free_buffers(wgm_app *a) {
                   a->d_oct_input, a->d_oct_second, a->d_oct_pools, a->d_oct_tree,
                   a->d_oct_ctr, a->d_oct_locks, a->d_oct_heads,
                   a->d_c4_board, a->d_c4_nodes, a->d_c4_pool, a->d_c4_locks,
-                  a->d_c4_heads, a->d_c4_ctr, a->d_ell, a->d_cb_ord, a->d_cb_colour,
+                  a->d_c4_heads, a->d_c4_ctr, a->d_ell, a->d_up_bits, a->d_up_cnt, a->d_up_wide, a->d_cb_ord, a->d_cb_colour,
                   a->d_cb_crank, a->d_cb_list, a->d_cb_hub, a->d_cb_cnt, a->d_hub_rank, a->d_hub_max, a->d_tcv, a->d_tcv4, a->d_cmax, a->d_cq,
                   a->d_cqctl};
   for (void *p : ptrs)
@@ -447,8 +447,38 @@ static int wgm_bfs_ell_layout(wgm_app *a, const int32_t *row_ptr) {
     if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   }
   cudaError_t e = wgm_launch_bfs_ell(W, a->V, a->d_row, a->d_col, a->d_ell, a->rt->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(a->rt->stream); /* runs may use another stream */
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   a->ell_w = W;
+  return WGM_OK;
+}
+
+/* In-edges of a large graph, for BFS from both sides (wgm_phase_bfs): where
+ * levels can hold WGM_BFS_UP_EDGES at all and rows are long enough that a
+ * vertex's first few in-edges stand for the rest. */
+static int wgm_bfs_up_layout(wgm_app *a, const int32_t *row_ptr) {
+  a->bfs_up = false;
+  const int V = a->V;
+  if (a->E < 2LL * WGM_BFS_UP_EDGES || a->E < 6LL * V) return WGM_OK;
+  const int64_t used = std::max(row_ptr[V - 1], row_ptr[V]);
+  cudaStream_t st = a->rt->stream;
+  cudaError_t e = cudaSuccess;
+  if (!a->d_trow) {
+    e = wgm_dmalloc(&a->d_trow, (size_t)V + 1);
+    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_tcol, (size_t)a->E);
+    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_up_bits, 3 * (((size_t)V + 31) / 32));
+    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_up_cnt, 3 * (size_t)WGM_LINE);
+    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_up_wide, (size_t)(a->E / WGM_BFS_UP_SCAN) + 2);
+  }
+  /* dist is free before a run: the in-degrees pass through it */
+  if (e == cudaSuccess)
+    e = wgm_launch_in_edges(V, used, a->d_row, a->d_col, a->d_trow, a->d_tcol, a->d_up_wide,
+                            (int *)a->d_out, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&a->up_nwide, a->d_up_wide, 4, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
+  a->bfs_up = true;
   return WGM_OK;
 }
 
@@ -474,6 +504,7 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
   }
   if (a->kind == WGM_APP_LONESTAR_BFS) {
     s = wgm_bfs_ell_layout(a, g->row_ptr);
+    if (s == WGM_OK) s = wgm_bfs_up_layout(a, g->row_ptr);
     if (s) return s;
   }
   if (a->kind == WGM_APP_PANNOTIA_COLOR) {
@@ -934,6 +965,18 @@ static cudaError_t wgm_app_enqueue(wgm_app *a, const wgm_launch &L, int grid, in
   if (wgm_app_fill_mega(a, &A) != WGM_OK) return cudaErrorInvalidValue;
   switch (a->kind) {
     case WGM_APP_LONESTAR_BFS:
+      if (a->bfs_up) {
+        wgm_bfs_up_args b;
+        b.trow = a->d_trow;
+        b.tcol = a->d_tcol;
+        b.bits = a->d_up_bits;
+        b.cnt = a->d_up_cnt;
+        b.wide = a->d_up_wide + 1;
+        b.nwide = a->up_nwide;
+        b.E = a->E;
+        return wgm_launch_bfs_two_way(L, A.ls, b, grid, block, stream);
+      }
+      [[fallthrough]];
     case WGM_APP_LONESTAR_SSSP:
       return wgm_launch_lonestar(a->kind == WGM_APP_LONESTAR_SSSP, L, A.ls, grid, block, stream);
     case WGM_APP_PANNOTIA_COLOR:
@@ -987,7 +1030,8 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
     if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
     hw = std::min(per_sm * a->rt->prop.multiProcessorCount, WGM_MAX_GROUPS);
   } else {
-    s = wgm_hw_bound_for(a->rt, wgm_kind_to_kernel(a->kind), block, &hw);
+    const int kid = a->bfs_up ? (int)WGM_K_BFS_TWO_WAY : wgm_kind_to_kernel(a->kind);
+    s = wgm_hw_bound_for(a->rt, kid, block, &hw);
   }
   if (s) return s;
   if (hw < 1) return WGM_ERR_INVALID;

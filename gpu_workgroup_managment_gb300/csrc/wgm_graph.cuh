@@ -121,6 +121,84 @@ __device__ __forceinline__ void wgm_two_seg_reduce(bool first, int v, float fv, 
   *f1 = fb;
 }
 
+/* First edge of each lane's row [e, end) that `hit` accepts (warp-collective;
+ * hit(valid, target, owner lane) is called by every lane).  Each lane first
+ * looks at four edges of its own row, then the warp shares the rows still
+ * open, 128 edges a step, split evenly among them.  At most `scan` edges of a
+ * row past its first four are looked at: `wide` tells that some are left.
+ * Returns whether the lane has its edge, at e; otherwise e is the first edge
+ * not looked at. */
+template <class Hit>
+__device__ __forceinline__ bool wgm_first_edge(const int *col, bool act, int &e, int end, int scan,
+                                               bool &wide, int *tab, Hit &&hit) {
+  const int lane = wgm_lane();
+  bool found = false;
+  {
+    int j[4];
+    bool h[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) j[q] = act && q < end - e ? __ldg(&col[e + q]) : -1;
+#pragma unroll
+    for (int q = 0; q < 4; q++) h[q] = hit(act && q < end - e, j[q], lane);
+    if (act) {
+      const int e0 = e;
+#pragma unroll
+      for (int q = 3; q >= 0; q--)
+        if (h[q]) {
+          found = true;
+          e = e0 + q;
+        }
+      if (!found) e += min(4, end - e);
+    }
+  }
+  wide = false;
+  const int elim = end - e > scan ? e + scan : end;
+  unsigned open = __ballot_sync(WGM_FULL, act && !found && e < end);
+  while (open) {
+    const int nopen = __popc(open);
+    const int ql = 31 - __clz(128 / nopen), quota = 1 << ql; /* 4 ... 128 */
+    const bool mine = (open >> lane) & 1u;
+    const int rank = __popc(open & wgm_lanemask_lt());
+    if (mine) tab[rank] = lane;
+    __syncwarp();
+    int j[4], own[4];
+    unsigned in = 0, h[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int sl = 32 * q + lane, oi = sl >> ql;
+      own[q] = oi < nopen ? tab[oi] : 0;
+      const int oe = __shfl_sync(WGM_FULL, e, own[q]), x = sl & (quota - 1);
+      const int lim = __shfl_sync(WGM_FULL, elim, own[q]);
+      const bool v = oi < nopen && x < lim - oe;
+      j[q] = v ? __ldg(&col[oe + x]) : -1;
+      in |= v ? 1u << q : 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      h[q] = __ballot_sync(WGM_FULL, hit((in >> q) & 1u, j[q], own[q]));
+    if (mine) {
+      /* this row's slots are [rank * quota, (rank + 1) * quota) */
+      const int s0 = rank << ql, w0 = s0 >> 5;
+      unsigned x = w0 == 0 ? h[0] : w0 == 1 ? h[1] : w0 == 2 ? h[2] : h[3];
+      int f = -1;
+      if (ql < 5) x = (x >> (s0 & 31)) & ((1u << quota) - 1u);
+      if (x) f = __ffs(x) - 1;
+      if (ql >= 6 && f < 0) { /* 64 or 128 slots */
+        const unsigned x1 = w0 == 0 ? h[1] : h[3];
+        if (x1) f = 31 + __ffs(x1);
+        if (ql == 7 && f < 0 && h[2]) f = 63 + __ffs(h[2]);
+        if (ql == 7 && f < 0 && h[3]) f = 95 + __ffs(h[3]);
+      }
+      found = f >= 0;
+      e = found ? e + f : e + min(quota, elim - e);
+      wide = !found && e == elim && elim < end;
+    }
+    __syncwarp();
+    open = __ballot_sync(WGM_FULL, mine && !found && e < elim);
+  }
+  return found;
+}
+
 /* ------------------------------------------------------------------------ */
 /* Lonestar BFS / SSSP                                                       */
 /* ------------------------------------------------------------------------ */
@@ -728,6 +806,189 @@ static __device__ int wgm_phase_lonestar(const wgm_launch &Lc, wgm_cta *c,
   *next_target = 1;
   *next_round = Lv + 1;
   return 1;
+}
+
+/* Lonestar BFS in two directions (standalone runs of large graphs).  A level
+ * whose worklist holds a good part of the edges walks every one of them for
+ * the few vertices still unreached (RMAT-20: 25 M edges for 0.2 M vertices);
+ * such a level is run from the other side: each unreached vertex looks
+ * through its in-edges until it meets a reached one (0.2-2 M looks).  An
+ * unreached vertex's reached in-neighbours are all of the level before, or
+ * it would have been reached sooner, so one bit per vertex answers a look
+ * (128 KB on RMAT-20: served by the L1).  Levels and their count are the
+ * worklist's: the vertex takes the running level, and a level whose new
+ * vertices have no out-edge is the last.
+ *
+ * Phases: (1,L) the worklist's level L, or, when its pieces hold more than
+ * WGM_BFS_UP_EDGES edges and a twentieth of the graph, the bits of the
+ * reached vertices instead and (2,L); (2,L) and (3,L) level L from the
+ * unreached side, (3,L) after the last one's verdict: nothing new to walk -
+ * done; fewer than V/64 new - the worklist again, from the distances, at
+ * (1,L).  RMAT-20: 0.39 -> 0.13 ms, most of it the first such level (0.6 M
+ * vertices with two looks each: the round trips row, in-edge, bit). */
+#define WGM_BFS_UP_EDGES (1 << 20)
+#define WGM_BFS_UP_SCAN 4096 /* in-edges of a vertex that one warp looks at */
+struct wgm_bfs_up_args {
+  const int *trow, *tcol; /* in-edges */
+  unsigned *bits;         /* [3][ceil(V/32)] reached, by level parity; without in-edges
+                             (never looked at, but no answer to a look either) */
+  int *cnt;               /* [3 lines] by level mod 3: new vertices, any of them with
+                             out-edges */
+  const int *wide;        /* vertices of more than WGM_BFS_UP_SCAN in-edges */
+  int nwide;
+  long long E;
+};
+
+/* Level L from the unreached side. */
+__device__ __forceinline__ void wgm_bfs_up_level(const wgm_cta *c, const wgm_lonestar_args &a,
+                                                 const wgm_bfs_up_args &b, int L,
+                                                 wgm_warp_smem *sm) {
+  __shared__ int s_new, s_walk;
+  const wgm_split s(c);
+  const int V = a.V, lane = s.lane, nword = (V + 31) >> 5;
+  const unsigned *cur = b.bits + (size_t)(L & 1) * nword;
+  unsigned *nxt = b.bits + (size_t)((L + 1) & 1) * nword;
+  const unsigned *none = b.bits + 2 * (size_t)nword;
+  int *cnt = &b.cnt[(L % 3) * WGM_LINE];
+  if (threadIdx.x == 0) s_new = s_walk = 0;
+  __syncthreads();
+  auto reached = [&](bool valid, int j, int) {
+    return valid && (__ldca(&cur[j >> 5]) >> (j & 31) & 1u);
+  };
+  auto take = [&](int v) { /* v is new: its distance, and whether it can go on */
+    a.dist[v] = (unsigned)L;
+    if (!s_walk && wgm_ls_degree(a.row, v) > 0) s_walk = 1;
+  };
+  int fresh = 0;
+  for (int k = s.gw; k < nword; k += s.NW) {
+    const unsigned m = __ldcg(&cur[k]), done = m | __ldcg(&none[k]);
+    if (done == WGM_FULL) {
+      if (lane == 0 && __ldcg(&nxt[k]) != m) atomicOr(&nxt[k], m);
+      continue;
+    }
+    const int v = k * 32 + lane;
+    const bool act = !((done >> lane) & 1u);
+    int e = 0, end = 0;
+    if (act) {
+      e = __ldg(&b.trow[v]);
+      end = __ldg(&b.trow[v + 1]);
+    }
+    bool wide; /* the whole grid looks on, below */
+    const bool f = wgm_first_edge(b.tcol, act, e, end, WGM_BFS_UP_SCAN, wide, sm->tab[s.warp],
+                                  reached);
+    if (f) take(v);
+    const unsigned nw = __ballot_sync(WGM_FULL, f);
+    fresh += __popc(nw);
+    if (lane == 0) atomicOr(&nxt[k], m | nw);
+  }
+  /* the rest of very long rows: S warps each, until one has its edge */
+  if (b.nwide > 0) {
+    const int S = max(1, s.NW / b.nwide), sub = s.gw % S, per = max(1, s.NW / S);
+    for (int h = s.gw / S; h < b.nwide && s.gw < per * S; h += per) {
+      const int v = __ldg(&b.wide[h]);
+      if (__ldcg(&cur[v >> 5]) >> (v & 31) & 1u) continue;
+      const int end = __ldg(&b.trow[v + 1]);
+      bool f = false;
+      for (long long x = (long long)__ldg(&b.trow[v]) + WGM_BFS_UP_SCAN + 128LL * sub;
+           x < end && !f; x += 128LL * S) {
+        if (__ldcg(&nxt[v >> 5]) >> (v & 31) & 1u) break; /* another warp has it */
+        int j[4];
+        bool h4 = false;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const bool in = x + 32 * q + lane < end;
+          j[q] = in ? __ldg(&b.tcol[x + 32 * q + lane]) : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) h4 |= reached(j[q] >= 0, j[q], lane);
+        f = __any_sync(WGM_FULL, h4);
+      }
+      if (f && lane == 0) {
+        const unsigned bit = 1u << (v & 31);
+        if (!(atomicOr(&nxt[v >> 5], bit) & bit)) {
+          take(v);
+          fresh++;
+        }
+      }
+      fresh = __shfl_sync(WGM_FULL, fresh, 0);
+    }
+  }
+  if (lane == 0 && fresh) atomicAdd(&s_new, fresh);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_new) {
+    atomicAdd(&cnt[0], s_new);
+    if (s_walk) cnt[1] = 1;
+  }
+}
+
+static __device__ int wgm_phase_bfs(const wgm_launch &Lc, wgm_cta *c, const wgm_lonestar_args &a,
+                                    const wgm_bfs_up_args &b, wgm_warp_smem *sm, wgm_step cur,
+                                    wgm_step *nxt) {
+  const wgm_split s(c);
+  const int V = a.V, L = cur.round;
+  if (cur.target == 1) {
+    const long long n = __ldcg(&a.cnt[(L % 3) * WGM_LINE]);
+    const long long edges = n * a.piece;
+    if (n <= a.cap && edges > WGM_BFS_UP_EDGES && edges > b.E / 20) {
+      const int nword = (V + 31) >> 5;
+      for (int k = s.gw; k < nword; k += s.NW) {
+        const int v = k * 32 + s.lane;
+        bool r = false, none = true;
+        if (v < V) {
+          r = __ldcg(&a.dist[v]) != WGM_LONESTAR_INF;
+          none = __ldg(&b.trow[v + 1]) == __ldg(&b.trow[v]);
+        }
+        const unsigned m = __ballot_sync(WGM_FULL, r), z = __ballot_sync(WGM_FULL, none);
+        if (s.lane < 3) b.bits[(size_t)s.lane * nword + k] = s.lane < 2 ? m : z;
+      }
+      if (c->id == 0 && threadIdx.x < 3) {
+        b.cnt[threadIdx.x * WGM_LINE] = 0;
+        b.cnt[threadIdx.x * WGM_LINE + 1] = 0;
+      }
+      *nxt = {2, L};
+      return WGM_PHASE_NEXT;
+    }
+  }
+  if (cur.target < 2)
+    return wgm_phase_lonestar<false>(Lc, c, a, sm, cur.target, cur.round, &nxt->target,
+                                     &nxt->round);
+  if (cur.target == 3) {
+    const int2 r = __ldcg(reinterpret_cast<const int2 *>(&b.cnt[((L + 2) % 3) * WGM_LINE]));
+    if (r.y == 0) {
+      if (c->id == 0 && threadIdx.x == 0 && a.levels_out) *a.levels_out = L;
+      return WGM_PHASE_DONE;
+    }
+    if (r.x < V / 64) {
+      /* few new vertices: their pieces as level L's worklist */
+      bool ok = true;
+      wgm_ls_out o;
+      o.counter = &a.cnt[(L % 3) * WGM_LINE];
+      o.o_start = a.wl_start + (size_t)(L & 1) * a.cap;
+      o.o_cnt = a.wl_cnt + (size_t)(L & 1) * a.cap;
+      o.o_u = a.wl_u ? a.wl_u + (size_t)(L & 1) * a.cap : nullptr;
+      o.cap = a.cap;
+      for (int k = s.gw * 32; k < V; k += s.NW * 32) {
+        const int v = k + s.lane;
+        const bool f = v < V && __ldcg(&a.dist[v]) == (unsigned)(L - 1);
+        ok &= wgm_out_push_vertices(a.row, a.piece, f, v, o);
+      }
+      if (!ok) wgm_fail(Lc, WGM_DEV_OVERFLOW, WGM_SITE_QUEUE, L);
+      *nxt = {1, L};
+      return WGM_PHASE_NEXT;
+    }
+  }
+  if (L > V + 2) { /* only a corrupt input gets here */
+    wgm_fail(Lc, WGM_DEV_BAD_INPUT, WGM_SITE_QUEUE, L);
+    return WGM_PHASE_DONE;
+  }
+  /* the worklist's counters, last read before (2,L): empty for its return */
+  if (c->id == 0 && threadIdx.x < 3) {
+    a.cnt[threadIdx.x * WGM_LINE] = 0;
+    if (threadIdx.x < 2) b.cnt[((L + 1) % 3) * WGM_LINE + threadIdx.x] = 0;
+  }
+  wgm_bfs_up_level(c, a, b, L, sm);
+  *nxt = {3, L + 1};
+  return WGM_PHASE_NEXT;
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1707,69 +1968,12 @@ __device__ __forceinline__ bool wgm_mis_visit(const wgm_launch &Lc, const wgm_mi
     e = r == 1 ? start : __ldcg(&a.ptr[i]);
   }
   const int e0 = e;
-  bool blocked = false;
-  if (act) {
-    int j[4];
-    bool hit[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) j[q] = q < end - e ? __ldg(&a.col[e + q]) : -1;
-#pragma unroll
-    for (int q = 0; q < 4; q++) hit[q] = j[q] >= 0 && wgm_mis_blocks(a, j[q], v, r);
-#pragma unroll
-    for (int q = 3; q >= 0; q--)
-      if (hit[q]) {
-        blocked = true;
-        e = e0 + q;
-      }
-    if (!blocked) e += min(4, end - e);
-  }
-  /* the rest of the longer rows, by the whole warp: a step looks at 128
-   * edges, shared evenly among the vertices still open */
-  bool wide = false;
-  const int elim = end - e > a.scan ? e + a.scan : end;
-  unsigned open = __ballot_sync(WGM_FULL, act && !blocked && e < end);
-  while (open) {
-    const int nopen = __popc(open);
-    const int ql = 31 - __clz(128 / nopen), quota = 1 << ql; /* 4 ... 128 */
-    const bool mine = (open >> lane) & 1u;
-    const int rank = __popc(open & wgm_lanemask_lt());
-    if (mine) tab[rank] = lane;
-    __syncwarp();
-    int j[4], own[4];
-    unsigned hit[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int sl = 32 * q + lane, oi = sl >> ql;
-      own[q] = oi < nopen ? tab[oi] : 0;
-      const int oe = __shfl_sync(WGM_FULL, e, own[q]), x = sl & (quota - 1);
-      const int lim = __shfl_sync(WGM_FULL, elim, own[q]);
-      j[q] = oi < nopen && x < lim - oe ? __ldg(&a.col[oe + x]) : -1;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const float ov = __shfl_sync(WGM_FULL, v, own[q]);
-      hit[q] = __ballot_sync(WGM_FULL, j[q] >= 0 && wgm_mis_blocks(a, j[q], ov, r));
-    }
-    if (mine) {
-      /* this vertex's slots are [rank * quota, (rank + 1) * quota) */
-      const int s0 = rank << ql, w0 = s0 >> 5;
-      unsigned h = w0 == 0 ? hit[0] : w0 == 1 ? hit[1] : w0 == 2 ? hit[2] : hit[3];
-      int f = -1;
-      if (ql < 5) h = (h >> (s0 & 31)) & ((1u << quota) - 1u);
-      if (h) f = __ffs(h) - 1;
-      if (ql >= 6 && f < 0) { /* 64 or 128 slots */
-        const unsigned h1 = w0 == 0 ? hit[1] : hit[3];
-        if (h1) f = 31 + __ffs(h1);
-        if (ql == 7 && f < 0 && hit[2]) f = 63 + __ffs(hit[2]);
-        if (ql == 7 && f < 0 && hit[3]) f = 95 + __ffs(hit[3]);
-      }
-      blocked = f >= 0;
-      e = blocked ? e + f : e + min(quota, elim - e);
-      wide = !blocked && e == elim && elim < end;
-    }
-    __syncwarp();
-    open = __ballot_sync(WGM_FULL, mine && !blocked && e < elim);
-  }
+  bool wide;
+  const bool blocked = wgm_first_edge(a.col, act, e, end, a.scan, wide, tab,
+                                      [&](bool valid, int j, int owner) {
+                                        const float ov = __shfl_sync(WGM_FULL, v, owner);
+                                        return valid && wgm_mis_blocks(a, j, ov, r);
+                                      });
   bool join = act && !blocked && !wide && v < BIG;
   if (join) {
     a.s_array[i] = 2;

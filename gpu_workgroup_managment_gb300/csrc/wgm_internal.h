@@ -65,6 +65,12 @@ struct wgm_app {
    * first such run */
   int color_mode = 0;
   int bfs_mode = -1; /* Lonestar BFS: -1 automatic, 0 grid, 1 one CTA */
+  /* BFS from both sides: reached bits, counters, vertices of very many in-edges
+   * (the in-edges are d_trow, d_tcol); bfs_up: the graph has them */
+  bool bfs_up = false;
+  unsigned *d_up_bits = nullptr;
+  int *d_up_cnt = nullptr, *d_up_wide = nullptr;
+  int up_nwide = 0;
   int *d_ell = nullptr; /* one-CTA BFS: ell_w columns per vertex (0: none) */
   int ell_w = 0;
   /* colour in priority blocks (wgm_color_layout): order and row pointers on

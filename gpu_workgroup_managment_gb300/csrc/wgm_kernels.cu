@@ -46,6 +46,118 @@ __global__ void __launch_bounds__(1024) wgm_k_bfs(wgm_launch L, wgm_lonestar_arg
   WGM_PERSISTENT_EPILOGUE
 }
 
+/* The same where in-edges are at hand (wgm_phase_bfs). */
+__global__ void __launch_bounds__(1024) wgm_k_bfs_two_way(wgm_launch L, wgm_lonestar_args a,
+                                                          wgm_bfs_up_args b) {
+  WGM_PERSISTENT_PROLOGUE
+  WGM_DRIVE(wgm_phase_bfs(L, &c, a, b, &sm, cur, nxt));
+  WGM_PERSISTENT_EPILOGUE
+}
+
+cudaError_t wgm_launch_bfs_two_way(const wgm_launch &L, const wgm_lonestar_args &a,
+                                   const wgm_bfs_up_args &b, int grid, int block, cudaStream_t s) {
+  wgm_k_bfs_two_way<<<grid, block, 0, s>>>(L, a, b);
+  return cudaGetLastError();
+}
+
+/* In-edges on the device: counts, their exclusive prefix, then the places
+ * taken (at).  Out-of-range columns have no place. */
+__global__ void __launch_bounds__(256) wgm_k_in_count(int V, long long E, const int *col, int *deg) {
+  for (long long e = blockIdx.x * 256LL + threadIdx.x; e < E; e += gridDim.x * 256LL) {
+    const int u = col[e];
+    if ((unsigned)u < (unsigned)V) atomicAdd(&deg[u], 1);
+  }
+}
+/* Exclusive prefix of deg[] in blocks of 8192: the blocks' sums, their
+ * prefix, then every place.  deg is zeroed for the places taken; vertices of
+ * more than WGM_BFS_UP_SCAN in-edges are listed (wide[0]: how many, then
+ * they). */
+#define WGM_IN_BLOCK 8192
+__device__ __forceinline__ int wgm_cta_scan(int x, int *warp_sum, int *total) {
+  const int lane = wgm_lane(), warp = threadIdx.x >> 5;
+  const int incl = wgm_warp_incl_scan(x);
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  const int w = wgm_warp_incl_scan(lane < (int)(blockDim.x >> 5) ? warp_sum[lane] : 0);
+  const int before = __shfl_sync(WGM_FULL, w, max(warp - 1, 0));
+  *total = __shfl_sync(WGM_FULL, w, 31);
+  __syncthreads();
+  return incl - x + (warp ? before : 0);
+}
+__global__ void __launch_bounds__(1024) wgm_k_in_sums(int V, const int *deg, int *sums) {
+  __shared__ int warp_sum[32];
+  int x = 0, total;
+  for (int q = 0; q < 8; q++) {
+    const long long i = (long long)blockIdx.x * WGM_IN_BLOCK + q * 1024 + threadIdx.x;
+    x += i < V ? deg[i] : 0;
+  }
+  wgm_cta_scan(x, warp_sum, &total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(1024) wgm_k_in_bases(int n, int *sums, int *last) {
+  __shared__ int warp_sum[32];
+  int base = 0;
+  for (int i0 = 0; i0 < n; i0 += 1024) {
+    const int i = i0 + threadIdx.x, x = i < n ? sums[i] : 0;
+    int total;
+    const int p = wgm_cta_scan(x, warp_sum, &total);
+    if (i < n) sums[i] = base + p;
+    base += total;
+  }
+  if (threadIdx.x == 0) *last = base;
+}
+__global__ void __launch_bounds__(1024) wgm_k_in_places(int V, int *deg, const int *bases,
+                                                        int *trow, int *wide) {
+  __shared__ int warp_sum[32];
+  int base = bases[blockIdx.x];
+  for (int q = 0; q < 8; q++) {
+    const long long i = (long long)blockIdx.x * WGM_IN_BLOCK + q * 1024 + threadIdx.x;
+    const int x = i < V ? deg[i] : 0;
+    int total;
+    const int p = wgm_cta_scan(x, warp_sum, &total);
+    if (i < V) {
+      trow[i] = base + p;
+      deg[i] = 0;
+      if (x > WGM_BFS_UP_SCAN) wide[1 + atomicAdd(wide, 1)] = (int)i;
+    }
+    base += total;
+  }
+}
+__global__ void __launch_bounds__(256) wgm_k_in_fill(int V, const int *row, const int *col,
+                                                     const int *trow, int *at, int *tcol) {
+  const int nw = gridDim.x * (blockDim.x >> 5), lane = wgm_lane();
+  for (int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < (V + 31) / 32; k += nw) {
+    const int v = 32 * k + lane;
+    const int s = v < V ? row[v] : 0, d = v < V ? max(row[v + 1] - s, 0) : 0;
+    const int incl = wgm_warp_incl_scan(d), total = __shfl_sync(WGM_FULL, incl, 31);
+    const int off = incl - d;
+    for (int w = 0; w < total; w += 32) {
+      const int sl = w + lane, own = wgm_owner_of(off, min(sl, total - 1));
+      const int e = __shfl_sync(WGM_FULL, s - off, own) + sl;
+      if (sl >= total) continue;
+      const int u = col[e];
+      if ((unsigned)u < (unsigned)V) tcol[trow[u] + atomicAdd(&at[u], 1)] = 32 * k + own;
+    }
+  }
+}
+
+/* trow [V+1], tcol [E], wide [E / WGM_BFS_UP_SCAN + 2], scratch [V] from the
+ * out-edges' first E columns. */
+cudaError_t wgm_launch_in_edges(int V, long long E, const int *row, const int *col, int *trow,
+                                int *tcol, int *wide, int *scratch, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(scratch, 0, (size_t)V * 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(wide, 0, 4, s);
+  if (e != cudaSuccess) return e;
+  wgm_k_in_count<<<1216, 256, 0, s>>>(V, E, col, scratch);
+  const int nb = (V + WGM_IN_BLOCK - 1) / WGM_IN_BLOCK;
+  int *sums = tcol; /* filled last */
+  wgm_k_in_sums<<<nb, 1024, 0, s>>>(V, scratch, sums);
+  wgm_k_in_bases<<<1, 1024, 0, s>>>(nb, sums, trow + V);
+  wgm_k_in_places<<<nb, 1024, 0, s>>>(V, scratch, sums, trow, wide);
+  wgm_k_in_fill<<<1216, 256, 0, s>>>(V, row, col, trow, scratch, tcol);
+  return cudaGetLastError();
+}
+
 __global__ void __launch_bounds__(1024) wgm_k_sssp(wgm_launch L, wgm_lonestar_args a) {
   WGM_PERSISTENT_PROLOGUE
   WGM_DRIVE(wgm_lonestar_step<true>(L, &c, a, &sm, cur, nxt));
@@ -372,6 +484,7 @@ const void *wgm_kernel_fn(int kid) {
     case WGM_K_BFS: return (const void *)wgm_k_bfs;
     case WGM_K_SSSP: return (const void *)wgm_k_sssp;
     case WGM_K_COLOR: return (const void *)wgm_k_color;
+    case WGM_K_BFS_TWO_WAY: return (const void *)wgm_k_bfs_two_way;
     case WGM_K_MIS: return (const void *)wgm_k_mis;
     case WGM_K_PSSSP: return (const void *)wgm_k_psssp;
     case WGM_K_PAGERANK: return (const void *)wgm_k_pagerank;

@@ -27,6 +27,7 @@ enum wgm_kernel_id {
   WGM_K_OCTREE,
   WGM_K_C4,
   WGM_K_BC,
+  WGM_K_BFS_TWO_WAY,
   WGM_K_COUNT
 };
 
@@ -51,6 +52,10 @@ cudaError_t wgm_launch_lonestar(bool sssp, const wgm_launch &L, const wgm_lonest
                                 int grid, int block, cudaStream_t s);
 cudaError_t wgm_launch_color(const wgm_launch &L, const wgm_color_args &a, int grid, int block,
                              cudaStream_t s);
+cudaError_t wgm_launch_bfs_two_way(const wgm_launch &L, const wgm_lonestar_args &a,
+                                   const wgm_bfs_up_args &b, int grid, int block, cudaStream_t s);
+cudaError_t wgm_launch_in_edges(int V, long long E, const int *row, const int *col, int *trow,
+                                int *tcol, int *wide, int *scratch, cudaStream_t s);
 cudaError_t wgm_launch_color_blocks(const wgm_launch &L, const wgm_color_args &a,
                                     const wgm_color_blocks_args &q, int grid, int block,
                                     cudaStream_t s);
