@@ -73,7 +73,7 @@ static bool wgm_needs_weights(int kind) {
 }
 /* (colour's hubs follow its priorities: wgm_color_layout) */
 static bool wgm_uses_static_hubs(int kind) {
-  return kind == WGM_APP_PANNOTIA_SSSP || kind == WGM_APP_PAGERANK;
+  return kind == WGM_APP_PANNOTIA_SSSP;
 }
 
 /* Reject graphs the kernels cannot walk safely.  The Lonestar loader quirk
@@ -145,7 +145,8 @@ static void wgm_app_free_buffers(wgm_app *a) {
   void *ptrs[] = {a->d_row,     a->d_col,       a->d_wt,      a->d_node_value, a->d_out,
                   a->d_wl_start, a->d_wl_cnt,   a->d_wl_u,
                   a->d_cnt,       a->d_stamp,   a->d_stop,
-                  a->d_mis_word, a->d_mis_mask, a->d_mis_wide, a->d_contrib,   a->d_dang,    a->d_hub_sum,    a->d_rounds,
+                  a->d_mis_word, a->d_mis_mask, a->d_mis_wide, a->d_contrib,   a->d_dang,    a->d_pr_order, a->d_pr_row,
+                  a->d_pr_col,  a->d_pr_parts, a->d_rounds,
                   a->hubs.ids,  a->hubs.prefix, a->hubs.wmap, a->d_trow, a->d_tcol,
                   a->d_oct_input, a->d_oct_second, a->d_oct_pools, a->d_oct_tree,
                   a->d_oct_ctr, a->d_oct_locks, a->d_oct_heads,
@@ -198,12 +199,6 @@ static int wgm_upload_hubs(wgm_app *a, const int32_t *row_ptr, const int *order)
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   a->hubs.H = (int)ids.size();
   a->hubs.total = prefix.back();
-  if (a->kind == WGM_APP_PAGERANK) {
-    if (a->d_hub_sum) cudaFree(a->d_hub_sum);
-    a->d_hub_sum = nullptr;
-    e = wgm_dmalloc(&a->d_hub_sum, (size_t)a->hubs.H);
-    if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
-  }
   return WGM_OK;
 }
 
@@ -482,6 +477,70 @@ static int wgm_bfs_up_layout(wgm_app *a, const int32_t *row_ptr) {
   return WGM_OK;
 }
 
+/* Edges a group at least (RMAT-14: 0.152 ms with 2048 to 8192, 0.28 with
+ * 16384), and the contributions kept in shared memory at most: the rest of
+ * the SM's 256 KB is the L1 of the columns and of the colder contributions.
+ * RMAT-22: 16384 5.78 ms, 32768 5.20, 40960 5.10, 45056 5.44, 55296 7.7. */
+#define WGM_PR_EDGES 4096
+#define WGM_PR_CACHED 40960
+/* PageRank's layout (wgm_pr_args): vertices by falling degree (a counting
+ * sort, equal degrees by number), rows and columns renumbered on the device. */
+static int wgm_pr_layout(wgm_app *a, const int32_t *row_ptr) {
+  const int V = a->V;
+  int most = 0;
+  for (int v = 0; v < V; v++) most = std::max(most, row_ptr[v + 1] - row_ptr[v]);
+  std::vector<int> at((size_t)most + 2, 0), order((size_t)V), prow((size_t)V + 1);
+  for (int v = 0; v < V; v++) at[most - (row_ptr[v + 1] - row_ptr[v]) + 1]++;
+  /* rows of more than x edges: at[most - x] once summed */
+  for (int x = 0; x <= most; x++) at[x + 1] += at[x];
+  auto above = [&](int x) { return x >= most ? 0 : at[most - x]; };
+  a->pr_rows = above(0);
+  /* parts of wide rows: 256 edges (one step of a warp) while the graph has
+   * fewer than that for every warp, up to 2048 */
+  a->pr_part_edges = 256;
+  while (a->pr_part_edges < 2048 &&
+         a->E / (32LL * a->rt->prop.multiProcessorCount) > 4LL * a->pr_part_edges)
+    a->pr_part_edges *= 2;
+  a->pr_wide = above(a->pr_part_edges);
+  a->pr_bin_row[0] = a->pr_wide;
+  for (int b = 1; b < WGM_PR_BINS; b++) a->pr_bin_row[b] = above(8 * (32 >> b));
+  a->pr_bin_row[WGM_PR_BINS] = a->pr_rows;
+  a->pr_bin_task[0] = 0;
+  for (int b = 0; b < WGM_PR_BINS; b++)
+    a->pr_bin_task[b + 1] =
+        a->pr_bin_task[b] + ((a->pr_bin_row[b + 1] - a->pr_bin_row[b] + (1 << b) - 1) >> b);
+  for (int v = 0; v < V; v++) order[at[most - (row_ptr[v + 1] - row_ptr[v])]++] = v;
+  prow[0] = 0;
+  for (int k = 0; k < a->pr_rows; k++)
+    prow[k + 1] = prow[k] + (row_ptr[order[k] + 1] - row_ptr[order[k]]);
+  /* parts of the wide rows: {part_row [parts], row_part [wide+1]} */
+  std::vector<int> parts, row_part(1, 0);
+  for (int k = 0; k < a->pr_wide; k++) {
+    const int m = (prow[k + 1] - prow[k] + a->pr_part_edges - 1) / a->pr_part_edges;
+    parts.insert(parts.end(), (size_t)m, k);
+    row_part.push_back((int)parts.size());
+  }
+  a->pr_parts = (int)parts.size();
+  parts.insert(parts.end(), row_part.begin(), row_part.end());
+  cudaStream_t st = a->rt->stream;
+  if (a->d_pr_parts) cudaFree(a->d_pr_parts);
+  a->d_pr_parts = nullptr;
+  cudaError_t e = wgm_dmalloc(&a->d_pr_parts, 2 * (size_t)a->pr_parts + 2 * (size_t)a->pr_wide + 1);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(a->d_pr_parts, parts.data(), parts.size() * 4, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(a->d_pr_order, order.data(), (size_t)V * 4,
+                                  cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(a->d_pr_row, prow.data(), ((size_t)a->pr_rows + 1) * 4,
+                        cudaMemcpyHostToDevice, st);
+  /* the ranks pass through the result buffer */
+  if (e == cudaSuccess)
+    e = wgm_launch_pr_layout(V, a->pr_rows, a->d_row, a->d_col, a->d_pr_order, (int *)a->d_out,
+                             a->d_pr_row, a->d_pr_col, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  return e == cudaSuccess ? WGM_OK : wgm_cuda_fail(a->rt, e);
+}
+
 extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
   if (!a || a->kind == WGM_APP_OCTREE || a->kind == WGM_APP_CONNECT_FOUR ||
       a->kind == WGM_APP_PLUGIN)
@@ -516,14 +575,11 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
     s = wgm_upload_transpose(a, g);
     if (s) return s;
   }
-  if (a->kind == WGM_APP_PAGERANK) {
-    /* Initial dangling mass: every vertex starts at 1/V. */
-    int64_t zero = 0;
-    for (int v = 0; v < a->V; v++) zero += (g->row_ptr[v + 1] == g->row_ptr[v]);
-    a->dang0 = (float)((double)zero / (double)a->V);
-  }
+  if (a->kind == WGM_APP_PAGERANK) return wgm_pr_layout(a, g->row_ptr);
   return WGM_OK;
 }
+
+static size_t wgm_pr_stride(int V) { return ((size_t)V + 3) & ~(size_t)3; }
 
 extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g,
                               wgm_app **out) {
@@ -601,8 +657,12 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
     case WGM_APP_PAGERANK:
       a->out_bytes = V * 4;
       if (e == cudaSuccess) e = cudaMalloc(&a->d_out, a->out_bytes);
-      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_contrib, 2 * V);
+      /* contrib: two rows of V rounded up to whole 16-byte words, and one more */
+      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_contrib, 2 * wgm_pr_stride(a->V));
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_dang, 3 * WGM_LINE);
+      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_pr_order, V);
+      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_pr_row, V + 1);
+      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_pr_col, E);
       break;
     case WGM_APP_PANNOTIA_BC:
       /* bc (out), dist, rho and sigma, the level lists and their starts */
@@ -886,17 +946,27 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
     case WGM_APP_PAGERANK: {
       wgm_pr_args &x = A->pr;
       x.V = a->V;
-      x.row = a->d_row;
-      x.col = a->d_col;
+      x.rows = a->pr_rows;
+      x.prow = a->d_pr_row;
+      x.pcol = a->d_pr_col;
+      x.order = a->d_pr_order;
       x.pr = (float *)a->d_out;
       x.contrib = a->d_contrib;
+      x.stride = wgm_pr_stride(a->V);
       x.dang = a->d_dang;
-      x.hub_sum = a->d_hub_sum;
-      x.hubs = wgm_hubs_view(a);
-      x.hub_threshold = a->hub_threshold;
+      x.wide = a->pr_wide;
+      x.parts = a->pr_parts;
+      x.part_edges = a->pr_part_edges;
+      x.part_row = a->d_pr_parts;
+      x.row_part = x.part_row + a->pr_parts;
+      x.part = (float *)(a->d_pr_parts + a->pr_parts + a->pr_wide + 1);
+      x.part_done = a->d_pr_parts + 2 * (size_t)a->pr_parts + a->pr_wide + 1;
+      std::copy(a->pr_bin_row, a->pr_bin_row + WGM_PR_BINS + 1, x.bin_row);
+      std::copy(a->pr_bin_task, a->pr_bin_task + WGM_PR_BINS + 1, x.bin_task);
+      x.cached = 0;
       x.iterations = a->iterations;
       x.damping = a->damping;
-      x.dang0 = a->dang0;
+      x.dangling = (float)(a->V - a->pr_rows);
       return WGM_OK;
     }
   }
@@ -992,8 +1062,19 @@ static cudaError_t wgm_app_enqueue(wgm_app *a, const wgm_launch &L, int grid, in
       return wgm_launch_mis(L, A.mis, grid, block, stream);
     case WGM_APP_PANNOTIA_SSSP:
       return wgm_launch_psssp(L, A.psssp, grid, block, stream);
-    case WGM_APP_PAGERANK:
+    case WGM_APP_PAGERANK: {
+      /* the contributions read most often, in what shared memory the groups
+       * of an SM leave one another */
+      const int sms = a->rt->prop.multiProcessorCount, per_sm = (grid + sms - 1) / sms;
+      if (a->pr_smem_block != block || a->pr_smem_per_sm != per_sm) {
+        cudaError_t e = wgm_pagerank_smem(block, per_sm, &a->pr_smem);
+        if (e != cudaSuccess) return e;
+        a->pr_smem_block = block;
+        a->pr_smem_per_sm = per_sm;
+      }
+      A.pr.cached = std::min({(a->pr_rows + 3) & ~3, a->pr_smem / 4, WGM_PR_CACHED});
       return wgm_launch_pagerank(L, A.pr, grid, block, stream);
+    }
     case WGM_APP_OCTREE:
       return wgm_launch_octree(L, A.oct, grid, block, stream);
     case WGM_APP_CONNECT_FOUR:
@@ -1063,6 +1144,14 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
     const long long want = ((long long)a->V / b + sms - 1) / sms * sms;
     *grid = (int)std::min<long long>(hw, std::max(sms, want));
   }
+  /* PageRank by default (block: wgm_app_block): one group per SM, whose
+   * shared memory holds the contributions read most often; fewer for small
+   * graphs, WGM_PR_EDGES edges each, since an iteration ends in a barrier. */
+  if (num_wgs <= 0 && a->kind == WGM_APP_PAGERANK) {
+    const long long sms = a->rt->prop.multiProcessorCount;
+    *grid = (int)std::min<long long>(std::min<long long>(hw, sms),
+                                     std::max<long long>(1, a->E / WGM_PR_EDGES));
+  }
   /* Pannotia SSSP by default: 1024 threads per SM (four 256-thread CTAs of
    * the six that fit), more only for graphs of more than one 256-thread CTA
    * per 32768 edges: on grids and RMAT graphs up to 7.6M edges four CTAs
@@ -1076,6 +1165,13 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
   return WGM_OK;
 }
 
+/* Threads per group of a standalone run: the runtime's, but PageRank on its
+ * default group count runs one group of 1024 per SM (its shared memory serves
+ * them all). */
+static int wgm_app_block(const wgm_app *a, int num_wgs) {
+  return a->kind == WGM_APP_PAGERANK && num_wgs <= 0 ? 1024 : wgm_block_size(a->rt);
+}
+
 extern "C" int wgm_launch_persistent(wgm_runtime *rt, wgm_app *a, int num_wgs, void *stream) {
   if (!rt || !a || a->rt != rt) return WGM_ERR_INVALID;
   cudaSetDevice(rt->device);
@@ -1083,7 +1179,7 @@ extern "C" int wgm_launch_persistent(wgm_runtime *rt, wgm_app *a, int num_wgs, v
     return wgm_bc_cta_launch(rt, a, stream ? (cudaStream_t)stream : rt->stream);
   if (wgm_bfs_cta_on(a) && num_wgs <= 1 && !rt->cfg.host_handshake)
     return wgm_bfs_cta_launch(rt, a, stream ? (cudaStream_t)stream : rt->stream);
-  int block = wgm_block_size(rt), grid = 0;
+  int block = wgm_app_block(a, num_wgs), grid = 0;
   int s = wgm_pick_grid(a, num_wgs, block, &grid);
   if (s) return s;
   if (rt->cfg.host_handshake) {
@@ -1126,7 +1222,7 @@ extern "C" int wgm_run_persistent(wgm_runtime *rt, wgm_app *a, int num_wgs,
     }
     return WGM_OK;
   }
-  int block = wgm_block_size(rt), grid = 0;
+  int block = wgm_app_block(a, num_wgs), grid = 0;
   int s = wgm_pick_grid(a, num_wgs, block, &grid);
   if (s) return s;
   const int handshake = rt->cfg.host_handshake ? 1 : 0;

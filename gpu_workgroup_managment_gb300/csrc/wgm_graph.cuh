@@ -2257,203 +2257,236 @@ static __device__ int wgm_phase_pannotia_sssp(const wgm_launch &Lc, wgm_cta *c,
 /* Pull PageRank (FP32; no reference implementation)                          */
 /* ------------------------------------------------------------------------ */
 
+/* PageRank's layout (wgm_pr_layout): vertices by descending degree ("rank"),
+ * rows and columns renumbered so.  Rows of a degree lie together, so a row is
+ * worked by as many lanes as it fills and no lane searches for its owner:
+ *   ranks [0, wide)          more than part_edges edges: a warp per part_edges;
+ *                            the last of them to finish adds up the parts
+ *   bin 0 [bin_row[0], ..)   a warp, 256 edges a step
+ *   bins 1..5                16, 8, 4, 2, 1 lanes, at most 8 edges a lane
+ * and the contributions read most often are the first ones: the first `cached`
+ * sit in shared memory (on RMAT-22, 55,000 of 4.2 M vertices take 57 % of all
+ * reads). */
+#define WGM_PR_BINS 6
+#define WGM_PR_BATCH 4
 struct wgm_pr_args {
-  int V;
-  const int *row;
-  const int *col;
-  float *pr;       /* [V] output */
-  float *contrib;  /* [2][V] pr/deg of the previous iteration */
-  float *dang;     /* [3 lines] dangling mass by iteration */
-  float *hub_sum;  /* [H] */
-  wgm_hubs hubs;
-  int hub_threshold;
+  int V, rows;       /* vertices; those with edges */
+  const int *prow;   /* [rows+1] by rank */
+  const int *pcol;   /* [E] ranks */
+  const int *order;  /* [V] vertex of each rank */
+  float *pr;         /* [V] output, by vertex */
+  float *contrib;    /* [2][stride] pr/deg of the previous iteration, by rank */
+  size_t stride;     /* >= V, whole 16-byte words */
+  float *dang;       /* [3 lines] by iteration mod 3: dangling mass; word 1 (int):
+                        units handed out */
+  int wide, parts;   /* wide rows; their parts of at most part_edges each */
+  int part_edges;
+  const int *part_row; /* [parts] rank of a part's row */
+  const int *row_part; /* [wide+1] first part of a row */
+  float *part;       /* [parts] sums */
+  int *part_done;    /* [wide] parts summed, zero between iterations */
+  int bin_row[WGM_PR_BINS + 1];  /* first rank of each bin, then `rows` */
+  int bin_task[WGM_PR_BINS + 1]; /* first warp task of each bin, then their count */
+  int cached;        /* contributions kept in dynamic shared memory */
   int iterations;
   float damping;
-  float dang0;     /* initial dangling mass: (zero-degree vertices)/V */
+  float dangling;    /* vertices without edges */
 };
 
-/* First stage of a PageRank hub step: the records of windows k0..k0+3
- * (first hub of each in hx), this lane's hub in each (hh) and the col
- * value of its slot (u; -1 past the end). */
-__device__ __forceinline__ void wgm_pr_hub_stage(const int4 *wrec, const int *col, int total,
-                                                 int nwin, int k0, int lane, int *hx, int *hh,
-                                                 int *u) {
-  int4 w[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) w[q] = __ldg(wrec + min(k0 + q, nwin - 1));
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    int e;
-    wgm_hub_slot(w[q], lane, &hh[q], &e);
-    hx[q] = w[q].x;
-    u[q] = (k0 + q < nwin && (k0 + q) * 32 + lane < total) ? __ldg(&col[e]) : -1;
-  }
-}
+extern __shared__ float wgm_pr_cache[];
 
-/* Hub sums of four windows of PageRank hub edges (values v, hub hh per
- * lane, first hub of each window hx), in groups of M consecutive windows.  A group's 32*M slots span at
- * most two hubs when every hub has at least 32*M edges (hub threshold >=
- * 32*M - 1): the group's first hub h0 and h0 + 1.  Each lane sums its M
- * values into those two, then one two-sum warp reduction and at most two
- * atomics serve the group.  Windows past the end hold zeros. */
-template <int M>
-__device__ __forceinline__ void wgm_pr_hub_sums(const int *hx, const int *hh, const float *v,
-                                                int k0, int nwin, int H, float *hub_sum) {
-#pragma unroll
-  for (int g = 0; g < 4; g += M) {
-    if (k0 + g >= nwin) break; /* warp-uniform */
-    const int h0 = hx[g];
-    float f0 = 0.f, f1 = 0.f;
-#pragma unroll
-    for (int q = g; q < g + M; q++) {
-      if (hh[q] == h0) f0 += v[q];
-      else f1 += v[q];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      f0 += __shfl_xor_sync(WGM_FULL, f0, o);
-      f1 += __shfl_xor_sync(WGM_FULL, f1, o);
-    }
-    if (wgm_lane() == 0) {
-      atomicAdd(&hub_sum[h0], f0);
-      if (h0 + 1 < H && f1 != 0.f) atomicAdd(&hub_sum[h0 + 1], f1);
-    }
-  }
+__device__ __forceinline__ float wgm_pr_gather(const float *cin, int cached, int u) {
+  return u < 0 ? 0.f : u < cached ? wgm_pr_cache[u] : __ldca(&cin[u]);
 }
 
 /* pr' = (1-d)/V + d*(sum_{u in N(v)} pr[u]/deg(u) + dangling/V).  Phases:
- * (0) init; (1,t) iteration t for non-hub vertices, hub sums accumulated over
- * the grid; (2,t) hub finalisation.  Per-vertex sums run in a fixed order (a
- * segmented warp scan per window), so only the dangling mass and hub sums
- * depend on atomic order. */
+ * (0) init; (1,t) iteration t, one barrier each.  Every row is summed by the
+ * same lanes in the same order in every run, and the dangling mass needs no
+ * sum: a vertex without edges has exactly the base value.
+ *
+ * What bounds an iteration: the gathers.  Contributions by rank put the
+ * hot ones into a few lines, which thousands of warps then ask one L2 slice
+ * for (1540 us an iteration with every gather from the L2); from shared
+ * memory they cost a few cycles, and the L1 takes the next ones.  RMAT-22
+ * (128 M edges): 566 us with vertex numbers, every gather from the L2 and an
+ * owner search per 32 edges -> 255 us; 174 us if every gather hit shared
+ * memory, which is what the columns and the instructions take.  The columns
+ * pass by the L1 (ldcs).  RMAT-14: 26 us (two barriers of 760 groups) -> 7 us,
+ * one barrier and the round trips bounds - columns - contributions - parts. */
 static __device__ int wgm_phase_pagerank(const wgm_launch &Lc, wgm_cta *c, const wgm_pr_args &a,
-                                         wgm_warp_smem *sm, wgm_step cur, wgm_step *nxt) {
+                                         wgm_step cur, wgm_step *nxt) {
   const wgm_split s(c);
-  const int V = a.V;
+  const int V = a.V, lane = s.lane;
   const float d = a.damping;
+  const int t = cur.round;
   if (cur.target == 0) {
-    for (int i = s.tid; i < V; i += s.nth) {
-      int deg = __ldg(&a.row[i + 1]) - __ldg(&a.row[i]);
-      float p = 1.0f / (float)V;
-      a.pr[i] = p;
-      a.contrib[i] = deg > 0 ? p / (float)deg : 0.f;
+    const float p = 1.0f / (float)V;
+    for (int k = s.tid; k < a.rows; k += s.nth)
+      a.contrib[k] = p / (float)(__ldg(&a.prow[k + 1]) - __ldg(&a.prow[k]));
+    if (a.iterations == 0)
+      for (int v = s.tid; v < V; v += s.nth) a.pr[v] = p;
+    if (c->id == 0 && threadIdx.x < 3) {
+      a.dang[threadIdx.x * WGM_LINE] = a.dangling * p;
+      reinterpret_cast<int *>(a.dang)[threadIdx.x * WGM_LINE + 1] = 0;
     }
-    for (int h = s.tid; h < a.hubs.H; h += s.nth) a.hub_sum[h] = 0.f;
-    if (c->id == 0 && threadIdx.x == 0) {
-      a.dang[0] = a.dang0;
-      a.dang[1 * WGM_LINE] = 0.f;
-      a.dang[2 * WGM_LINE] = 0.f;
-    }
+    for (int k = s.tid; k < a.wide; k += s.nth) a.part_done[k] = 0;
     *nxt = {1, 0};
     return WGM_PHASE_NEXT;
   }
-  const int t = cur.round;
-  const float *cin = a.contrib + (size_t)(t & 1) * V;
-  float *cout = a.contrib + (size_t)((t + 1) & 1) * V;
-  const float base = (1.0f - d) / (float)V + d * __ldcg(&a.dang[(t % 3) * WGM_LINE]) / (float)V;
-  if (cur.target == 2) {
-    for (int h = s.tid; h < a.hubs.H; h += s.nth) {
-      int v = __ldg(&a.hubs.ids[h]);
-      int dg = __ldg(&a.row[v + 1]) - __ldg(&a.row[v]);
-      float p = base + d * __ldcg(&a.hub_sum[h]);
-      a.pr[v] = p;
-      cout[v] = p / (float)dg;
-      a.hub_sum[h] = 0.f;
-    }
-    *nxt = {1, t + 1};
-    return WGM_PHASE_NEXT;
-  }
   if (t >= a.iterations) return WGM_PHASE_DONE;
-  if (c->id == 0 && threadIdx.x == 0) a.dang[((t + 2) % 3) * WGM_LINE] = 0.f;
-  const int lane = s.lane, warp = s.warp;
-  float *acc = reinterpret_cast<float *>(sm->acc[warp]);
-  float dl = 0.f;
-  for (int b = s.gw * 32; b < V; b += s.NW * 32) {
-    int i = b + lane, deg = 0, start = 0, dfull = 0;
-    if (i < V) {
-      start = __ldg(&a.row[i]);
-      dfull = __ldg(&a.row[i + 1]) - start;
-      deg = dfull > a.hub_threshold ? 0 : dfull;
+  const float *cin = a.contrib + (size_t)(t & 1) * a.stride;
+  float *cout = a.contrib + (size_t)((t + 1) & 1) * a.stride;
+  const float base = (1.0f - d) / (float)V + d * __ldcg(&a.dang[(t % 3) * WGM_LINE]) / (float)V;
+  const bool last = t + 1 == a.iterations;
+  int *grab = reinterpret_cast<int *>(a.dang) + (t % 3) * WGM_LINE + 1;
+  if (c->id == 0 && threadIdx.x == 0) {
+    a.dang[((t + 1) % 3) * WGM_LINE] = a.dangling * base;
+    reinterpret_cast<int *>(a.dang)[((t + 2) % 3) * WGM_LINE + 1] = 0;
+  }
+  const int cached = a.cached;
+  if (cached > 0) { /* a multiple of 4, contrib's rows 16-byte aligned */
+    /* each group starts elsewhere, or all would ask for the same lines at once */
+    const int turn = (int)((long long)cached * c->id / c->ngroups) & ~3;
+    for (int i = 4 * threadIdx.x; i < cached; i += 4 * blockDim.x) {
+      const int j = i < cached - turn ? i + turn : i + turn - cached;
+      *reinterpret_cast<float4 *>(&wgm_pr_cache[j]) =
+          __ldcg(reinterpret_cast<const float4 *>(&cin[j]));
     }
-    acc[lane] = 0.f;
-    const int incl = wgm_warp_incl_scan(deg);
-    const int total = __shfl_sync(WGM_FULL, incl, 31);
-    const int off = incl - deg;
-    const int ebase = start - off;
-    __syncwarp();
-    /* windows of 32 edge slots, four at a time: the col loads of the four
-     * windows, then their gathers, are in flight together; each window's
-     * contributions are then summed per owner by a segmented scan, windows
-     * in order, so a vertex's sum has a fixed order */
-    for (int w = 0; w < total; w += 128) {
-      int own[4], u[4];
-      float v[4];
+    __syncthreads();
+  }
+  auto finish = [&](int k, int deg, float sum) {
+    const float p = base + d * sum;
+    cout[k] = p / (float)deg;
+    if (last) a.pr[__ldg(&a.order[k])] = p;
+  };
+  /* Sum of the edges r0 + l, + g, ... below r0 + n, eight in flight; the next
+   * eight columns are read beside this step's contributions. */
+  auto row_sum = [&](int r0, int n, int l, int g) {
+    float sum = 0.f;
+    int u[8];
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int sl = w + 32 * q + lane;
-        const int o = wgm_owner_of(off, min(sl, total - 1));
-        own[q] = sl < total ? o : -1;
-        const int e = __shfl_sync(WGM_FULL, ebase, o) + sl;
-        u[q] = own[q] >= 0 ? __ldg(&a.col[e]) : 0;
+    for (int q = 0; q < 8; q++) u[q] = l + q * g < n ? __ldcs(&a.pcol[r0 + l + q * g]) : -1;
+    for (int i = l; __any_sync(WGM_FULL, i < n); i += 8 * g) {
+      float v[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = wgm_pr_gather(cin, cached, u[q]);
+      const int j = i + 8 * g;
+#pragma unroll
+      for (int q = 0; q < 8; q++) u[q] = j + q * g < n ? __ldcs(&a.pcol[r0 + j + q * g]) : -1;
+#pragma unroll
+      for (int q = 0; q < 8; q++) sum += v[q];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float y = __shfl_xor_sync(WGM_FULL, sum, o);
+      if (o < g) sum += y;
+    }
+    return sum;
+  };
+  /* Work in order of falling degree: a part of a wide row, a row of bin 0, or
+   * `batch` warp tasks of the other bins.  Three quarters go round the warps
+   * by number, the rest are handed out as warps get free. */
+  const int long_units = a.parts + a.bin_task[1];
+  const int tasks = a.bin_task[WGM_PR_BINS] - a.bin_task[1];
+  const int batch = max(1, min(WGM_PR_BATCH, tasks / (4 * s.NW)));
+  const int units = long_units + (tasks + batch - 1) / batch;
+  const int fixed = (int)(3LL * units / 4 / s.NW) * s.NW; /* whole rounds */
+  int unit = s.gw;
+  while (unit < units) {
+    int next = unit + s.NW;
+    if (next >= fixed) {
+      if (lane == 0) next = atomicAdd(grab, 1);
+      next = __shfl_sync(WGM_FULL, next, 0) + max(fixed, s.NW);
+    }
+    if (unit < a.parts) {
+      const int k = __ldg(&a.part_row[unit]), p0 = __ldg(&a.row_part[k]);
+      const int m = __ldg(&a.row_part[k + 1]) - p0;
+      const int r0 = __ldg(&a.prow[k]), n = __ldg(&a.prow[k + 1]) - r0;
+      const int off = (unit - p0) * a.part_edges;
+      const float x = row_sum(r0 + off, min(a.part_edges, n - off), lane, 32);
+      int done = 0;
+      if (lane == 0) {
+        a.part[unit] = x;
+        done = wgm_atom_add_acqrel_gpu(&a.part_done[k], 1) == m - 1;
       }
+      if (__shfl_sync(WGM_FULL, done, 0)) { /* the row's last part: all are there */
+        float y = 0.f;
+        for (int i = lane; i < m; i += 32) y += __ldcg(&a.part[p0 + i]);
 #pragma unroll
-      for (int q = 0; q < 4; q++) v[q] = own[q] >= 0 ? __ldcg(&cin[u[q]]) : 0.f;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        float x = v[q];
-        const int ow = own[q];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          float y = __shfl_up_sync(WGM_FULL, x, o);
-          int oy = __shfl_up_sync(WGM_FULL, ow, o);
-          if (lane >= o && oy == ow) x += y;
+        for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(WGM_FULL, y, o);
+        if (lane == 0) {
+          a.part_done[k] = 0;
+          finish(k, n, y);
         }
-        int nx = __shfl_down_sync(WGM_FULL, ow, 1);
-        if (ow >= 0 && (lane == 31 || nx != ow)) acc[ow] += x;
-        __syncwarp();
+      }
+    } else if (unit < long_units) {
+      const int k = a.bin_row[0] + unit - a.parts;
+      const int r0 = __ldg(&a.prow[k]), n = __ldg(&a.prow[k + 1]) - r0;
+      const float x = row_sum(r0, n, lane, 32);
+      if (lane == 0) finish(k, n, x);
+    } else {
+      const int x0 = a.bin_task[1] + (unit - long_units) * batch;
+      const int x1 = min(x0 + batch, a.bin_task[WGM_PR_BINS]);
+      /* rows of at most 8 edges a lane, in a pipeline over the tasks: the row
+       * bounds of task x + 2 and the columns of task x + 1 are read beside
+       * the contributions of task x */
+      auto locate = [&](int x, int &k, int &g, int &r0, int &n) {
+        int bn = 1, first = a.bin_row[1], task = a.bin_task[1], end = a.bin_row[2];
+#pragma unroll
+        for (int q = 2; q < WGM_PR_BINS; q++)
+          if (x >= a.bin_task[q]) {
+            bn = q;
+            first = a.bin_row[q];
+            task = a.bin_task[q];
+            end = a.bin_row[q + 1];
+          }
+        g = 32 >> bn;
+        k = first + ((x - task) << bn) + (lane >> (5 - bn));
+        r0 = n = 0;
+        if (x < x1 && k < end) {
+          r0 = __ldg(&a.prow[k]);
+          n = __ldg(&a.prow[k + 1]) - r0;
+        }
+      };
+      auto columns = [&](int g, int r0, int n, int (&u)[8]) {
+        const int l = lane & (g - 1);
+#pragma unroll
+        for (int q = 0; q < 8; q++) u[q] = l + q * g < n ? __ldcs(&a.pcol[r0 + l + q * g]) : -1;
+      };
+      int k0, g0, r0, n0, k1, g1, r1, n1, u[8];
+      locate(x0, k0, g0, r0, n0);
+      locate(x0 + 1, k1, g1, r1, n1);
+      columns(g0, r0, n0, u);
+      for (int x = x0; x < x1; x++) {
+        float v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[q] = wgm_pr_gather(cin, cached, u[q]);
+        columns(g1, r1, n1, u);
+        int k2, g2, r2, n2;
+        locate(x + 2, k2, g2, r2, n2);
+        float sum = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; q++) sum += v[q];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const float y = __shfl_xor_sync(WGM_FULL, sum, o);
+          if (o < g0) sum += y;
+        }
+        if (n0 > 0 && (lane & (g0 - 1)) == 0) finish(k0, n0, sum);
+        k0 = k1;
+        g0 = g1;
+        n0 = n1;
+        k1 = k2;
+        g1 = g2;
+        r1 = r2;
+        n1 = n2;
       }
     }
-    __syncwarp();
-    if (i < V && dfull <= a.hub_threshold) {
-      float p = base + d * acc[lane];
-      a.pr[i] = p;
-      cout[i] = dfull > 0 ? p / (float)dfull : 0.f;
-      if (dfull == 0) dl += p;
-    }
+    unit = next;
   }
-  /* hub edges: four windows per warp step, summed in groups of M windows,
-   * in a two-stage pipeline: the next step's window records and col loads
-   * (two dependent round trips) are issued before this step's gathers are
-   * summed, so each step waits for about one round trip instead of three */
-  const int nwin = (a.hubs.total + 31) >> 5;
-  const int4 *wrec = reinterpret_cast<const int4 *>(a.hubs.wmap);
-  const int kstep = s.NW * 4;
-  int k0 = s.gw * 4;
-  int hx[4], hh[4], u[4];
-  if (k0 < nwin) wgm_pr_hub_stage(wrec, a.col, a.hubs.total, nwin, k0, lane, hx, hh, u);
-  for (; k0 < nwin; k0 += kstep) {
-    float v[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) v[q] = u[q] >= 0 ? __ldcg(&cin[u[q]]) : 0.f;
-    int cx[4], ch[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      cx[q] = hx[q];
-      ch[q] = hh[q];
-    }
-    if (k0 + kstep < nwin)
-      wgm_pr_hub_stage(wrec, a.col, a.hubs.total, nwin, k0 + kstep, lane, hx, hh, u);
-    if (a.hub_threshold >= 127)
-      wgm_pr_hub_sums<4>(cx, ch, v, k0, nwin, a.hubs.H, a.hub_sum);
-    else if (a.hub_threshold >= 63)
-      wgm_pr_hub_sums<2>(cx, ch, v, k0, nwin, a.hubs.H, a.hub_sum);
-    else
-      wgm_pr_hub_sums<1>(cx, ch, v, k0, nwin, a.hubs.H, a.hub_sum);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) dl += __shfl_xor_sync(WGM_FULL, dl, o);
-  if (lane == 0 && dl != 0.f) atomicAdd(&a.dang[((t + 1) % 3) * WGM_LINE], dl);
-  *nxt = (a.hubs.H > 0) ? wgm_step{2, t} : wgm_step{1, t + 1};
+  if (last)
+    for (int k = a.rows + s.tid; k < V; k += s.nth) a.pr[__ldg(&a.order[k])] = base;
+  *nxt = {1, t + 1};
   return WGM_PHASE_NEXT;
 }
 

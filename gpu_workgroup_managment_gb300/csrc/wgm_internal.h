@@ -56,7 +56,7 @@ struct wgm_app {
   int2 *d_mis_word = nullptr; /* independent set: {status, value bits} */
   unsigned *d_mis_mask = nullptr;
   int4 *d_mis_wide = nullptr;
-  float *d_contrib = nullptr, *d_dang = nullptr, *d_hub_sum = nullptr;
+  float *d_contrib = nullptr, *d_dang = nullptr;
   int *d_rounds = nullptr;
   /* colour: in-edge CSR when the graph is not symmetric (else the graph) */
   int *d_trow = nullptr, *d_tcol = nullptr;
@@ -86,7 +86,11 @@ struct wgm_app {
   int cq_cap = 0;
   int source = 0;
   float damping = 0.85f;
-  float dang0 = 0.f;
+  /* PageRank: rows and columns by falling degree (wgm_pr_layout) */
+  int *d_pr_order = nullptr, *d_pr_row = nullptr, *d_pr_col = nullptr;
+  int *d_pr_parts = nullptr; /* part_row, row_part, part sums, part_done */
+  int pr_rows = 0, pr_wide = 0, pr_parts = 0, pr_part_edges = 256, pr_bin_row[7] = {}, pr_bin_task[7] = {};
+  int pr_smem = 0, pr_smem_block = 0, pr_smem_per_sm = 0; /* wgm_pagerank_smem's answer */
   int iterations = 20;
   int bc_sources = 0; /* betweenness centrality: sources 0 .. bc_sources-1 */
   int bc_mode = 0;    /* 0: one source at a time over the grid, 1: sources over CTAs */

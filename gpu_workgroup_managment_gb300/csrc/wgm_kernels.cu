@@ -404,12 +404,69 @@ __global__ void __maxnreg__(40) wgm_k_psssp(wgm_launch L, wgm_psssp_args a) {
   WGM_PERSISTENT_EPILOGUE
 }
 
-/* 48 registers (no spills): five 256-thread CTAs per SM instead of four,
- * more gathers in flight for a kernel bound by their latency */
-__global__ void __maxnreg__(48) wgm_k_pagerank(wgm_launch L, wgm_pr_args a) {
-  WGM_PERSISTENT_PROLOGUE
-  WGM_DRIVE(wgm_phase_pagerank(L, &c, a, &sm, cur, nxt));
+__global__ void __launch_bounds__(1024) wgm_k_pagerank(wgm_launch L, wgm_pr_args a) {
+  WGM_PERSISTENT_PROLOGUE_TASKS
+  WGM_DRIVE(wgm_phase_pagerank(L, &c, a, cur, nxt));
   WGM_PERSISTENT_EPILOGUE
+}
+
+/* Dynamic shared memory that `per_sm` groups of `block` threads can each
+ * have on an SM, in bytes (0: they do not fit with any). */
+cudaError_t wgm_pagerank_smem(int block, int per_sm, int *bytes) {
+  int dev = 0, sm_bytes = 0, most = 0, fit = 0;
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, wgm_k_pagerank);
+  if (e != cudaSuccess) return e;
+  most -= (int)fa.sharedSizeBytes;
+  /* the limit is the kernel's, whoever launches it next: always the most */
+  e = cudaFuncSetAttribute(wgm_k_pagerank, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  if (e != cudaSuccess) return e;
+  /* 1 KB of each group's share is the system's */
+  int b = std::min(most, sm_bytes / per_sm - 1024 - (int)fa.sharedSizeBytes) & ~1023;
+  if (b > 0) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, wgm_k_pagerank, block, b);
+  *bytes = b > 0 && fit >= per_sm ? b : 0;
+  return e;
+}
+
+/* PageRank's layout: ranks, then rows and columns by rank (a warp per row). */
+__global__ void __launch_bounds__(256) wgm_k_pr_rank(int V, const int *order, int *rank) {
+  for (int k = blockIdx.x * 256 + threadIdx.x; k < V; k += gridDim.x * 256) rank[order[k]] = k;
+}
+__global__ void __launch_bounds__(256) wgm_k_pr_rows(int rows, const int *row, const int *col,
+                                                     const int *order, const int *rank,
+                                                     const int *prow, int *pcol) {
+  const int nw = gridDim.x * 8, lane = wgm_lane();
+  for (int k0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; k0 < rows; k0 += nw * 32) {
+    const int k = k0 + lane;
+    const int from = k < rows ? row[order[k]] : 0, to = k < rows ? prow[k] : 0;
+    const int n = k < rows ? prow[k + 1] - to : 0;
+    const int incl = wgm_warp_incl_scan(n), total = __shfl_sync(WGM_FULL, incl, 31);
+    const int off = incl - n;
+    for (int w = 0; w < total; w += 128) {
+      int c[4], at[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int sl = w + 32 * q + lane, own = wgm_owner_of(off, min(sl, total - 1));
+        const int e = __shfl_sync(WGM_FULL, from - off, own) + sl;
+        at[q] = __shfl_sync(WGM_FULL, to - off, own) + sl;
+        c[q] = sl < total ? __ldcs(&col[e]) : -1;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (c[q] >= 0) pcol[at[q]] = __ldg(&rank[c[q]]);
+    }
+  }
+}
+cudaError_t wgm_launch_pr_layout(int V, int rows, const int *row, const int *col, const int *order,
+                                 int *rank, const int *prow, int *pcol, cudaStream_t s) {
+  wgm_k_pr_rank<<<std::min((V + 255) / 256, 1216), 256, 0, s>>>(V, order, rank);
+  wgm_k_pr_rows<<<1216, 256, 0, s>>>(rows, row, col, order, rank, prow, pcol);
+  return cudaGetLastError();
 }
 
 /* os_freq (test_suite/os_freq/device/os_freq.cl:8-46): discovery, then
@@ -521,7 +578,7 @@ cudaError_t wgm_launch_psssp(const wgm_launch &L, const wgm_psssp_args &a, int g
 }
 cudaError_t wgm_launch_pagerank(const wgm_launch &L, const wgm_pr_args &a, int grid, int block,
                                 cudaStream_t s) {
-  wgm_k_pagerank<<<grid, block, 0, s>>>(L, a);
+  wgm_k_pagerank<<<grid, block, (size_t)a.cached * 4, s>>>(L, a);
   return cudaGetLastError();
 }
 cudaError_t wgm_launch_octree(const wgm_launch &L, const wgm_octree_args &a, int grid, int block,

@@ -92,7 +92,7 @@ __device__ __forceinline__ void wgm_mega_run_app(const wgm_launch &L, const wgm_
       break;
     case WGM_K_PAGERANK:
       wgm_drive(L, pc, start, sync, [&](wgm_step cur, wgm_step *nxt) {
-        return wgm_phase_pagerank(L, pc, A.pr, sm, cur, nxt);
+        return wgm_phase_pagerank(L, pc, A.pr, cur, nxt);
       });
       break;
     case WGM_K_BC:
