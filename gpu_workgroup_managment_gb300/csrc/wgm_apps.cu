@@ -738,6 +738,7 @@ extern "C" int wgm_app_set_bc_mode(wgm_app *a, int32_t mode) {
   return WGM_OK;
 }
 
+#define WGM_BC_CTA_THREADS 1024
 /* Sources spread over CTAs (bc_mode 1): a plain launch of resident CTAs, no
  * discovery and no host handshake, so the launch generation is untouched. */
 static int wgm_bc_cta_launch(wgm_runtime *rt, wgm_app *a, cudaStream_t s) {
@@ -746,8 +747,7 @@ static int wgm_bc_cta_launch(wgm_runtime *rt, wgm_app *a, cudaStream_t s) {
   std::memset(&A, 0, sizeof(A));
   int st = wgm_app_fill_mega(a, &A);
   if (st) return st;
-  /* 512 threads: on RMAT-12 4.2 ms against 5.7 (256), 8.8 (128), 6.5 (1024) */
-  cudaError_t e = wgm_launch_bc_cta(A.bc, a->d_cnt + 2 * WGM_LINE, 512, s);
+  cudaError_t e = wgm_launch_bc_cta(A.bc, a->d_cnt + 2 * WGM_LINE, WGM_BC_CTA_THREADS, s);
   if (e != cudaSuccess) return wgm_cuda_fail(rt, e);
   return WGM_OK;
 }

@@ -2659,9 +2659,48 @@ static __device__ int wgm_phase_bc(const wgm_launch &Lc, wgm_cta *c, const wgm_b
 #define WGM_BC_CTA_MAX_V 10240
 
 
+/* Vertices a warp takes of a level of n at a time.  They are handed out, for a
+ * hub's edges keep a warp long: RMAT-12, all sources, 4.14 ms with 32
+ * vertices a warp in turn, 2.72 handed out (512 threads), 2.38 with 1024, a
+ * quarter of a warp's share at a time 2.31 (an eighth 2.38), and with two
+ * windows of edges in flight 2.18 (four 2.22).  A vertex at a time, 128 of
+ * its edges together, was slower (2.72): most rows fill less than a warp. */
+#define WGM_BC_SHARE 4
+#define WGM_BC_K 2 /* 32-edge windows in flight */
+__device__ __forceinline__ int wgm_bc_per(int n, int nw) {
+  return max(1, min(32, (n + WGM_BC_SHARE * nw - 1) / (WGM_BC_SHARE * nw)));
+}
+__device__ __forceinline__ int wgm_bc_grab(int *counter, int per) {
+  int b = 0;
+  if (wgm_lane() == 0) b = atomicAdd(counter, per);
+  return __shfl_sync(WGM_FULL, b, 0);
+}
+
+/* f(valid, target, x of its row's lane) for the edges of the lanes' rows. */
+template <class F>
+__device__ __forceinline__ void wgm_bc_edges(const int *col, int start, int deg, float x, F &&f) {
+  const int lane = wgm_lane(), incl = wgm_warp_incl_scan(deg);
+  const int total = __shfl_sync(WGM_FULL, incl, 31), off = incl - deg;
+  for (int w = 0; w < total; w += 32 * WGM_BC_K) {
+    int j[WGM_BC_K];
+    float xo[WGM_BC_K];
+    bool in[WGM_BC_K];
+#pragma unroll
+    for (int q = 0; q < WGM_BC_K; q++) {
+      const int sl = w + 32 * q + lane, own = wgm_owner_of(off, min(sl, total - 1));
+      const int e = __shfl_sync(WGM_FULL, start - off, own) + sl;
+      xo[q] = __shfl_sync(WGM_FULL, x, own);
+      in[q] = sl < total;
+      j[q] = in[q] ? __ldg(&col[e]) : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < WGM_BC_K; q++) f(in[q], j[q], xo[q]);
+  }
+}
+
 static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, int src, int *dist, float *rho,
-                                  float *sig, int *order, int *ls, int *s_cnt, int *tab) {
-  const int V = a.V, lane = wgm_lane(), warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+                                         float *sig, int *order, int *ls, int *s_cnt) {
+  const int V = a.V, lane = wgm_lane(), nw = blockDim.x >> 5;
   for (int i = threadIdx.x; i < V; i += blockDim.x) {
     dist[i] = i == src ? 0 : -1;
     rho[i] = i == src ? WGM_BC_SCALE : 0.f;
@@ -2671,83 +2710,77 @@ static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, int src, int *dis
     order[0] = src;
     ls[0] = 0;
     ls[1] = 1;
-    *s_cnt = 0;
+    s_cnt[0] = 0;
+    s_cnt[1] = 0;
   }
   __syncthreads();
   int L = 0, S = 0, n = 1;
   for (;;) {
-    const int S1 = S + n;
-    for (int b = warp * 32; b < n; b += nw * 32) {
+    const int S1 = S + n, per = wgm_bc_per(n, nw);
+    for (;;) {
+      const int b = wgm_bc_grab(&s_cnt[1], per);
+      if (b >= n) break;
       const int k = b + lane;
-      int v = 0, start = 0, deg = 0;
+      int start = 0, deg = 0;
       float rv = 0.f;
-      if (k < n) {
-        v = order[S + k];
+      if (lane < per && k < n) {
+        const int v = order[S + k];
         start = __ldg(&a.row[v]);
         deg = __ldg(&a.row[v + 1]) - start;
         rv = rho[v];
       }
-      const int incl = wgm_warp_incl_scan(deg);
-      const int total = __shfl_sync(WGM_FULL, incl, 31);
-      const int off = incl - deg;
-      wgm_for_each_edge(off, deg, start - off, total, 0, 32, tab + warp * 32,
-                        [&](bool valid, int e, int owner) {
-                          const float ro = __shfl_sync(WGM_FULL, rv, owner);
-                          bool found = false;
-                          int w = 0;
-                          if (valid) {
-                            w = __ldg(&a.col[e]);
-                            int d = dist[w];
-                            if (d < 0) {
-                              d = atomicCAS(&dist[w], -1, L + 1);
-                              found = d == -1;
-                              if (found) d = L + 1;
-                            }
-                            if (d == L + 1) atomicAdd(&rho[w], ro);
-                          }
-                          wgm_warp_push(found, w, s_cnt, order + S1, V - S1, false);
-                        });
+      wgm_bc_edges(a.col, start, deg, rv, [&](bool valid, int w, float ro) {
+        bool found = false;
+        if (valid) {
+          int d = dist[w];
+          if (d < 0) {
+            d = atomicCAS(&dist[w], -1, L + 1);
+            found = d == -1;
+            if (found) d = L + 1;
+          }
+          if (d == L + 1) atomicAdd(&rho[w], ro);
+        }
+        wgm_warp_push(found, w, &s_cnt[0], order + S1, V - S1, false);
+      });
     }
     __syncthreads();
-    const int n2 = *s_cnt;
+    const int n2 = s_cnt[0];
     __syncthreads();
     if (threadIdx.x == 0) {
-      *s_cnt = 0;
+      s_cnt[0] = 0;
+      s_cnt[1] = 0;
       ls[L + 2] = S1 + n2;
     }
+    __syncthreads();
     if (n2 == 0) break;
     S = S1;
     n = n2;
     L++;
   }
-  __syncthreads();
   for (int l = L; l >= 0; l--) {
-    const int B = ls[l], E = ls[l + 1];
-    for (int b = B + warp * 32; b < E; b += nw * 32) {
+    const int B = ls[l], E = ls[l + 1], per = wgm_bc_per(E - B, nw);
+    /* the levels' grab counters take turns: the other one is cleared here,
+     * after its last grab and before its next */
+    int *grab = &s_cnt[1 + ((L - l) & 1)];
+    if (threadIdx.x == 0) s_cnt[1 + ((L - l + 1) & 1)] = 0;
+    for (;;) {
+      const int b = B + wgm_bc_grab(grab, per);
+      if (b >= E) break;
       const int k = b + lane;
+      const bool have = lane < per && k < E;
       int v = 0, start = 0, deg = 0;
-      float rv = 1.f, sv = 0.f;
-      if (k < E) {
+      float sv = 0.f, fv = 0.f; /* fv: what a predecessor takes per path */
+      if (have) {
         v = order[k];
         start = __ldg(&a.trow[v]);
         deg = l > 0 ? __ldg(&a.trow[v + 1]) - start : 0;
-        rv = rho[v];
         sv = sig[v];
+        fv = (WGM_BC_SCALE + sv) / rho[v];
       }
-      const int incl = wgm_warp_incl_scan(deg);
-      const int total = __shfl_sync(WGM_FULL, incl, 31);
-      const int off = incl - deg;
-      wgm_for_each_edge(off, deg, start - off, total, 0, 32, tab + warp * 32,
-                        [&](bool valid, int e, int owner) {
-                          const float ri = __shfl_sync(WGM_FULL, rv, owner);
-                          const float si = __shfl_sync(WGM_FULL, sv, owner);
-                          if (valid) {
-                            const int w = __ldg(&a.tcol[e]);
-                            if (dist[w] == l - 1)
-                              atomicAdd(&sig[w], rho[w] / ri * (WGM_BC_SCALE + si));
-                          }
-                        });
-      if (k < E && v != src && sv != 0.f) atomicAdd(&a.bc[v], sv / WGM_BC_SCALE);
+      wgm_bc_edges(a.tcol, start, deg, fv, [&](bool valid, int w, float fo) {
+        if (valid && dist[w] == l - 1) atomicAdd(&sig[w], rho[w] * fo);
+      });
+      if (have && v != src && sv != 0.f) atomicAdd(&a.bc[v], sv / WGM_BC_SCALE);
     }
     __syncthreads();
   }

@@ -509,8 +509,7 @@ __global__ void __launch_bounds__(1024) wgm_k_bc(wgm_launch L, wgm_bc_args a) {
  * and no grid barrier. */
 __global__ void __launch_bounds__(1024) wgm_k_bc_cta(wgm_bc_args a, int *queue) {
   extern __shared__ int wgm_bc_dyn[];
-  __shared__ int tab[32 * 32];
-  __shared__ int s_cnt, s_src;
+  __shared__ int s_cnt[3], s_src; /* vertices found; two grab counters */
   int *dist = wgm_bc_dyn;
   float *rho = reinterpret_cast<float *>(dist + a.V);
   float *sig = rho + a.V;
@@ -522,7 +521,7 @@ __global__ void __launch_bounds__(1024) wgm_k_bc_cta(wgm_bc_args a, int *queue) 
     const int src = s_src;
     __syncthreads();
     if (src >= a.num_sources) break;
-    wgm_bc_cta_source(a, src, dist, rho, sig, order, ls, &s_cnt, tab);
+    wgm_bc_cta_source(a, src, dist, rho, sig, order, ls, s_cnt);
     if (threadIdx.x == 0 && a.rounds_out) atomicAdd(a.rounds_out, 1);
   }
 }
