@@ -574,17 +574,88 @@ __device__ __forceinline__ bool wgm_ls_chunk(const int *row, const int *col, con
   return ok;
 }
 
+/* One piece on one warp, an edge per lane: the walker of a level with no more
+ * pieces than warps (a high-diameter graph's).  Such a level is a chain of
+ * dependent round trips, so everything that is not one is left out: no owner
+ * search, no scans, and the pushes are counted by ballots unless a vertex
+ * has several pieces.  A piece of more than 8 edges keeps the pre-check: on
+ * a dense graph most of its atomics would fail, thousands of them on a hub's
+ * word.  A 509x517 grid's SSSP: 5.8 -> 5.1 us a level. */
+template <bool SSSP>
+__device__ __forceinline__ bool wgm_ls_piece(const wgm_lonestar_args &a, int L, int start, int deg,
+                                             int src, const wgm_ls_out &o) {
+  const int lane = wgm_lane(), V = a.V, P = a.piece;
+  unsigned long long *word = reinterpret_cast<unsigned long long *>(a.stamp);
+  bool ok = true;
+  for (int w = 0; w < deg; w += 32) {
+    const bool in = lane < deg - w;
+    const int e = start + w + lane;
+    int u = in ? __ldg(&a.col[e]) : -1, rs = 0, d = 0;
+    unsigned alt = 0;
+    bool f = in;
+    if (SSSP) {
+      const unsigned wk = in ? __ldg(&a.wt[e]) : WGM_LONESTAR_INF;
+      alt = __ldcg(reinterpret_cast<const unsigned *>(a.stamp) + 2 * (size_t)src + 1) + wk;
+      f = wk < WGM_LONESTAR_INF; /* sssp.cl:120 */
+    }
+    f = f && (unsigned)u < (unsigned)V; /* bfs.cl:116 */
+    if (deg > 8 && f)
+      f = SSSP ? alt < __ldcg(reinterpret_cast<const unsigned *>(a.stamp) + 2 * (size_t)u + 1)
+               : __ldcg(&a.dist[u]) == WGM_LONESTAR_INF;
+    if (f) {
+      rs = __ldg(&a.row[u]);
+      d = __ldg(&a.row[u + 1]);
+      if (SSSP) {
+        const unsigned long long old =
+            atomicMin(&word[u], ((unsigned long long)alt << 32) | (unsigned)L);
+        f = (unsigned)(old >> 32) > alt && (unsigned)old != (unsigned)L;
+      } else {
+        f = atomicCAS(&a.dist[u], WGM_LONESTAR_INF, (unsigned)L) == WGM_LONESTAR_INF;
+      }
+    }
+    d = f ? max(d - rs, 0) : 0; /* a vertex without edges is not queued */
+    const unsigned m = __ballot_sync(WGM_FULL, d > 0);
+    if (m == 0) continue;
+    int at = __popc(m & wgm_lanemask_lt()), np = d > 0 ? 1 : 0, n = __popc(m);
+    if (__any_sync(WGM_FULL, d > P)) {
+      np = (d + P - 1) / P;
+      at = wgm_warp_incl_scan(np);
+      n = __shfl_sync(WGM_FULL, at, 31);
+      at -= np;
+    }
+    int base = 0;
+    if (lane == 0) base = wgm_out_reserve(o, n);
+    base = __shfl_sync(WGM_FULL, base, 0);
+    if (base + n > o.cap) {
+      ok = false;
+      continue;
+    }
+    if (np <= WGM_LS_LANE_PIECES)
+      for (int q = 0; q < np; q++)
+        wgm_out_put(o, base + at + q, rs + q * P, min(P, d - q * P), u);
+    /* high-degree vertices: the whole warp writes their pieces */
+    for (unsigned big = __ballot_sync(WGM_FULL, np > WGM_LS_LANE_PIECES); big; big &= big - 1) {
+      const int j = __ffs(big) - 1;
+      const int bs = __shfl_sync(WGM_FULL, rs, j), bd = __shfl_sync(WGM_FULL, d, j);
+      const int bu = __shfl_sync(WGM_FULL, u, j), bsl = base + __shfl_sync(WGM_FULL, at, j);
+      const int bn = __shfl_sync(WGM_FULL, np, j);
+      for (int q = lane; q < bn; q += 32)
+        wgm_out_put(o, bsl + q, bs + q * P, min(P, bd - q * P), bu);
+    }
+  }
+  return ok;
+}
+
 /* One level: every warp takes 32 consecutive pieces of the input list (one
  * per lane) and walks their edges with wgm_ls_chunk; a piece holds at most
  * `piece` edges, so no warp ever holds more than 32*piece edges of a level. */
 template <bool SSSP>
 __device__ __forceinline__ bool wgm_ls_level(const wgm_launch &Lc, wgm_cta *c,
-                                             const wgm_lonestar_args &a, int L,
-                                             wgm_warp_smem *sm) {
+                                             const wgm_lonestar_args &a, int L, int n,
+                                             const int3 &first) {
   const int lane = wgm_lane(), warp = threadIdx.x >> 5;
   const int nwarps_cta = blockDim.x >> 5;
   const int gw = c->id * nwarps_cta + warp, NW = c->ngroups * nwarps_cta;
-  const int n = __ldcg(&a.cnt[(L % 3) * WGM_LINE]);
   const size_t in_off = (size_t)(L & 1) * a.cap, out_off = (size_t)((L + 1) & 1) * a.cap;
   const int *i_start = a.wl_start + in_off, *i_cnt = a.wl_cnt + in_off;
   const int *i_u = a.wl_u ? a.wl_u + in_off : nullptr;
@@ -595,6 +666,8 @@ __device__ __forceinline__ bool wgm_ls_level(const wgm_launch &Lc, wgm_cta *c,
   o.o_u = a.wl_u ? a.wl_u + out_off : nullptr;
   o.cap = a.cap;
   bool ok = true;
+  if (n <= NW && (!SSSP || a.packed))
+    return gw >= n || wgm_ls_piece<SSSP>(a, L, first.x, first.y, first.z, o);
   /* pieces per warp: 32, or fewer when the list is short, so a small
    * frontier spreads over every warp instead of queueing on a few */
   const int per = max(1, min(32, (n + NW - 1) / NW));
@@ -613,7 +686,6 @@ __device__ __forceinline__ bool wgm_ls_level(const wgm_launch &Lc, wgm_cta *c,
       ok &= wgm_ls_chunk<SSSP>(a.row, a.col, a.wt, a.dist, a.stamp, a.V, a.piece, L, start, deg,
                                src, o);
   }
-  (void)sm;
   return ok;
 }
 
@@ -783,7 +855,17 @@ static __device__ int wgm_phase_lonestar(const wgm_launch &Lc, wgm_cta *c,
     *next_round = 1;
     return 1;
   }
-  int n = __ldcg(&a.cnt[(Lv % 3) * WGM_LINE]);
+  /* this warp's piece of a short level, read beside the level's size (any
+   * words, when the list is shorter) */
+  int3 first = make_int3(0, 0, 0);
+  const int gw = c->id * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (gw < a.cap) {
+    const size_t i = (size_t)(Lv & 1) * a.cap + gw;
+    first.x = __ldcg(&a.wl_start[i]);
+    first.y = __ldcg(&a.wl_cnt[i]);
+    if (SSSP) first.z = __ldcg(&a.wl_u[i]);
+  }
+  const int n = __ldcg(&a.cnt[(Lv % 3) * WGM_LINE]);
   if (n == 0) {
     if (c->id == 0 && threadIdx.x == 0 && a.levels_out) *a.levels_out = Lv;
     if (SSSP && a.packed) { /* the distances out of the packed words */
@@ -802,7 +884,7 @@ static __device__ int wgm_phase_lonestar(const wgm_launch &Lc, wgm_cta *c,
     return 0;
   }
   if (c->id == 0 && threadIdx.x == 0) a.cnt[((Lv + 2) % 3) * WGM_LINE] = 0;
-  if (!wgm_ls_level<SSSP>(Lc, c, a, Lv, sm)) wgm_fail(Lc, WGM_DEV_OVERFLOW, WGM_SITE_QUEUE, Lv);
+  if (!wgm_ls_level<SSSP>(Lc, c, a, Lv, n, first)) wgm_fail(Lc, WGM_DEV_OVERFLOW, WGM_SITE_QUEUE, Lv);
   *next_target = 1;
   *next_round = Lv + 1;
   return 1;
