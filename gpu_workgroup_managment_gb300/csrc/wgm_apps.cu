@@ -71,11 +71,6 @@ static bool wgm_is_lonestar(int kind) {
 static bool wgm_needs_weights(int kind) {
   return kind == WGM_APP_LONESTAR_SSSP || kind == WGM_APP_PANNOTIA_SSSP;
 }
-/* (colour's hubs follow its priorities: wgm_color_layout) */
-static bool wgm_uses_static_hubs(int kind) {
-  return kind == WGM_APP_PANNOTIA_SSSP;
-}
-
 /* Reject graphs the kernels cannot walk safely.  The Lonestar loader quirk
  * (row_ptr[V] one less than the edge count, lonestar bfs.h:43) is accepted for
  * the Lonestar apps; their kernels also skip out-of-range destinations like
@@ -108,8 +103,8 @@ static int wgm_validate_graph(int kind, const wgm_graph_desc *g) {
   return WGM_OK;
 }
 
-/* Hub layout for the static-frontier apps (see wgm_hubs in wgm_graph.cuh);
- * hubs in the order of `order` (vertex order when null). */
+/* Colour's hub layout (see wgm_hubs in wgm_graph.cuh), in the order of
+ * `order`. */
 static void wgm_build_hubs(int V, const int32_t *row_ptr, const int *order, int T,
                            std::vector<int> &ids, std::vector<int> &prefix,
                            std::vector<int> &wmap) {
@@ -117,7 +112,7 @@ static void wgm_build_hubs(int V, const int32_t *row_ptr, const int *order, int 
   prefix.assign(1, 0);
   wmap.clear();
   for (int k = 0; k < V; k++) {
-    const int v = order ? order[k] : k;
+    const int v = order[k];
     int d = row_ptr[v + 1] - row_ptr[v];
     if (d > T) {
       ids.push_back(v);
@@ -145,8 +140,7 @@ static void wgm_app_free_buffers(wgm_app *a) {
   void *ptrs[] = {a->d_row,     a->d_col,       a->d_wt,      a->d_node_value, a->d_out,
                   a->d_wl_start, a->d_wl_cnt,   a->d_wl_u,
                   a->d_cnt,       a->d_stamp,   a->d_stop,
-                  a->d_mis_word, a->d_mis_mask, a->d_mis_wide, a->d_contrib,   a->d_dang,    a->d_pr_order, a->d_pr_row,
-                  a->d_pr_col,  a->d_pr_parts, a->d_rounds,
+                  a->d_mis_word, a->d_mis_mask, a->d_mis_wide, a->d_contrib,   a->d_dang,    a->d_rk_order, a->d_rk_parts, a->d_rounds,
                   a->hubs.ids,  a->hubs.prefix, a->hubs.wmap, a->d_trow, a->d_tcol,
                   a->d_oct_input, a->d_oct_second, a->d_oct_pools, a->d_oct_tree,
                   a->d_oct_ctr, a->d_oct_locks, a->d_oct_heads,
@@ -483,9 +477,27 @@ static int wgm_bfs_up_layout(wgm_app *a, const int32_t *row_ptr) {
  * RMAT-22: 16384 5.78 ms, 32768 5.20, 40960 5.10, 45056 5.44, 55296 7.7. */
 #define WGM_PR_EDGES 4096
 #define WGM_PR_CACHED 40960
-/* PageRank's layout (wgm_pr_args): vertices by falling degree (a counting
- * sort, equal degrees by number), rows and columns renumbered on the device. */
-static int wgm_pr_layout(wgm_app *a, const int32_t *row_ptr) {
+static wgm_rank_rows wgm_rank_view(const wgm_app *a) {
+  wgm_rank_rows r;
+  r.rows = a->rk_rows;
+  r.prow = a->d_rk_row;
+  r.pcol = a->d_rk_col;
+  r.pwt = a->d_rk_wt;
+  r.order = a->d_rk_order;
+  r.wide = a->rk_wide;
+  r.parts = a->rk_parts;
+  r.part_edges = a->rk_part_edges;
+  r.part_row = a->d_rk_parts;
+  r.row_part = r.part_row + a->rk_parts;
+  std::copy(a->rk_bin_row, a->rk_bin_row + WGM_RANK_BINS + 1, r.bin_row);
+  std::copy(a->rk_bin_task, a->rk_bin_task + WGM_RANK_BINS + 1, r.bin_task);
+  return r;
+}
+
+/* Layout by rank (wgm_rank_rows): vertices by falling degree (a counting
+ * sort, equal degrees by number), rows, columns and weights renumbered on the
+ * device. */
+static int wgm_rank_layout(wgm_app *a, const int32_t *row_ptr) {
   const int V = a->V;
   int most = 0;
   for (int v = 0; v < V; v++) most = std::max(most, row_ptr[v + 1] - row_ptr[v]);
@@ -494,49 +506,54 @@ static int wgm_pr_layout(wgm_app *a, const int32_t *row_ptr) {
   /* rows of more than x edges: at[most - x] once summed */
   for (int x = 0; x <= most; x++) at[x + 1] += at[x];
   auto above = [&](int x) { return x >= most ? 0 : at[most - x]; };
-  a->pr_rows = above(0);
+  a->rk_rows = above(0);
   /* parts of wide rows: 256 edges (one step of a warp) while the graph has
    * fewer than that for every warp, up to 2048 */
-  a->pr_part_edges = 256;
-  while (a->pr_part_edges < 2048 &&
-         a->E / (32LL * a->rt->prop.multiProcessorCount) > 4LL * a->pr_part_edges)
-    a->pr_part_edges *= 2;
-  a->pr_wide = above(a->pr_part_edges);
-  a->pr_bin_row[0] = a->pr_wide;
-  for (int b = 1; b < WGM_PR_BINS; b++) a->pr_bin_row[b] = above(8 * (32 >> b));
-  a->pr_bin_row[WGM_PR_BINS] = a->pr_rows;
-  a->pr_bin_task[0] = 0;
-  for (int b = 0; b < WGM_PR_BINS; b++)
-    a->pr_bin_task[b + 1] =
-        a->pr_bin_task[b] + ((a->pr_bin_row[b + 1] - a->pr_bin_row[b] + (1 << b) - 1) >> b);
+  a->rk_part_edges = 256;
+  while (a->rk_part_edges < 2048 &&
+         a->E / (32LL * a->rt->prop.multiProcessorCount) > 4LL * a->rk_part_edges)
+    a->rk_part_edges *= 2;
+  a->rk_wide = above(a->rk_part_edges);
+  a->rk_bin_row[0] = a->rk_wide;
+  for (int b = 1; b < WGM_RANK_BINS; b++) a->rk_bin_row[b] = above(8 * (32 >> b));
+  a->rk_bin_row[WGM_RANK_BINS] = a->rk_rows;
+  a->rk_bin_task[0] = 0;
+  for (int b = 0; b < WGM_RANK_BINS; b++)
+    a->rk_bin_task[b + 1] =
+        a->rk_bin_task[b] + ((a->rk_bin_row[b + 1] - a->rk_bin_row[b] + (1 << b) - 1) >> b);
   for (int v = 0; v < V; v++) order[at[most - (row_ptr[v + 1] - row_ptr[v])]++] = v;
   prow[0] = 0;
-  for (int k = 0; k < a->pr_rows; k++)
+  for (int k = 0; k < a->rk_rows; k++)
     prow[k + 1] = prow[k] + (row_ptr[order[k] + 1] - row_ptr[order[k]]);
   /* parts of the wide rows: {part_row [parts], row_part [wide+1]} */
   std::vector<int> parts, row_part(1, 0);
-  for (int k = 0; k < a->pr_wide; k++) {
-    const int m = (prow[k + 1] - prow[k] + a->pr_part_edges - 1) / a->pr_part_edges;
+  for (int k = 0; k < a->rk_wide; k++) {
+    const int m = (prow[k + 1] - prow[k] + a->rk_part_edges - 1) / a->rk_part_edges;
     parts.insert(parts.end(), (size_t)m, k);
     row_part.push_back((int)parts.size());
   }
-  a->pr_parts = (int)parts.size();
+  a->rk_parts = (int)parts.size();
   parts.insert(parts.end(), row_part.begin(), row_part.end());
   cudaStream_t st = a->rt->stream;
-  if (a->d_pr_parts) cudaFree(a->d_pr_parts);
-  a->d_pr_parts = nullptr;
-  cudaError_t e = wgm_dmalloc(&a->d_pr_parts, 2 * (size_t)a->pr_parts + 2 * (size_t)a->pr_wide + 1);
+  if (a->d_rk_parts) cudaFree(a->d_rk_parts);
+  a->d_rk_parts = nullptr;
+  cudaError_t e = wgm_dmalloc(&a->d_rk_parts, 2 * (size_t)a->rk_parts + 2 * (size_t)a->rk_wide + 1);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(a->d_pr_parts, parts.data(), parts.size() * 4, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(a->d_pr_order, order.data(), (size_t)V * 4,
+    e = cudaMemcpyAsync(a->d_rk_parts, parts.data(), parts.size() * 4, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(a->d_rk_order, order.data(), (size_t)V * 4,
                                   cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(a->d_pr_row, prow.data(), ((size_t)a->pr_rows + 1) * 4,
+    e = cudaMemcpyAsync(a->d_rk_row, prow.data(), ((size_t)a->rk_rows + 1) * 4,
                         cudaMemcpyHostToDevice, st);
-  /* the ranks pass through the result buffer */
+  if (e == cudaSuccess && a->d_wt) { /* least weight: INT_MAX before any */
+    const int none = INT32_MAX;
+    e = cudaMemcpyAsync(a->d_cnt, &none, 4, cudaMemcpyHostToDevice, st);
+  }
+  /* PageRank's ranks only pass through: its result buffer holds them */
   if (e == cudaSuccess)
-    e = wgm_launch_pr_layout(V, a->pr_rows, a->d_row, a->d_col, a->d_pr_order, (int *)a->d_out,
-                             a->d_pr_row, a->d_pr_col, st);
+    e = wgm_launch_rank_layout(V, wgm_rank_view(a), a->d_row, a->d_col, (const int *)a->d_wt,
+                               a->d_rk_of ? a->d_rk_of : (int *)a->d_out, a->d_rk_col, a->d_rk_wt,
+                               a->d_cnt, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e == cudaSuccess ? WGM_OK : wgm_cuda_fail(a->rt, e);
 }
@@ -557,10 +574,6 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
   if (e == cudaSuccess && wgm_needs_weights(a->kind) && a->E > 0)
     e = cudaMemcpyAsync(a->d_wt, g->weights, (size_t)a->E * 4, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
-  if (wgm_uses_static_hubs(a->kind)) {
-    s = wgm_upload_hubs(a, g->row_ptr, nullptr);
-    if (s) return s;
-  }
   if (a->kind == WGM_APP_LONESTAR_BFS) {
     s = wgm_bfs_ell_layout(a, g->row_ptr);
     if (s == WGM_OK) s = wgm_bfs_up_layout(a, g->row_ptr);
@@ -575,8 +588,24 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
     s = wgm_upload_transpose(a, g);
     if (s) return s;
   }
-  if (a->kind == WGM_APP_PAGERANK) return wgm_pr_layout(a, g->row_ptr);
+  if (a->kind == WGM_APP_PAGERANK || a->kind == WGM_APP_PANNOTIA_SSSP)
+    return wgm_rank_layout(a, g->row_ptr);
   return WGM_OK;
+}
+
+/* The layout by rank in one allocation (d_rk_order owns it). */
+static cudaError_t wgm_rank_alloc(wgm_app *a, bool weighted) {
+  const size_t V = (size_t)a->V, E = (size_t)a->E;
+  cudaError_t e = wgm_dmalloc(&a->d_rk_order, 2 * V + 1 + E + (weighted ? E + 2 * V : 0));
+  if (e != cudaSuccess) return e;
+  a->d_rk_row = a->d_rk_order + V;
+  a->d_rk_col = a->d_rk_row + V + 1;
+  if (weighted) {
+    a->d_rk_wt = a->d_rk_col + E;
+    a->d_rk_of = a->d_rk_wt + E;
+    a->d_rk_x = a->d_rk_of + V;
+  }
+  return cudaSuccess;
 }
 
 static size_t wgm_pr_stride(int V) { return ((size_t)V + 3) & ~(size_t)3; }
@@ -652,7 +681,9 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
     case WGM_APP_PANNOTIA_SSSP:
       a->out_bytes = V * 4;
       if (e == cudaSuccess) e = cudaMalloc(&a->d_out, a->out_bytes);
-      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_stop, 3 * WGM_LINE);
+      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_stop, 6 * WGM_LINE);
+      if (e == cudaSuccess) e = wgm_rank_alloc(a, true);
+      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cnt, 1); /* least weight */
       break;
     case WGM_APP_PAGERANK:
       a->out_bytes = V * 4;
@@ -660,9 +691,7 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
       /* contrib: two rows of V rounded up to whole 16-byte words, and one more */
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_contrib, 2 * wgm_pr_stride(a->V));
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_dang, 3 * WGM_LINE);
-      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_pr_order, V);
-      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_pr_row, V + 1);
-      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_pr_col, E);
+      if (e == cudaSuccess) e = wgm_rank_alloc(a, false);
       break;
     case WGM_APP_PANNOTIA_BC:
       /* bc (out), dist, rho and sigma, the level lists and their starts */
@@ -932,13 +961,12 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
     case WGM_APP_PANNOTIA_SSSP: {
       wgm_psssp_args &x = A->psssp;
       x.V = a->V;
-      x.row = a->d_row;
-      x.col = a->d_col;
-      x.data = (const int *)a->d_wt;
+      x.R = wgm_rank_view(a);
+      x.rank = a->d_rk_of;
+      x.xr = a->d_rk_x;
       x.x = (int *)a->d_out;
       x.stop = a->d_stop;
-      x.hubs = wgm_hubs_view(a);
-      x.hub_threshold = a->hub_threshold;
+      x.wmin = a->d_cnt;
       x.source = a->source;
       x.rounds_out = a->d_rounds;
       return WGM_OK;
@@ -946,27 +974,17 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
     case WGM_APP_PAGERANK: {
       wgm_pr_args &x = A->pr;
       x.V = a->V;
-      x.rows = a->pr_rows;
-      x.prow = a->d_pr_row;
-      x.pcol = a->d_pr_col;
-      x.order = a->d_pr_order;
+      x.R = wgm_rank_view(a);
       x.pr = (float *)a->d_out;
       x.contrib = a->d_contrib;
       x.stride = wgm_pr_stride(a->V);
       x.dang = a->d_dang;
-      x.wide = a->pr_wide;
-      x.parts = a->pr_parts;
-      x.part_edges = a->pr_part_edges;
-      x.part_row = a->d_pr_parts;
-      x.row_part = x.part_row + a->pr_parts;
-      x.part = (float *)(a->d_pr_parts + a->pr_parts + a->pr_wide + 1);
-      x.part_done = a->d_pr_parts + 2 * (size_t)a->pr_parts + a->pr_wide + 1;
-      std::copy(a->pr_bin_row, a->pr_bin_row + WGM_PR_BINS + 1, x.bin_row);
-      std::copy(a->pr_bin_task, a->pr_bin_task + WGM_PR_BINS + 1, x.bin_task);
+      x.part = (float *)(a->d_rk_parts + a->rk_parts + a->rk_wide + 1);
+      x.part_done = a->d_rk_parts + 2 * (size_t)a->rk_parts + a->rk_wide + 1;
       x.cached = 0;
       x.iterations = a->iterations;
       x.damping = a->damping;
-      x.dangling = (float)(a->V - a->pr_rows);
+      x.dangling = (float)(a->V - a->rk_rows);
       return WGM_OK;
     }
   }
@@ -1072,7 +1090,7 @@ static cudaError_t wgm_app_enqueue(wgm_app *a, const wgm_launch &L, int grid, in
         a->pr_smem_block = block;
         a->pr_smem_per_sm = per_sm;
       }
-      A.pr.cached = std::min({(a->pr_rows + 3) & ~3, a->pr_smem / 4, WGM_PR_CACHED});
+      A.pr.cached = std::min({(a->rk_rows + 3) & ~3, a->pr_smem / 4, WGM_PR_CACHED});
       return wgm_launch_pagerank(L, A.pr, grid, block, stream);
     }
     case WGM_APP_OCTREE:

@@ -2200,20 +2200,198 @@ static __device__ int wgm_phase_mis(const wgm_launch &Lc, wgm_cta *c, const wgm_
 }
 
 /* ------------------------------------------------------------------------ */
+/* Rows by falling degree (PageRank, Pannotia SSSP)                          */
+/* ------------------------------------------------------------------------ */
+
+/* Layout of the apps that pull over every row (wgm_rank_layout): vertices by
+ * descending degree ("rank"), rows and columns renumbered so.  Rows of a
+ * degree lie together, so a row is worked by as many lanes as it fills and no
+ * lane searches for its owner:
+ *   ranks [0, wide)          more than part_edges edges: a warp per part_edges
+ *   bin 0 [bin_row[0], ..)   a warp, 256 edges a step
+ *   bins 1..5                16, 8, 4, 2, 1 lanes, at most 8 edges a lane */
+#define WGM_RANK_BINS 6
+#define WGM_RANK_BATCH 4
+#define WGM_RANK_ROUNDS 8
+struct wgm_rank_rows {
+  int rows;          /* vertices with edges */
+  const int *prow;   /* [rows+1] by rank */
+  const int *pcol;   /* [E] ranks */
+  const int *pwt;    /* [E] weights (may be null) */
+  const int *order;  /* [V] vertex of each rank */
+  int wide, parts;   /* wide rows; their parts of at most part_edges each */
+  int part_edges;
+  const int *part_row; /* [parts] rank of a part's row */
+  const int *row_part; /* [wide+1] first part of a row */
+  int bin_row[WGM_RANK_BINS + 1];  /* first rank of each bin, then `rows` */
+  int bin_task[WGM_RANK_BINS + 1]; /* first warp task of each bin, then their count */
+};
+
+/* Every row once: op.none() is the sum of nothing, op.edge(u, w) an edge's
+ * term (u < 0: none), op.join(x, y) adds two; then op.row(k, n, x) gets row
+ * k's n edges' sum and op.part(unit, k, x) that of one part of a wide row
+ * (by lane 0), with op.after_part(unit, k) called by the whole warp.  Rows
+ * that op.skip(k) names are left out (no row or part of them is reported).
+ * `grab` hands out work, zero before. */
+template <bool WEIGHTED, class T, class Op>
+__device__ __forceinline__ void wgm_rank_pull(const wgm_rank_rows &R, const wgm_split &s, int *grab,
+                                              Op &&op) {
+  const int lane = s.lane;
+  auto columns = [&](int r0, int n, int l, int g, int (&u)[8], int (&w)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const bool in = l + q * g < n;
+      u[q] = in ? __ldcs(&R.pcol[r0 + l + q * g]) : -1;
+      w[q] = WEIGHTED && in ? __ldcs(&R.pwt[r0 + l + q * g]) : 0;
+    }
+  };
+  auto reduce = [&](T x, int g) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const T y = __shfl_xor_sync(WGM_FULL, x, o);
+      if (o < g) x = op.join(x, y);
+    }
+    return x;
+  };
+  /* the edges r0 .. r0 + n on a warp, eight a lane in flight; the next eight
+   * columns are read beside this step's terms */
+  auto long_row = [&](int r0, int n) {
+    T x = op.none();
+    int u[8], w[8];
+    columns(r0, n, lane, 32, u, w);
+    for (int i = lane; __any_sync(WGM_FULL, i < n); i += 256) {
+      T v[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) v[q] = op.edge(u[q], w[q]);
+      columns(r0, n, i + 256, 32, u, w);
+#pragma unroll
+      for (int q = 0; q < 8; q++) x = op.join(x, v[q]);
+    }
+    return reduce(x, 32);
+  };
+  /* Work in order of falling degree: a part of a wide row, a row of bin 0, or
+   * `batch` warp tasks of the other bins, round the warps by number; with more
+   * than WGM_RANK_ROUNDS rounds the last quarter is handed out as warps get
+   * free (on fewer, every warp would queue at the counter at once). */
+  const int long_units = R.parts + R.bin_task[1];
+  const int tasks = R.bin_task[WGM_RANK_BINS] - R.bin_task[1];
+  const int batch = max(1, min(WGM_RANK_BATCH, tasks / (4 * s.NW)));
+  const int units = long_units + (tasks + batch - 1) / batch;
+  const int fixed = units <= WGM_RANK_ROUNDS * s.NW
+                        ? units
+                        : (int)(3LL * units / 4 / s.NW) * s.NW; /* whole rounds */
+  int unit = s.gw;
+  while (unit < units) {
+    int next = unit + s.NW;
+    if (next >= fixed && fixed < units) {
+      if (lane == 0) next = atomicAdd(grab, 1);
+      next = __shfl_sync(WGM_FULL, next, 0) + max(fixed, s.NW);
+    }
+    if (unit < long_units) {
+      const bool part = unit < R.parts;
+      const int k = part ? __ldg(&R.part_row[unit]) : R.bin_row[0] + unit - R.parts;
+      const int r0 = __ldg(&R.prow[k]), n = __ldg(&R.prow[k + 1]) - r0;
+      const int off = part ? (unit - __ldg(&R.row_part[k])) * R.part_edges : 0;
+      if (!op.skip(k)) {
+        const T x = long_row(r0 + off, part ? min(R.part_edges, n - off) : n);
+        if (lane == 0) {
+          if (part) op.part(unit, k, x);
+          else op.row(k, n, x);
+        }
+        if (part) op.after_part(unit, k, n);
+      }
+    } else {
+      const int x0 = R.bin_task[1] + (unit - long_units) * batch;
+      const int x1 = min(x0 + batch, R.bin_task[WGM_RANK_BINS]);
+      /* rows of at most 8 edges a lane, in a pipeline over the tasks: the row
+       * bounds of task x + 2 and the columns of task x + 1 are read beside
+       * the terms of task x */
+      auto locate = [&](int x, int &k, int &g, int &r0, int &n) {
+        int bn = 1, first = R.bin_row[1], task = R.bin_task[1], end = R.bin_row[2];
+#pragma unroll
+        for (int q = 2; q < WGM_RANK_BINS; q++)
+          if (x >= R.bin_task[q]) {
+            bn = q;
+            first = R.bin_row[q];
+            task = R.bin_task[q];
+            end = R.bin_row[q + 1];
+          }
+        g = 32 >> bn;
+        k = first + ((x - task) << bn) + (lane >> (5 - bn));
+        r0 = n = 0;
+        if (x < x1 && k < end) {
+          const bool skip = op.skip(k);
+          r0 = __ldg(&R.prow[k]);
+          n = skip ? 0 : __ldg(&R.prow[k + 1]) - r0;
+        }
+      };
+      int k0, g0, r0, n0, k1, g1, r1, n1, u[8], w[8];
+      locate(x0, k0, g0, r0, n0);
+      locate(x0 + 1, k1, g1, r1, n1);
+      columns(r0, n0, lane & (g0 - 1), g0, u, w);
+      for (int x = x0; x < x1; x++) {
+        T v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[q] = op.edge(u[q], w[q]);
+        columns(r1, n1, lane & (g1 - 1), g1, u, w);
+        int k2, g2, r2, n2;
+        locate(x + 2, k2, g2, r2, n2);
+        T sum = op.none();
+#pragma unroll
+        for (int q = 0; q < 8; q++) sum = op.join(sum, v[q]);
+        sum = reduce(sum, g0);
+        if (n0 > 0 && (lane & (g0 - 1)) == 0) op.row(k0, n0, sum);
+        k0 = k1;
+        g0 = g1;
+        n0 = n1;
+        k1 = k2;
+        g1 = g2;
+        r1 = r2;
+        n1 = n2;
+      }
+    }
+    unit = next;
+  }
+}
+
+/* ------------------------------------------------------------------------ */
 /* Pannotia SSSP (pull min-plus)                                             */
 /* ------------------------------------------------------------------------ */
 
 struct wgm_psssp_args {
   int V;
-  const int *row;
-  const int *col;
-  const int *data;
-  int *x;    /* [V] output cost (sssp.h:168 reads x) */
-  int *stop; /* [3 lines] */
-  wgm_hubs hubs;
-  int hub_threshold;
+  wgm_rank_rows R;
+  const int *rank; /* [V] rank of each vertex */
+  int *xr;         /* [V] cost by rank */
+  int *x;          /* [V] output cost (sssp.h:168 reads x) */
+  int *stop;       /* [6 lines] by round mod 3: work handed out; then least cost that
+                      changed (INT_MAX: none) */
+  const int *wmin; /* least edge weight */
   int source;
   int *rounds_out;
+};
+
+/* One pass of x[v] = min(x[v], min_j data[j] + x[col[j]]) (wgm_rank_pull). */
+struct wgm_psssp_op {
+  int *xr;
+  int bound;           /* costs up to here cannot fall in this pass */
+  int least = INT_MAX; /* least cost that this thread lowered */
+  __device__ __forceinline__ bool skip(int k) const { return __ldcg(&xr[k]) <= bound; }
+  __device__ __forceinline__ int none() const { return INT_MAX; }
+  __device__ __forceinline__ int edge(int u, int w) const {
+    return u < 0 ? INT_MAX : w + __ldca(&xr[u]);
+  }
+  __device__ __forceinline__ int join(int x, int y) const { return min(x, y); }
+  __device__ __forceinline__ void row(int k, int, int x) {
+    if (x < __ldcg(&xr[k])) {
+      xr[k] = x; /* the row's only writer */
+      least = min(least, x);
+    }
+  }
+  __device__ __forceinline__ void part(int, int k, int x) {
+    if (x < __ldcg(&xr[k]) && atomicMin(&xr[k], x) > x) least = min(least, x);
+  }
+  __device__ __forceinline__ void after_part(int, int, int) {}
 };
 
 /* sssp.cl's vector_assign / spmv_min_dot_plus / vector_diff (three barriers
@@ -2222,22 +2400,42 @@ struct wgm_psssp_args {
  * iteration and this chaotic (in-place) iteration both stop at the fixpoint
  * of the min-plus system started from x = BIG_NUM except x[source] = 0, which
  * is unique (the shortest-path distances, BIG_NUM where unreachable), so the
- * returned vector is identical; only the round count can be smaller.
- * Phases: (0) init; (1,r) one relaxation pass (after the exit test of r-1). */
+ * returned vector is identical; only the round count can be smaller.  Costs
+ * are read through the L1: one that another SM has lowered since was lowered
+ * in this round, so a next one follows and reads it (a barrier empties the
+ * L1).
+ * A pass leaves out the rows it cannot change.  With no negative weight, a
+ * cost can only fall to (least cost that changed in the pass before) + (least
+ * weight) or above: what changed earlier was read in the pass before, or was
+ * too large by the same test.  Rows at or under that bound - nearly all of
+ * them in the last passes - cost one word.  A 200,003-vertex RMAT graph of
+ * 4.5 M edges: 12 passes of 44 us (an owner search and a shared-memory
+ * minimum per edge, hubs by windows) -> 18 passes of 25 to 12 us, 0.51 ->
+ * 0.33 ms; reading past the L1 takes 15 passes but 1.0 ms, for the hubs'
+ * costs share a few lines.  One update of the least changed cost per group:
+ * one per warp made a pass 260 us.
+ * Phases: (0) init; (1,r) one relaxation pass (after the exit test of r-1);
+ * the costs go out by vertex when it ends. */
 static __device__ int wgm_phase_pannotia_sssp(const wgm_launch &Lc, wgm_cta *c,
-                                              const wgm_psssp_args &a, wgm_warp_smem *sm,
-                                              wgm_step cur, wgm_step *nxt) {
+                                              const wgm_psssp_args &a, wgm_step cur,
+                                              wgm_step *nxt) {
   const wgm_split s(c);
   const int V = a.V;
+  int *changed = a.stop + 3 * WGM_LINE;
   if (cur.target == 0) {
-    for (int i = s.tid; i < V; i += s.nth) a.x[i] = (i == a.source) ? 0 : WGM_PANNOTIA_BIG;
-    if (c->id == 0 && threadIdx.x == 0)
-      for (int k = 0; k < 3; k++) a.stop[k * WGM_LINE] = 0;
+    const int src = __ldg(&a.rank[a.source]);
+    for (int k = s.tid; k < V; k += s.nth) a.xr[k] = k == src ? 0 : WGM_PANNOTIA_BIG;
+    if (c->id == 0 && threadIdx.x < 3) {
+      a.stop[threadIdx.x * WGM_LINE] = 0;
+      changed[threadIdx.x * WGM_LINE] = INT_MAX;
+    }
     *nxt = {1, 1};
     return WGM_PHASE_NEXT;
   }
   const int r = cur.round;
-  if (r > 1 && __ldcg(&a.stop[((r - 1) % 3) * WGM_LINE]) == 0) {
+  const int before = r > 1 ? __ldcg(&changed[((r - 1) % 3) * WGM_LINE]) : 0;
+  if (before == INT_MAX) {
+    for (int k = s.tid; k < V; k += s.nth) a.x[__ldg(&a.R.order[k])] = __ldcg(&a.xr[k]);
     if (c->id == 0 && threadIdx.x == 0 && a.rounds_out) *a.rounds_out = r - 1;
     return WGM_PHASE_DONE;
   }
@@ -2245,92 +2443,21 @@ static __device__ int wgm_phase_pannotia_sssp(const wgm_launch &Lc, wgm_cta *c,
     wgm_fail(Lc, WGM_DEV_BAD_INPUT, WGM_SITE_QUEUE, r);
     return WGM_PHASE_DONE;
   }
-  if (c->id == 0 && threadIdx.x == 0) a.stop[((r + 1) % 3) * WGM_LINE] = 0;
-  bool changed = false;
-  const int lane = s.lane, warp = s.warp;
-  for (int b = s.gw * 32; b < V; b += s.NW * 32) {
-    int i = b + lane, deg = 0, start = 0;
-    if (i < V) {
-      start = __ldg(&a.row[i]);
-      int d = __ldg(&a.row[i + 1]) - start;
-      deg = d > a.hub_threshold ? 0 : d;
-    }
-    sm->acc[warp][lane] = INT_MAX;
-    int incl = wgm_warp_incl_scan(deg);
-    int total = __shfl_sync(WGM_FULL, incl, 31);
-    int off = incl - deg;
-    __syncwarp();
-    /* four 32-edge windows per step: their col and weight loads, then their
-     * x gathers, in flight together (a min is exact in any order) */
-    const int ebase = start - off;
-    for (int w = 0; w < total; w += 128) {
-      int own[4], j[4], wt[4], xj[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int sl = w + 32 * q + lane;
-        const int o = wgm_owner_of(off, min(sl, total - 1));
-        own[q] = sl < total ? o : -1;
-        const int e = __shfl_sync(WGM_FULL, ebase, o) + sl;
-        j[q] = own[q] >= 0 ? __ldg(&a.col[e]) : 0;
-        wt[q] = own[q] >= 0 ? __ldg(&a.data[e]) : 0;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; q++) xj[q] = own[q] >= 0 ? __ldcg(&a.x[j[q]]) : 0;
-#pragma unroll
-      for (int q = 0; q < 4; q++)
-        if (own[q] >= 0) atomicMin(&sm->acc[warp][own[q]], wt[q] + xj[q]);
-    }
-    __syncwarp();
-    if (deg > 0) {
-      int cand = sm->acc[warp][lane];
-      if (cand < __ldcg(&a.x[i])) {
-        atomicMin(&a.x[i], cand);
-        changed = true;
-      }
-    }
+  if (c->id == 0 && threadIdx.x == 0) {
+    a.stop[((r + 1) % 3) * WGM_LINE] = 0;
+    changed[((r + 1) % 3) * WGM_LINE] = INT_MAX;
   }
-  /* hub edges: four windows per warp step, their records, col and weight
-   * loads, and x gathers in flight together */
-  const int nwin = (a.hubs.total + 31) >> 5;
-  const int4 *wrec = reinterpret_cast<const int4 *>(a.hubs.wmap);
-  for (int k0 = s.gw * 4; k0 < nwin; k0 += s.NW * 4) {
-    int4 w[4];
-    int hh[4], j[4], wt[4], xj[4];
-    bool val[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int k = min(k0 + q, nwin - 1);
-      w[q] = __ldg(wrec + k);
-      val[q] = k0 + q < nwin && (k0 + q) * 32 + lane < a.hubs.total;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      int e;
-      wgm_hub_slot(w[q], lane, &hh[q], &e);
-      j[q] = val[q] ? __ldg(&a.col[e]) : 0;
-      wt[q] = val[q] ? __ldg(&a.data[e]) : 0;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) xj[q] = val[q] ? __ldcg(&a.x[j[q]]) : 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      if (k0 + q >= nwin) break; /* warp-uniform */
-      const int h0 = w[q].x;
-      int m0, m1;
-      float f0, f1;
-      wgm_two_seg_reduce(hh[q] == h0, val[q] ? wt[q] + xj[q] : INT_MAX, 0.f, 1, &m0, &m1,
-                         &f0, &f1);
-      if (lane == 0) {
-        const int v0 = __ldg(&a.hubs.ids[h0]);
-        if (m0 < __ldcg(&a.x[v0]) && atomicMin(&a.x[v0], m0) > m0) changed = true;
-        if (h0 + 1 < a.hubs.H && m1 != INT_MAX) {
-          const int v1 = __ldg(&a.hubs.ids[h0 + 1]);
-          if (m1 < __ldcg(&a.x[v1]) && atomicMin(&a.x[v1], m1) > m1) changed = true;
-        }
-      }
-    }
-  }
-  if (__any_sync(WGM_FULL, changed) && lane == 0) a.stop[(r % 3) * WGM_LINE] = 1;
+  const int wmin = __ldg(a.wmin);
+  wgm_psssp_op op{a.xr, INT_MIN};
+  if (r > 1 && wmin >= 0) op.bound = (int)min((long long)INT_MAX, (long long)before + wmin);
+  __shared__ int s_least; /* one update per group: the word is everybody's */
+  if (threadIdx.x == 0) s_least = INT_MAX;
+  __syncthreads();
+  wgm_rank_pull<true, int>(a.R, s, &a.stop[(r % 3) * WGM_LINE], op);
+  if (op.least != INT_MAX) atomicMin(&s_least, op.least);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_least != INT_MAX)
+    atomicMin(&changed[(r % 3) * WGM_LINE], s_least);
   *nxt = {1, r + 1};
   return WGM_PHASE_NEXT;
 }
@@ -2339,36 +2466,19 @@ static __device__ int wgm_phase_pannotia_sssp(const wgm_launch &Lc, wgm_cta *c,
 /* Pull PageRank (FP32; no reference implementation)                          */
 /* ------------------------------------------------------------------------ */
 
-/* PageRank's layout (wgm_pr_layout): vertices by descending degree ("rank"),
- * rows and columns renumbered so.  Rows of a degree lie together, so a row is
- * worked by as many lanes as it fills and no lane searches for its owner:
- *   ranks [0, wide)          more than part_edges edges: a warp per part_edges;
- *                            the last of them to finish adds up the parts
- *   bin 0 [bin_row[0], ..)   a warp, 256 edges a step
- *   bins 1..5                16, 8, 4, 2, 1 lanes, at most 8 edges a lane
- * and the contributions read most often are the first ones: the first `cached`
- * sit in shared memory (on RMAT-22, 55,000 of 4.2 M vertices take 57 % of all
- * reads). */
-#define WGM_PR_BINS 6
-#define WGM_PR_BATCH 4
+/* Rows by rank; the contributions read most often are the first ones: the
+ * first `cached` sit in shared memory (on RMAT-22, 41,000 of 4.2 M vertices
+ * take 56 % of all reads). */
 struct wgm_pr_args {
-  int V, rows;       /* vertices; those with edges */
-  const int *prow;   /* [rows+1] by rank */
-  const int *pcol;   /* [E] ranks */
-  const int *order;  /* [V] vertex of each rank */
+  int V;
+  wgm_rank_rows R;
   float *pr;         /* [V] output, by vertex */
   float *contrib;    /* [2][stride] pr/deg of the previous iteration, by rank */
   size_t stride;     /* >= V, whole 16-byte words */
   float *dang;       /* [3 lines] by iteration mod 3: dangling mass; word 1 (int):
-                        units handed out */
-  int wide, parts;   /* wide rows; their parts of at most part_edges each */
-  int part_edges;
-  const int *part_row; /* [parts] rank of a part's row */
-  const int *row_part; /* [wide+1] first part of a row */
+                        work handed out */
   float *part;       /* [parts] sums */
   int *part_done;    /* [wide] parts summed, zero between iterations */
-  int bin_row[WGM_PR_BINS + 1];  /* first rank of each bin, then `rows` */
-  int bin_task[WGM_PR_BINS + 1]; /* first warp task of each bin, then their count */
   int cached;        /* contributions kept in dynamic shared memory */
   int iterations;
   float damping;
@@ -2377,9 +2487,42 @@ struct wgm_pr_args {
 
 extern __shared__ float wgm_pr_cache[];
 
-__device__ __forceinline__ float wgm_pr_gather(const float *cin, int cached, int u) {
-  return u < 0 ? 0.f : u < cached ? wgm_pr_cache[u] : __ldca(&cin[u]);
-}
+/* One iteration over the rows (wgm_rank_pull). */
+struct wgm_pr_op {
+  const wgm_pr_args &a;
+  const float *cin;
+  float *cout;
+  float base;
+  bool last;
+  __device__ __forceinline__ bool skip(int) const { return false; }
+  __device__ __forceinline__ float none() const { return 0.f; }
+  __device__ __forceinline__ float edge(int u, int) const {
+    return u < 0 ? 0.f : u < a.cached ? wgm_pr_cache[u] : __ldca(&cin[u]);
+  }
+  __device__ __forceinline__ float join(float x, float y) const { return x + y; }
+  __device__ __forceinline__ void row(int k, int deg, float sum) const {
+    const float p = base + a.damping * sum;
+    cout[k] = p / (float)deg;
+    if (last) a.pr[__ldg(&a.R.order[k])] = p;
+  }
+  __device__ __forceinline__ void part(int unit, int, float x) const { a.part[unit] = x; }
+  /* the last part to finish adds up its row's, in their order */
+  __device__ __forceinline__ void after_part(int, int k, int n) const {
+    const int lane = wgm_lane(), p0 = __ldg(&a.R.row_part[k]);
+    const int m = __ldg(&a.R.row_part[k + 1]) - p0;
+    int done = 0;
+    if (lane == 0) done = wgm_atom_add_acqrel_gpu(&a.part_done[k], 1) == m - 1;
+    if (!__shfl_sync(WGM_FULL, done, 0)) return;
+    float y = 0.f;
+    for (int i = lane; i < m; i += 32) y += __ldcg(&a.part[p0 + i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(WGM_FULL, y, o);
+    if (lane == 0) {
+      a.part_done[k] = 0;
+      row(k, n, y);
+    }
+  }
+};
 
 /* pr' = (1-d)/V + d*(sum_{u in N(v)} pr[u]/deg(u) + dangling/V).  Phases:
  * (0) init; (1,t) iteration t, one barrier each.  Every row is summed by the
@@ -2398,20 +2541,23 @@ __device__ __forceinline__ float wgm_pr_gather(const float *cin, int cached, int
 static __device__ int wgm_phase_pagerank(const wgm_launch &Lc, wgm_cta *c, const wgm_pr_args &a,
                                          wgm_step cur, wgm_step *nxt) {
   const wgm_split s(c);
-  const int V = a.V, lane = s.lane;
+  const int V = a.V;
   const float d = a.damping;
   const int t = cur.round;
   if (cur.target == 0) {
     const float p = 1.0f / (float)V;
-    for (int k = s.tid; k < a.rows; k += s.nth)
-      a.contrib[k] = p / (float)(__ldg(&a.prow[k + 1]) - __ldg(&a.prow[k]));
+    for (int k = s.tid; k < a.R.rows; k += s.nth)
+      a.contrib[k] = p / (float)(__ldg(&a.R.prow[k + 1]) - __ldg(&a.R.prow[k]));
     if (a.iterations == 0)
       for (int v = s.tid; v < V; v += s.nth) a.pr[v] = p;
     if (c->id == 0 && threadIdx.x < 3) {
       a.dang[threadIdx.x * WGM_LINE] = a.dangling * p;
       reinterpret_cast<int *>(a.dang)[threadIdx.x * WGM_LINE + 1] = 0;
     }
-    for (int k = s.tid; k < a.wide; k += s.nth) a.part_done[k] = 0;
+    for (int k = s.tid; k < a.R.wide; k += s.nth) a.part_done[k] = 0;
+    /* a vertex without edges of its own gives nothing to rows that name it */
+    for (size_t k = a.R.rows + s.tid; k < a.stride; k += s.nth)
+      a.contrib[k] = a.contrib[a.stride + k] = 0.f;
     *nxt = {1, 0};
     return WGM_PHASE_NEXT;
   }
@@ -2436,138 +2582,10 @@ static __device__ int wgm_phase_pagerank(const wgm_launch &Lc, wgm_cta *c, const
     }
     __syncthreads();
   }
-  auto finish = [&](int k, int deg, float sum) {
-    const float p = base + d * sum;
-    cout[k] = p / (float)deg;
-    if (last) a.pr[__ldg(&a.order[k])] = p;
-  };
-  /* Sum of the edges r0 + l, + g, ... below r0 + n, eight in flight; the next
-   * eight columns are read beside this step's contributions. */
-  auto row_sum = [&](int r0, int n, int l, int g) {
-    float sum = 0.f;
-    int u[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) u[q] = l + q * g < n ? __ldcs(&a.pcol[r0 + l + q * g]) : -1;
-    for (int i = l; __any_sync(WGM_FULL, i < n); i += 8 * g) {
-      float v[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++) v[q] = wgm_pr_gather(cin, cached, u[q]);
-      const int j = i + 8 * g;
-#pragma unroll
-      for (int q = 0; q < 8; q++) u[q] = j + q * g < n ? __ldcs(&a.pcol[r0 + j + q * g]) : -1;
-#pragma unroll
-      for (int q = 0; q < 8; q++) sum += v[q];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float y = __shfl_xor_sync(WGM_FULL, sum, o);
-      if (o < g) sum += y;
-    }
-    return sum;
-  };
-  /* Work in order of falling degree: a part of a wide row, a row of bin 0, or
-   * `batch` warp tasks of the other bins.  Three quarters go round the warps
-   * by number, the rest are handed out as warps get free. */
-  const int long_units = a.parts + a.bin_task[1];
-  const int tasks = a.bin_task[WGM_PR_BINS] - a.bin_task[1];
-  const int batch = max(1, min(WGM_PR_BATCH, tasks / (4 * s.NW)));
-  const int units = long_units + (tasks + batch - 1) / batch;
-  const int fixed = (int)(3LL * units / 4 / s.NW) * s.NW; /* whole rounds */
-  int unit = s.gw;
-  while (unit < units) {
-    int next = unit + s.NW;
-    if (next >= fixed) {
-      if (lane == 0) next = atomicAdd(grab, 1);
-      next = __shfl_sync(WGM_FULL, next, 0) + max(fixed, s.NW);
-    }
-    if (unit < a.parts) {
-      const int k = __ldg(&a.part_row[unit]), p0 = __ldg(&a.row_part[k]);
-      const int m = __ldg(&a.row_part[k + 1]) - p0;
-      const int r0 = __ldg(&a.prow[k]), n = __ldg(&a.prow[k + 1]) - r0;
-      const int off = (unit - p0) * a.part_edges;
-      const float x = row_sum(r0 + off, min(a.part_edges, n - off), lane, 32);
-      int done = 0;
-      if (lane == 0) {
-        a.part[unit] = x;
-        done = wgm_atom_add_acqrel_gpu(&a.part_done[k], 1) == m - 1;
-      }
-      if (__shfl_sync(WGM_FULL, done, 0)) { /* the row's last part: all are there */
-        float y = 0.f;
-        for (int i = lane; i < m; i += 32) y += __ldcg(&a.part[p0 + i]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(WGM_FULL, y, o);
-        if (lane == 0) {
-          a.part_done[k] = 0;
-          finish(k, n, y);
-        }
-      }
-    } else if (unit < long_units) {
-      const int k = a.bin_row[0] + unit - a.parts;
-      const int r0 = __ldg(&a.prow[k]), n = __ldg(&a.prow[k + 1]) - r0;
-      const float x = row_sum(r0, n, lane, 32);
-      if (lane == 0) finish(k, n, x);
-    } else {
-      const int x0 = a.bin_task[1] + (unit - long_units) * batch;
-      const int x1 = min(x0 + batch, a.bin_task[WGM_PR_BINS]);
-      /* rows of at most 8 edges a lane, in a pipeline over the tasks: the row
-       * bounds of task x + 2 and the columns of task x + 1 are read beside
-       * the contributions of task x */
-      auto locate = [&](int x, int &k, int &g, int &r0, int &n) {
-        int bn = 1, first = a.bin_row[1], task = a.bin_task[1], end = a.bin_row[2];
-#pragma unroll
-        for (int q = 2; q < WGM_PR_BINS; q++)
-          if (x >= a.bin_task[q]) {
-            bn = q;
-            first = a.bin_row[q];
-            task = a.bin_task[q];
-            end = a.bin_row[q + 1];
-          }
-        g = 32 >> bn;
-        k = first + ((x - task) << bn) + (lane >> (5 - bn));
-        r0 = n = 0;
-        if (x < x1 && k < end) {
-          r0 = __ldg(&a.prow[k]);
-          n = __ldg(&a.prow[k + 1]) - r0;
-        }
-      };
-      auto columns = [&](int g, int r0, int n, int (&u)[8]) {
-        const int l = lane & (g - 1);
-#pragma unroll
-        for (int q = 0; q < 8; q++) u[q] = l + q * g < n ? __ldcs(&a.pcol[r0 + l + q * g]) : -1;
-      };
-      int k0, g0, r0, n0, k1, g1, r1, n1, u[8];
-      locate(x0, k0, g0, r0, n0);
-      locate(x0 + 1, k1, g1, r1, n1);
-      columns(g0, r0, n0, u);
-      for (int x = x0; x < x1; x++) {
-        float v[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) v[q] = wgm_pr_gather(cin, cached, u[q]);
-        columns(g1, r1, n1, u);
-        int k2, g2, r2, n2;
-        locate(x + 2, k2, g2, r2, n2);
-        float sum = 0.f;
-#pragma unroll
-        for (int q = 0; q < 8; q++) sum += v[q];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float y = __shfl_xor_sync(WGM_FULL, sum, o);
-          if (o < g0) sum += y;
-        }
-        if (n0 > 0 && (lane & (g0 - 1)) == 0) finish(k0, n0, sum);
-        k0 = k1;
-        g0 = g1;
-        n0 = n1;
-        k1 = k2;
-        g1 = g2;
-        r1 = r2;
-        n1 = n2;
-      }
-    }
-    unit = next;
-  }
+  wgm_pr_op op{a, cin, cout, base, last};
+  wgm_rank_pull<false, float>(a.R, s, grab, op);
   if (last)
-    for (int k = a.rows + s.tid; k < V; k += s.nth) a.pr[__ldg(&a.order[k])] = base;
+    for (int k = a.R.rows + s.tid; k < V; k += s.nth) a.pr[__ldg(&a.R.order[k])] = base;
   *nxt = {1, t + 1};
   return WGM_PHASE_NEXT;
 }

@@ -86,10 +86,13 @@ struct wgm_app {
   int cq_cap = 0;
   int source = 0;
   float damping = 0.85f;
-  /* PageRank: rows and columns by falling degree (wgm_pr_layout) */
-  int *d_pr_order = nullptr, *d_pr_row = nullptr, *d_pr_col = nullptr;
-  int *d_pr_parts = nullptr; /* part_row, row_part, part sums, part_done */
-  int pr_rows = 0, pr_wide = 0, pr_parts = 0, pr_part_edges = 256, pr_bin_row[7] = {}, pr_bin_task[7] = {};
+  /* PageRank, Pannotia SSSP: rows, columns and weights by falling degree
+   * (wgm_rank_layout) */
+  int *d_rk_order = nullptr, *d_rk_row = nullptr, *d_rk_col = nullptr, *d_rk_wt = nullptr;
+  int *d_rk_of = nullptr, *d_rk_x = nullptr; /* Pannotia SSSP: rank of a vertex, cost by rank */
+  int *d_rk_parts = nullptr; /* part_row, row_part, part sums, part_done */
+  int rk_rows = 0, rk_wide = 0, rk_parts = 0, rk_part_edges = 256, rk_bin_row[7] = {},
+      rk_bin_task[7] = {};
   int pr_smem = 0, pr_smem_block = 0, pr_smem_per_sm = 0; /* wgm_pagerank_smem's answer */
   int iterations = 20;
   int bc_sources = 0; /* betweenness centrality: sources 0 .. bc_sources-1 */

@@ -397,10 +397,9 @@ cudaError_t wgm_launch_bfs_cta(const wgm_lonestar_args &a, int W, const int *ell
   return cudaGetLastError();
 }
 
-/* 40 registers (no spills): six 256-thread CTAs per SM instead of four */
-__global__ void __maxnreg__(40) wgm_k_psssp(wgm_launch L, wgm_psssp_args a) {
-  WGM_PERSISTENT_PROLOGUE
-  WGM_DRIVE(wgm_phase_pannotia_sssp(L, &c, a, &sm, cur, nxt));
+__global__ void __launch_bounds__(1024) wgm_k_psssp(wgm_launch L, wgm_psssp_args a) {
+  WGM_PERSISTENT_PROLOGUE_TASKS
+  WGM_DRIVE(wgm_phase_pannotia_sssp(L, &c, a, cur, nxt));
   WGM_PERSISTENT_EPILOGUE
 }
 
@@ -433,39 +432,68 @@ cudaError_t wgm_pagerank_smem(int block, int per_sm, int *bytes) {
   return e;
 }
 
-/* PageRank's layout: ranks, then rows and columns by rank (a warp per row). */
-__global__ void __launch_bounds__(256) wgm_k_pr_rank(int V, const int *order, int *rank) {
+/* Layout by rank: ranks, then columns and weights. */
+__global__ void __launch_bounds__(256) wgm_k_rank_of(int V, const int *order, int *rank) {
   for (int k = blockIdx.x * 256 + threadIdx.x; k < V; k += gridDim.x * 256) rank[order[k]] = k;
 }
-__global__ void __launch_bounds__(256) wgm_k_pr_rows(int rows, const int *row, const int *col,
-                                                     const int *order, const int *rank,
-                                                     const int *prow, int *pcol) {
+__global__ void __launch_bounds__(256) wgm_k_rank_rows(wgm_rank_rows R, const int *row,
+                                                       const int *col, const int *wt,
+                                                       const int *rank, int *pcol, int *pwt,
+                                                       int *wmin) {
   const int nw = gridDim.x * 8, lane = wgm_lane();
-  for (int k0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 32; k0 < rows; k0 += nw * 32) {
-    const int k = k0 + lane;
-    const int from = k < rows ? row[order[k]] : 0, to = k < rows ? prow[k] : 0;
-    const int n = k < rows ? prow[k + 1] - to : 0;
+  int least = INT_MAX;
+  /* parts of wide rows, then four rows at a time */
+  const long long units = R.parts + (R.rows - R.wide + 3LL) / 4;
+  for (long long unit = blockIdx.x * 8 + (threadIdx.x >> 5); unit < units; unit += nw) {
+    int from = 0, to = 0, n = 0;
+    if (unit < R.parts) {
+      const int k = R.part_row[unit], off = (int)(unit - R.row_part[k]) * R.part_edges;
+      if (lane == 0) {
+        from = row[R.order[k]] + off;
+        to = R.prow[k] + off;
+        n = min(R.part_edges, R.prow[k + 1] - to);
+      }
+    } else {
+      const long long k = R.wide + (unit - R.parts) * 4 + lane;
+      if (lane < 4 && k < R.rows) {
+        from = row[R.order[k]];
+        to = R.prow[k];
+        n = R.prow[k + 1] - to;
+      }
+    }
     const int incl = wgm_warp_incl_scan(n), total = __shfl_sync(WGM_FULL, incl, 31);
     const int off = incl - n;
     for (int w = 0; w < total; w += 128) {
-      int c[4], at[4];
+      int c[4], x[4], at[4];
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const int sl = w + 32 * q + lane, own = wgm_owner_of(off, min(sl, total - 1));
         const int e = __shfl_sync(WGM_FULL, from - off, own) + sl;
         at[q] = __shfl_sync(WGM_FULL, to - off, own) + sl;
         c[q] = sl < total ? __ldcs(&col[e]) : -1;
+        x[q] = wt && sl < total ? __ldcs(&wt[e]) : 0;
       }
 #pragma unroll
       for (int q = 0; q < 4; q++)
-        if (c[q] >= 0) pcol[at[q]] = __ldg(&rank[c[q]]);
+        if (c[q] >= 0) {
+          pcol[at[q]] = __ldg(&rank[c[q]]);
+          if (wt) {
+            pwt[at[q]] = x[q];
+            least = min(least, x[q]);
+          }
+        }
     }
   }
+  if (wt) {
+    least = __reduce_min_sync(WGM_FULL, least);
+    if (lane == 0) atomicMin(wmin, least);
+  }
 }
-cudaError_t wgm_launch_pr_layout(int V, int rows, const int *row, const int *col, const int *order,
-                                 int *rank, const int *prow, int *pcol, cudaStream_t s) {
-  wgm_k_pr_rank<<<std::min((V + 255) / 256, 1216), 256, 0, s>>>(V, order, rank);
-  wgm_k_pr_rows<<<1216, 256, 0, s>>>(rows, row, col, order, rank, prow, pcol);
+cudaError_t wgm_launch_rank_layout(int V, const wgm_rank_rows &R, const int *row, const int *col,
+                                   const int *wt, int *rank, int *pcol, int *pwt, int *wmin,
+                                   cudaStream_t s) {
+  wgm_k_rank_of<<<std::min((V + 255) / 256, 1216), 256, 0, s>>>(V, R.order, rank);
+  wgm_k_rank_rows<<<1216, 256, 0, s>>>(R, row, col, wt, rank, pcol, pwt, wmin);
   return cudaGetLastError();
 }
 

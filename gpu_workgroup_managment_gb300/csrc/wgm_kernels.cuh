@@ -80,8 +80,9 @@ cudaError_t wgm_launch_color_async(const wgm_launch &L, const wgm_color_args &a,
 cudaError_t wgm_launch_psssp(const wgm_launch &L, const wgm_psssp_args &a, int grid, int block,
                              cudaStream_t s);
 cudaError_t wgm_pagerank_smem(int block, int per_sm, int *bytes);
-cudaError_t wgm_launch_pr_layout(int V, int rows, const int *row, const int *col, const int *order,
-                                 int *rank, const int *prow, int *pcol, cudaStream_t s);
+cudaError_t wgm_launch_rank_layout(int V, const wgm_rank_rows &R, const int *row, const int *col,
+                                   const int *wt, int *rank, int *pcol, int *pwt, int *wmin,
+                                   cudaStream_t s);
 cudaError_t wgm_launch_pagerank(const wgm_launch &L, const wgm_pr_args &a, int grid, int block,
                                 cudaStream_t s);
 cudaError_t wgm_launch_octree(const wgm_launch &L, const wgm_octree_args &a, int grid, int block,

@@ -87,7 +87,7 @@ __device__ __forceinline__ void wgm_mega_run_app(const wgm_launch &L, const wgm_
       break;
     case WGM_K_PSSSP:
       wgm_drive(L, pc, start, sync, [&](wgm_step cur, wgm_step *nxt) {
-        return wgm_phase_pannotia_sssp(L, pc, A.psssp, sm, cur, nxt);
+        return wgm_phase_pannotia_sssp(L, pc, A.psssp, cur, nxt);
       });
       break;
     case WGM_K_PAGERANK:
