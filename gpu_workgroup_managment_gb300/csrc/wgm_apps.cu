@@ -136,7 +136,24 @@ static void wgm_build_hubs(int V, const int32_t *row_ptr, const int *order, int 
   }
 }
 
+/* A word of the runtime's mapped round counts, while there are any. */
+static void wgm_rounds_take(wgm_app *a) {
+  std::lock_guard<std::mutex> hold(a->rt->rounds_mutex);
+  for (int i = 0; i < WGM_ROUNDS_SLOTS; i++)
+    if (!a->rt->rounds_used[i]) {
+      a->rt->rounds_used[i] = true;
+      a->rounds_slot = i;
+      __atomic_store_n(a->rt->rounds + i, 0, __ATOMIC_RELEASE);
+      return;
+    }
+}
+
 static void wgm_app_free_buffers(wgm_app *a) {
+  if (a->rounds_slot >= 0) {
+    std::lock_guard<std::mutex> hold(a->rt->rounds_mutex);
+    a->rt->rounds_used[a->rounds_slot] = false;
+    a->rounds_slot = -1;
+  }
   void *ptrs[] = {a->d_row,     a->d_col,       a->d_wt,      a->d_node_value, a->d_out,
                   a->d_wl_start, a->d_wl_cnt,   a->d_wl_u,
                   a->d_cnt,       a->d_stamp,   a->d_stop,
@@ -630,7 +647,9 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
   const size_t V = (size_t)a->V, E = (size_t)a->E;
   cudaError_t e = wgm_dmalloc(&a->d_row, V + 1);
   if (e == cudaSuccess) e = wgm_dmalloc(&a->d_col, E);
-  if (e == cudaSuccess) e = wgm_dmalloc(&a->d_rounds, 1);
+  /* centrality's kernels count rounds with atomics: those stay on the device */
+  if (kind != WGM_APP_PANNOTIA_BC) wgm_rounds_take(a);
+  if (e == cudaSuccess && a->rounds_slot < 0) e = wgm_dmalloc(&a->d_rounds, 1);
   if (e == cudaSuccess && wgm_needs_weights(kind)) e = wgm_dmalloc(&a->d_wt, E);
   switch (kind) {
     case WGM_APP_LONESTAR_BFS:
@@ -838,6 +857,10 @@ static wgm_hubs wgm_hubs_view(const wgm_app *a) {
   return h;
 }
 
+static int *wgm_rounds_out(const wgm_app *a) {
+  return a->rounds_slot >= 0 ? a->rt->rounds_dev + a->rounds_slot : a->d_rounds;
+}
+
 /* Fill the kernel arguments of the app (also used by the megakernel). */
 int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
   if (a->kind == WGM_APP_PLUGIN) return WGM_ERR_INVALID; /* its own megakernel */
@@ -915,7 +938,7 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.cnt = a->d_cnt;
       x.stamp = a->d_stamp;
       x.source = a->source;
-      x.levels_out = a->d_rounds;
+      x.levels_out = wgm_rounds_out(a);
       x.packed = a->kind == WGM_APP_LONESTAR_SSSP ? 1 : 0;
       return WGM_OK;
     }
@@ -928,7 +951,7 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.color = (int *)a->d_out;
       x.hubs = wgm_hubs_view(a);
       x.hub_threshold = a->hub_threshold;
-      x.rounds_out = a->d_rounds;
+      x.rounds_out = wgm_rounds_out(a);
       x.trow = a->d_trow ? a->d_trow : a->d_row;
       x.tcol = a->d_tcol ? a->d_tcol : a->d_col;
       x.pending = a->d_stamp;
@@ -955,7 +978,7 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.wide = a->d_mis_wide;
       x.wide_cap = (int)wgm_mis_wide_cap(a);
       x.scan = wgm_mis_scan_edges(a);
-      x.rounds_out = a->d_rounds;
+      x.rounds_out = wgm_rounds_out(a);
       return WGM_OK;
     }
     case WGM_APP_PANNOTIA_SSSP: {
@@ -968,7 +991,7 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.stop = a->d_stop;
       x.wmin = a->d_cnt;
       x.source = a->source;
-      x.rounds_out = a->d_rounds;
+      x.rounds_out = wgm_rounds_out(a);
       return WGM_OK;
     }
     case WGM_APP_PAGERANK: {
@@ -1235,8 +1258,7 @@ extern "C" int wgm_run_persistent(wgm_runtime *rt, wgm_app *a, int num_wgs,
       cudaEventElapsedTime(&ms, rt->ev0, rt->ev1);
       stats->kernel_ms = ms;
       int rounds = 0;
-      if (cudaMemcpy(&rounds, a->d_rounds, 4, cudaMemcpyDeviceToHost) == cudaSuccess)
-        stats->rounds = rounds;
+      if (wgm_app_rounds(a, &rounds) == WGM_OK) stats->rounds = rounds;
     }
     return WGM_OK;
   }
@@ -1477,6 +1499,12 @@ extern "C" int wgm_app_rounds(wgm_app *a, int *rounds) {
   if (a->kind == WGM_APP_PLUGIN) {
     *rounds = 0;
     return a->vt.rounds ? a->vt.rounds(a->vt.user, rounds) : WGM_OK;
+  }
+  if (a->rounds_slot >= 0) {
+    cudaError_t e = cudaStreamSynchronize(a->rt->stream);
+    if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
+    *rounds = __atomic_load_n(a->rt->rounds + a->rounds_slot, __ATOMIC_ACQUIRE);
+    return WGM_OK;
   }
   int h = 0;
   cudaError_t e = cudaMemcpyAsync(&h, a->d_rounds, 4, cudaMemcpyDeviceToHost, a->rt->stream);

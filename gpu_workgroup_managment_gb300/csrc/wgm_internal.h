@@ -7,11 +7,14 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
 #include <vector>
 
 #include "../../include/wgm.h"
 #include "wgm_common.h"
 #include "wgm_device.cuh"
+
+#define WGM_ROUNDS_SLOTS 256
 
 struct wgm_runtime {
   wgm_config cfg{};
@@ -21,6 +24,11 @@ struct wgm_runtime {
   wgm_dev_state *st = nullptr;        /* device */
   wgm_host_flags *hf = nullptr;       /* mapped pinned host memory */
   wgm_host_flags *hf_dev = nullptr;   /* its device alias */
+  /* Round counts in mapped memory behind the flags, a word per app: the
+   * host reads one without a copy (about 10 us of a 60 us call). */
+  int *rounds = nullptr, *rounds_dev = nullptr;
+  std::mutex rounds_mutex;
+  bool rounds_used[WGM_ROUNDS_SLOTS] = {};
   char *d_scratch = nullptr;          /* 64 bytes of small kernel outputs */
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t tev0 = nullptr, tev1 = nullptr; /* wgm_timer_* */
@@ -58,6 +66,7 @@ struct wgm_app {
   int4 *d_mis_wide = nullptr;
   float *d_contrib = nullptr, *d_dang = nullptr;
   int *d_rounds = nullptr;
+  int rounds_slot = -1; /* word of rt->rounds that the kernels write instead, if any */
   /* colour: in-edge CSR when the graph is not symmetric (else the graph) */
   int *d_trow = nullptr, *d_tcol = nullptr;
   int2 *d_tcv = nullptr; /* colour: in-edges beside their neighbour's value */

@@ -112,9 +112,13 @@ extern "C" int wgm_runtime_create(const wgm_config *cfg, wgm_runtime **out) {
   RT_TRY(cudaStreamCreateWithFlags(&rt->stream, cudaStreamNonBlocking));
   RT_TRY(cudaMalloc((void **)&rt->st, sizeof(wgm_dev_state)));
   RT_TRY(cudaMemset(rt->st, 0, sizeof(wgm_dev_state)));
-  RT_TRY(cudaHostAlloc((void **)&rt->hf, sizeof(wgm_host_flags), cudaHostAllocMapped));
+  RT_TRY(cudaHostAlloc((void **)&rt->hf,
+                       sizeof(wgm_host_flags) + WGM_ROUNDS_SLOTS * sizeof(int),
+                       cudaHostAllocMapped));
   wgm_clear_flags(rt->hf);
   RT_TRY(cudaHostGetDevicePointer((void **)&rt->hf_dev, rt->hf, 0));
+  rt->rounds = (int *)(rt->hf + 1);
+  rt->rounds_dev = (int *)(rt->hf_dev + 1);
   RT_TRY(cudaMalloc((void **)&rt->d_scratch, 64));
   RT_TRY(cudaMemset(rt->d_scratch, 0, 64));
   RT_TRY(cudaEventCreate(&rt->ev0));
