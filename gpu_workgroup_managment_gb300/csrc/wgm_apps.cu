@@ -665,7 +665,7 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_wl_cnt, 2 * (size_t)a->wl_cap);
       if (e == cudaSuccess && kind == WGM_APP_LONESTAR_SSSP)
         e = wgm_dmalloc(&a->d_wl_u, 2 * (size_t)a->wl_cap);
-      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cnt, 3 * WGM_LINE);
+      if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cnt, 6 * WGM_LINE);
       /* SSSP: 64-bit {level tag, distance} words (wgm_ls_chunk PACK) */
       if (e == cudaSuccess && kind == WGM_APP_LONESTAR_SSSP) e = wgm_dmalloc(&a->d_stamp, 2 * V);
       break;
@@ -936,6 +936,7 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.cap = a->wl_cap;
       x.piece = a->piece;
       x.cnt = a->d_cnt;
+      x.grab = a->d_cnt + 3 * WGM_LINE;
       x.stamp = a->d_stamp;
       x.source = a->source;
       x.levels_out = wgm_rounds_out(a);
