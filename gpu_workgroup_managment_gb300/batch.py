@@ -95,7 +95,7 @@ class Batch:
 
     def configure_teams(self, team_edges: int = 0, max_team: int = 0) -> None:
         """A job of E edges runs on ceil(E / team_edges) CTAs, at most max_team
-        (0 = defaults: total edges / grid, a quarter of the grid)."""
+        (0 = defaults: total edges / (2 x grid), a quarter of the grid)."""
         check(lib.wgm_batch_configure_teams(self._h, team_edges, max_team), "configure_teams")
 
     def configure_local(self, rounds: int) -> None:

@@ -465,13 +465,17 @@ static int wgm_batch_grid(wgm_batch *b, int *grid) {
 }
 
 /* Team sizes and the slot queue for a grid of `grid` CTAs: a job of E edges
- * gets ceil(E / team_edges) CTAs, at most max_team; its slots (job, rank)
+ * gets ceil(E / team_edges) CTAs, at most max_team (by default two CTAs for
+ * each one's even share: a launch ends with its longest chain of levels, the
+ * SSSP of the largest grids, and larger teams shorten it - 128 graphs of 2^8
+ * to 2^16.5 vertices 3.50 -> 3.17 ms, 512 of 2^8 to 2^15 2.95 -> 2.65; four
+ * cost more CTA time than they save, 3.28 and 2.75); its slots (job, rank)
  * follow each other in the queue, largest job first. */
 static int wgm_batch_teams(wgm_batch *b, int grid) {
   long long etot = 0;
   for (auto &j : b->jobs) etot += b->gE[j.graph];
   long long te = b->team_edges > 0 ? b->team_edges
-                                   : std::max(1LL << 15, (etot + grid - 1) / std::max(grid, 1));
+                                   : std::max(1LL << 15, (etot / 2 + grid - 1) / std::max(grid, 1));
   int mt = b->max_team > 0 ? std::min(b->max_team, grid) : std::max(1, grid / 4);
   std::vector<int2> slots;
   for (int q = 0; q < b->njobs; q++) {

@@ -374,7 +374,8 @@ int wgm_batch_graph_offsets(wgm_batch *b, int64_t *row_off, int64_t *col_off);
 /* threads per CTA, CTAs per SM (0: occupancy maximum), piece (0: per graph). */
 int wgm_batch_configure(wgm_batch *b, int threads_per_cta, int ctas_per_sm, int piece);
 /* Team sizing: a job of E edges runs on ceil(E / team_edges) CTAs, at most
- * max_team.  0 selects the defaults: total edges / grid, a quarter of the grid. */
+ * max_team.  0 selects the defaults: total edges / (2 x grid), a quarter of the
+ * grid. */
 int wgm_batch_configure_teams(wgm_batch *b, int64_t team_edges, int max_team);
 int wgm_batch_team_info(wgm_batch *b, int64_t *team_edges, int *max_team);
 /* Warp-local continuation: after its share of a level a warp relaxes the
