@@ -17,9 +17,17 @@
  * windows of 32 edges: lane j of a window handles edge slot w+j, its owner is
  * found with one __reduce_or_sync and a clz, so col[] is read coalesced and no
  * CTA-wide __syncthreads is needed inside the edge loop (the reference's
- * block scan is serial in work-item 0, bfs.cl:43-51).  Vertices whose degree
- * exceeds `hub_threshold` ("hubs") skip the warp path; their edges are spread
- * over every warp of the grid so one hub never stalls a level.
+ * block scan is serial in work-item 0, bfs.cl:43-51).  Long rows never stall
+ * a level: Lonestar rows are queued in pieces, colour spreads the edges of
+ * vertices above `hub_threshold` over every warp, MIS hands rows past twice
+ * that to the whole grid, and PageRank and Pannotia SSSP cut theirs into parts.
+ *
+ * Two habits of the memory system shape what follows (measured on GB300).
+ * Words that many SMs read and write at once cost about 50 ns an access, so a
+ * mark is stored once, a count or a minimum leaves a group once, and hot words
+ * are read through the L1 (a barrier's acquire empties it).  And a dependent
+ * access costs 305 cycles from the L2 (an atomic 707) against 28 from shared
+ * memory, so short phases are counted in round trips.
  */
 #ifndef WGM_GRAPH_CUH
 #define WGM_GRAPH_CUH
@@ -91,34 +99,6 @@ __device__ __forceinline__ void wgm_hub_window(const wgm_hubs &hb, const int *ro
   wgm_hub_slot(w, lane, &h, &e);
   (void)row;
   f(valid, h, e);
-}
-
-/* Reduce `v` over the lanes holding hub h0 and hub h0+1 separately; lane 0
- * receives both results.  op: 0 = max (int bits), 1 = min (int bits), 2 = fp32 sum. */
-__device__ __forceinline__ void wgm_two_seg_reduce(bool first, int v, float fv, int op,
-                                                   int *r0, int *r1, float *f0,
-                                                   float *f1) {
-  int a = first ? v : (op == 0 ? INT_MIN : INT_MAX);
-  int b = first ? (op == 0 ? INT_MIN : INT_MAX) : v;
-  float fa = first ? fv : 0.f, fb = first ? 0.f : fv;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    int ya = __shfl_xor_sync(WGM_FULL, a, o), yb = __shfl_xor_sync(WGM_FULL, b, o);
-    float ga = __shfl_xor_sync(WGM_FULL, fa, o), gb = __shfl_xor_sync(WGM_FULL, fb, o);
-    if (op == 0) {
-      a = max(a, ya);
-      b = max(b, yb);
-    } else if (op == 1) {
-      a = min(a, ya);
-      b = min(b, yb);
-    }
-    fa += ga;
-    fb += gb;
-  }
-  *r0 = a;
-  *r1 = b;
-  *f0 = fa;
-  *f1 = fb;
 }
 
 /* First edge of each lane's row [e, end) that `hit` accepts (warp-collective;
@@ -1321,13 +1301,11 @@ static __device__ int wgm_phase_color(const wgm_launch &Lc, wgm_cta *c, const wg
           const int v = __ldg(&a.hubs.ids[h]);
           cntv = __ldg(&a.node_value[__ldg(&a.col[e])]) > __ldg(&a.node_value[v]) ? 1 : 0;
         }
-        int m0, m1;
-        float f0, f1;
-        wgm_two_seg_reduce(h == h0, 0, (float)cntv, 2, &m0, &m1, &f0, &f1);
+        const int n0 = __reduce_add_sync(WGM_FULL, h == h0 ? cntv : 0);
+        const int n1 = __reduce_add_sync(WGM_FULL, h == h0 ? 0 : cntv);
         if (lane == 0) {
-          if (f0 > 0.f) atomicAdd(&a.pending[__ldg(&a.hubs.ids[h0])], (int)f0);
-          if (f1 > 0.f && h0 + 1 < a.hubs.H)
-            atomicAdd(&a.pending[__ldg(&a.hubs.ids[h0 + 1])], (int)f1);
+          if (n0 > 0) atomicAdd(&a.pending[__ldg(&a.hubs.ids[h0])], n0);
+          if (n1 > 0 && h0 + 1 < a.hubs.H) atomicAdd(&a.pending[__ldg(&a.hubs.ids[h0 + 1])], n1);
         }
       });
     }

@@ -86,7 +86,8 @@ typedef struct wgm_config {
   int discovery_extra_rounds;  /* discovery.cl:43 (reference mode) */
   int barrier_kind;            /* WGM_BARRIER_* */
   int tree_fanin;              /* groups per leaf of WGM_BARRIER_TREE */
-  int hub_threshold;           /* degree above which edges spread grid-wide */
+  int hub_threshold;           /* colour: degree above which edges spread grid-wide
+                                  (MIS: edges of a vertex, at twice this) */
   uint64_t spin_timeout_ns;    /* budget of every device wait */
   uint64_t run_timeout_ns;     /* host budget of one blocking run; then abort */
   uint64_t discovery_window_ns;/* ticket discovery closing window */
