@@ -162,7 +162,7 @@ static void wgm_app_free_buffers(wgm_app *a) {
                   a->d_oct_input, a->d_oct_second, a->d_oct_pools, a->d_oct_tree,
                   a->d_oct_ctr, a->d_oct_locks, a->d_oct_heads,
                   a->d_c4_board, a->d_c4_nodes, a->d_c4_pool, a->d_c4_locks,
-                  a->d_c4_heads, a->d_c4_ctr, a->d_ell, a->d_up_bits, a->d_up_cnt, a->d_up_wide, a->d_cb_ord, a->d_cb_colour,
+                  a->d_c4_heads, a->d_c4_ctr, a->d_bc64, a->d_ell, a->d_up_bits, a->d_up_cnt, a->d_up_wide, a->d_cb_ord, a->d_cb_colour,
                   a->d_cb_crank, a->d_cb_list, a->d_cb_hub, a->d_cb_cnt, a->d_hub_rank, a->d_hub_max, a->d_tcv, a->d_tcv4, a->d_cmax, a->d_cq,
                   a->d_cqctl};
   for (void *p : ptrs)
@@ -722,6 +722,7 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_contrib, 2 * V);
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_wl_u, V);
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_wl_start, V + 2);
+      if (e == cudaSuccess && a->bc_mode == 1) e = wgm_dmalloc(&a->d_bc64, V);
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cnt, 3 * WGM_LINE);
       break;
   }
@@ -795,7 +796,8 @@ static int wgm_bc_cta_launch(wgm_runtime *rt, wgm_app *a, cudaStream_t s) {
   std::memset(&A, 0, sizeof(A));
   int st = wgm_app_fill_mega(a, &A);
   if (st) return st;
-  cudaError_t e = wgm_launch_bc_cta(A.bc, a->d_cnt + 2 * WGM_LINE, WGM_BC_CTA_THREADS, s);
+  cudaError_t e = wgm_launch_bc_cta(A.bc, a->d_bc64, a->d_cnt + 2 * WGM_LINE, WGM_BC_CTA_THREADS,
+                                    s);
   if (e != cudaSuccess) return wgm_cuda_fail(rt, e);
   return WGM_OK;
 }

@@ -2366,7 +2366,7 @@ struct wgm_psssp_args {
   int *x;          /* [V] output cost (sssp.h:168 reads x) */
   int *stop;       /* [6 lines] by round mod 3: work handed out; then least cost that
                       changed (INT_MAX: none) */
-  const int *wmin; /* least edge weight */
+  const int *wmin; /* least edge weight; negative where a pass has to take every row */
   int source;
   int *rounds_out;
 };
@@ -2754,7 +2754,9 @@ static __device__ int wgm_phase_bc(const wgm_launch &Lc, wgm_cta *c, const wgm_b
  * sigma, the level lists and their starts in shared memory (20 bytes per
  * vertex) and __syncthreads as the level barrier; bc gathers the
  * dependencies with global float atomics.  Same arithmetic as wgm_phase_bc,
- * no grid barrier at all: sources, not levels, are the parallel units.  For
+ * no grid barrier at all: sources, not levels, are the parallel units.  A
+ * vertex's dependencies are added in double precision (a sum over thousands of
+ * sources in an order that changes from run to run) and rounded once.  For
  * graphs of at most WGM_BC_CTA_MAX_V vertices. */
 #define WGM_BC_CTA_MAX_V 10240
 
@@ -2798,8 +2800,8 @@ __device__ __forceinline__ void wgm_bc_edges(const int *col, int start, int deg,
   }
 }
 
-static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, int src, int *dist, float *rho,
-                                         float *sig, int *order, int *ls, int *s_cnt) {
+static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, double *bc64, int src, int *dist,
+                                         float *rho, float *sig, int *order, int *ls, int *s_cnt) {
   const int V = a.V, lane = wgm_lane(), nw = blockDim.x >> 5;
   for (int i = threadIdx.x; i < V; i += blockDim.x) {
     dist[i] = i == src ? 0 : -1;
@@ -2880,7 +2882,7 @@ static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, int src, int *dis
       wgm_bc_edges(a.tcol, start, deg, fv, [&](bool valid, int w, float fo) {
         if (valid && dist[w] == l - 1) atomicAdd(&sig[w], rho[w] * fo);
       });
-      if (have && v != src && sv != 0.f) atomicAdd(&a.bc[v], sv / WGM_BC_SCALE);
+      if (have && v != src && sv != 0.f) atomicAdd(&bc64[v], (double)(sv / WGM_BC_SCALE));
     }
     __syncthreads();
   }

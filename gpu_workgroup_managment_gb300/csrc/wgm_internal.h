@@ -105,6 +105,7 @@ struct wgm_app {
   int pr_smem = 0, pr_smem_block = 0, pr_smem_per_sm = 0; /* wgm_pagerank_smem's answer */
   int iterations = 20;
   int bc_sources = 0; /* betweenness centrality: sources 0 .. bc_sources-1 */
+  double *d_bc64 = nullptr; /* centrality, sources over CTAs: the sums */
   int bc_mode = 0;    /* 0: one source at a time over the grid, 1: sources over CTAs */
   bool has_node_values = false;
   /* octree (WGM_APP_OCTREE): d_out holds the particles, V their count */

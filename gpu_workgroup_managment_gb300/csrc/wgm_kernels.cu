@@ -479,7 +479,8 @@ __global__ void __launch_bounds__(256) wgm_k_rank_rows(wgm_rank_rows R, const in
           pcol[at[q]] = __ldg(&rank[c[q]]);
           if (wt) {
             pwt[at[q]] = x[q];
-            least = min(least, x[q]);
+            /* a weight that can wrap a cost rules the test out, like a negative one */
+            least = min(least, x[q] > INT_MAX - WGM_PANNOTIA_BIG ? -1 : x[q]);
           }
         }
     }
@@ -535,7 +536,8 @@ __global__ void __launch_bounds__(1024) wgm_k_bc(wgm_launch L, wgm_bc_args a) {
 /* Betweenness centrality, sources spread over CTAs (wgm_bc_cta_source):
  * a plain grid of resident CTAs pulling sources from a queue, no discovery
  * and no grid barrier. */
-__global__ void __launch_bounds__(1024) wgm_k_bc_cta(wgm_bc_args a, int *queue) {
+__global__ void __launch_bounds__(1024) wgm_k_bc_cta(wgm_bc_args a, double *bc64,
+                                                     int *queue) {
   extern __shared__ int wgm_bc_dyn[];
   __shared__ int s_cnt[3], s_src; /* vertices found; two grab counters */
   int *dist = wgm_bc_dyn;
@@ -549,9 +551,17 @@ __global__ void __launch_bounds__(1024) wgm_k_bc_cta(wgm_bc_args a, int *queue) 
     const int src = s_src;
     __syncthreads();
     if (src >= a.num_sources) break;
-    wgm_bc_cta_source(a, src, dist, rho, sig, order, ls, s_cnt);
+    wgm_bc_cta_source(a, bc64, src, dist, rho, sig, order, ls, s_cnt);
     if (threadIdx.x == 0 && a.rounds_out) atomicAdd(a.rounds_out, 1);
   }
+  /* the last CTA to finish rounds the sums */
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_src = atomicAdd(queue + 1, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s_src) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < a.V; i += blockDim.x) a.bc[i] = (float)__ldcg(&bc64[i]);
 }
 
 /* Standalone connect-four look-ahead (connect_four.cl:350-487 without a
@@ -618,7 +628,8 @@ cudaError_t wgm_launch_bc(const wgm_launch &L, const wgm_bc_args &a, int grid, i
   wgm_k_bc<<<grid, block, 0, s>>>(L, a);
   return cudaGetLastError();
 }
-cudaError_t wgm_launch_bc_cta(const wgm_bc_args &a, int *queue, int block, cudaStream_t s) {
+cudaError_t wgm_launch_bc_cta(const wgm_bc_args &a, double *bc64, int *queue, int block,
+                              cudaStream_t s) {
   const size_t smem = (size_t)a.V * 20 + 16;
   cudaError_t e = cudaFuncSetAttribute(wgm_k_bc_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
@@ -628,11 +639,11 @@ cudaError_t wgm_launch_bc_cta(const wgm_bc_args &a, int *queue, int block, cudaS
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  e = cudaMemsetAsync(a.bc, 0, (size_t)a.V * 4, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(queue, 0, 4, s);
+  e = cudaMemsetAsync(bc64, 0, (size_t)a.V * 8, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(queue, 0, 8, s);
   if (e == cudaSuccess && a.rounds_out) e = cudaMemsetAsync(a.rounds_out, 0, 4, s);
   if (e != cudaSuccess) return e;
-  wgm_k_bc_cta<<<per_sm * sms, block, smem, s>>>(a, queue);
+  wgm_k_bc_cta<<<per_sm * sms, block, smem, s>>>(a, bc64, queue);
   return cudaGetLastError();
 }
 cudaError_t wgm_launch_c4(const wgm_launch &L, const wgm_c4_args &a, int grid, int block,
