@@ -943,6 +943,7 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.source = a->source;
       x.levels_out = wgm_rounds_out(a);
       x.packed = a->kind == WGM_APP_LONESTAR_SSSP ? 1 : 0;
+      x.low_degree = x.packed && a->E <= 8LL * a->V ? 1 : 0;
       return WGM_OK;
     }
     case WGM_APP_PANNOTIA_COLOR: {

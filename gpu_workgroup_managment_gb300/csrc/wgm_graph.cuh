@@ -202,6 +202,7 @@ struct wgm_lonestar_args {
   int source;
   int *levels_out; /* number of levels run (written by group 0) */
   int packed = 0;  /* SSSP relaxes packed words (wgm_ls_chunk PACK) */
+  int low_degree = 0; /* SSSP: average degree at most 8 (wgm_ls_narrow) */
   int *grab = nullptr; /* [3 lines] chunks of a wide level handed out, by level mod 3 */
 };
 
@@ -559,13 +560,79 @@ __device__ __forceinline__ bool wgm_ls_chunk(const int *row, const int *col, con
   return ok;
 }
 
+/* Relax the lanes' rows (rs, d, at most 32 edges in all; source distance
+ * `from`), an edge per lane; the lanes come back with the vertices that they
+ * improved and claimed (u; row rs, d; d = 0: none). */
+__device__ __forceinline__ unsigned wgm_ls_relax32(const wgm_lonestar_args &a, int L, int &u,
+                                                   int &rs, int &d, unsigned from) {
+  const int lane = wgm_lane();
+  unsigned long long *word = reinterpret_cast<unsigned long long *>(a.stamp);
+  const int incl = wgm_warp_incl_scan(d), total = __shfl_sync(WGM_FULL, incl, 31);
+  const int off = incl - d, own = wgm_owner_of(off, min(lane, total - 1));
+  const int e = __shfl_sync(WGM_FULL, rs - off, own) + lane;
+  from = __shfl_sync(WGM_FULL, from, own);
+  bool f = lane < total;
+  u = f ? __ldg(&a.col[e]) : -1;
+  const unsigned wk = f ? __ldg(&a.wt[e]) : WGM_LONESTAR_INF;
+  f = f && wk < WGM_LONESTAR_INF /* sssp.cl:120 */ && (unsigned)u < (unsigned)a.V /* bfs.cl:116 */;
+  rs = d = 0;
+  if (f) {
+    rs = __ldg(&a.row[u]);
+    d = __ldg(&a.row[u + 1]);
+    const unsigned alt = from + wk;
+    const unsigned long long old =
+        atomicMin(&word[u], ((unsigned long long)alt << 32) | (unsigned)L);
+    f = (unsigned)(old >> 32) > alt && (unsigned)old != (unsigned)L;
+    d = f ? max(d - rs, 0) : 0; /* a vertex without edges is not queued */
+  }
+  return __ballot_sync(WGM_FULL, d > 0);
+}
+
+/* SSSP, a narrow level of low-degree vertices: the lanes' pieces (start, deg,
+ * src; at most 32 edges in all), then the vertices they improve at once
+ * instead of in the next level, as long as their edges fit the warp, up to
+ * WGM_LS_HOPS times.  A hop is two atomics' round trips, a level also the
+ * list's and the barrier's.  A vertex is given up before it is relaxed: one
+ * 64-bit AND clears its level tag and returns its distance, so an improvement
+ * that comes later finds another tag and queues the vertex, and one that came
+ * before is in the distance that is relaxed - every improvement is still
+ * followed by a relaxation that reads it.  509x517 grid: 759 levels, 3.95 ms
+ * without hops; 581 and 3.45 with one, 514 and 3.39 with two, 481 and 3.16
+ * with three, 455 and 3.33 with five (more hops relax distances that are not
+ * final yet). */
+#define WGM_LS_HOPS 3
+__device__ __forceinline__ bool wgm_ls_narrow(const wgm_lonestar_args &a, int L, int start, int deg,
+                                              int src, const wgm_ls_out &o) {
+  const int lane = wgm_lane(), P = a.piece;
+  unsigned long long *word = reinterpret_cast<unsigned long long *>(a.stamp);
+  int u = src, rs = start, d = deg;
+  unsigned from = 0;
+  if (d > 0) from = __ldcg(reinterpret_cast<const unsigned *>(a.stamp) + 2 * (size_t)src + 1);
+  unsigned m = wgm_ls_relax32(a, L, u, rs, d, from);
+  for (int hop = 0; hop < WGM_LS_HOPS && m; hop++) {
+    if (__reduce_add_sync(WGM_FULL, d) > 32) break;
+    if (d > 0) from = (unsigned)(atomicAnd(&word[u], 0xffffffff00000000ull) >> 32);
+    m = wgm_ls_relax32(a, L, u, rs, d, from);
+  }
+  if (m == 0) return true;
+  const int np = d > 0 ? (d + P - 1) / P : 0, incl = wgm_warp_incl_scan(np);
+  const int n = __shfl_sync(WGM_FULL, incl, 31);
+  int base = 0;
+  if (lane == 0) base = wgm_out_reserve(o, n);
+  base = __shfl_sync(WGM_FULL, base, 0);
+  if (base + n > o.cap) return false;
+  for (int q = 0; q < np; q++)
+    wgm_out_put(o, base + incl - np + q, rs + q * P, min(P, d - q * P), u);
+  return true;
+}
+
 /* One piece on one warp, an edge per lane: the walker of a level with no more
  * pieces than warps (a high-diameter graph's).  Such a level is a chain of
  * dependent round trips, so everything that is not one is left out: no owner
  * search, no scans, and the pushes are counted by ballots unless a vertex
  * has several pieces.  A piece of more than 8 edges keeps the pre-check: on
  * a dense graph most of its atomics would fail, thousands of them on a hub's
- * word.  A 509x517 grid's SSSP: 5.8 -> 5.1 us a level. */
+ * word.  (SSSP of low average degree goes by wgm_ls_narrow.) */
 template <bool SSSP>
 __device__ __forceinline__ bool wgm_ls_piece(const wgm_lonestar_args &a, int L, int start, int deg,
                                              int src, const wgm_ls_out &o) {
@@ -651,7 +718,8 @@ __device__ __forceinline__ bool wgm_ls_level(const wgm_launch &Lc, wgm_cta *c,
   o.o_u = a.wl_u ? a.wl_u + out_off : nullptr;
   o.cap = a.cap;
   bool ok = true;
-  if (n <= NW && (!SSSP || a.packed))
+  const bool narrow = SSSP && a.packed && a.low_degree && n <= 8 * NW;
+  if (n <= NW && (!SSSP || a.packed) && !narrow)
     return gw >= n || wgm_ls_piece<SSSP>(a, L, first.x, first.y, first.z, o);
   /* pieces per warp: 32, or fewer when the list is short, so a small
    * frontier spreads over every warp instead of queueing on a few */
@@ -672,7 +740,9 @@ __device__ __forceinline__ bool wgm_ls_level(const wgm_launch &Lc, wgm_cta *c,
       deg = __ldcg(&i_cnt[i]);
       if (SSSP) src = __ldcg(&i_u[i]);
     }
-    if (SSSP && a.packed)
+    if (narrow && __reduce_add_sync(WGM_FULL, deg) <= 32)
+      ok &= wgm_ls_narrow(a, L, start, deg, src, o);
+    else if (SSSP && a.packed)
       ok &= wgm_ls_chunk<SSSP, true, SSSP>(a.row, a.col, a.wt,
                                            reinterpret_cast<unsigned *>(a.stamp), a.stamp, a.V,
                                            a.piece, L, start, deg, src, o);
