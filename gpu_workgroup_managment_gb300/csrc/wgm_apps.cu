@@ -722,7 +722,7 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_contrib, 2 * V);
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_wl_u, V);
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_wl_start, V + 2);
-      if (e == cudaSuccess && a->bc_mode == 1) e = wgm_dmalloc(&a->d_bc64, V);
+      if (e == cudaSuccess && a->bc_mode == 1) e = wgm_dmalloc(&a->d_bc64, V + 1);
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cnt, 3 * WGM_LINE);
       break;
   }
@@ -787,7 +787,13 @@ extern "C" int wgm_app_set_bc_mode(wgm_app *a, int32_t mode) {
   return WGM_OK;
 }
 
-#define WGM_BC_CTA_THREADS 1024
+/* Threads a source: small graphs fill the SM with more CTAs, each with a
+ * cheaper barrier; once shared memory (20 bytes a vertex) holds only two CTAs,
+ * 1024 threads fill it.  256 / 512 / 1024 threads, ms: RMAT 500 0.062 / 0.066
+ * / 0.086, 1000 0.113 / 0.130 / 0.174, 2000 0.549 / 0.493 / 0.631, 3000 0.716
+ * / 0.548 / 0.647, 4096 3.71 / 2.35 / 2.12; grid 24 x 24 0.141 / 0.145 /
+ * 0.272. */
+static int wgm_bc_cta_threads(int V) { return V <= 1024 ? 256 : V <= 3584 ? 512 : 1024; }
 /* Sources spread over CTAs (bc_mode 1): a plain launch of resident CTAs, no
  * discovery and no host handshake, so the launch generation is untouched. */
 static int wgm_bc_cta_launch(wgm_runtime *rt, wgm_app *a, cudaStream_t s) {
@@ -796,8 +802,8 @@ static int wgm_bc_cta_launch(wgm_runtime *rt, wgm_app *a, cudaStream_t s) {
   std::memset(&A, 0, sizeof(A));
   int st = wgm_app_fill_mega(a, &A);
   if (st) return st;
-  cudaError_t e = wgm_launch_bc_cta(A.bc, a->d_bc64, a->d_cnt + 2 * WGM_LINE, WGM_BC_CTA_THREADS,
-                                    s);
+  cudaError_t e = wgm_launch_bc_cta(A.bc, a->d_bc64, (int)a->E, a->E <= 4LL * a->V,
+                                    wgm_bc_cta_threads(a->V), s);
   if (e != cudaSuccess) return wgm_cuda_fail(rt, e);
   return WGM_OK;
 }

@@ -2831,48 +2831,89 @@ static __device__ int wgm_phase_bc(const wgm_launch &Lc, wgm_cta *c, const wgm_b
 #define WGM_BC_CTA_MAX_V 10240
 
 
-/* Vertices a warp takes of a level of n at a time.  They are handed out, for a
- * hub's edges keep a warp long: RMAT-12, all sources, 4.14 ms with 32
- * vertices a warp in turn, 2.72 handed out (512 threads), 2.38 with 1024, a
- * quarter of a warp's share at a time 2.31 (an eighth 2.38), and with two
- * windows of edges in flight 2.18 (four 2.22).  A vertex at a time, 128 of
- * its edges together, was slower (2.72): most rows fill less than a warp. */
+/* Vertices a warp takes of a level of n at a time: at least `few` (two windows
+ * of edges at the graph's average degree), and a quarter of an even share.  A
+ * level of more than one share per warp is handed out, for a hub's edges
+ * keep a warp long: RMAT-12, all sources, 4.14 ms with 32 vertices a warp in
+ * turn, 2.72 handed out (512 threads), 2.38 with 1024, a quarter of a warp's
+ * share at a time 2.31 (an eighth 2.38), and with two windows of edges in
+ * flight 2.18 (four 2.22).  A vertex at a time, 128 of its edges together,
+ * was slower (2.72): most rows fill less than a warp.  An edge's row comes
+ * from a table of the window's row starts (five dependent shuffles: 2.25,
+ * the table 2.12).  EVEN, for graphs of degree up to 4 on average, whose rows
+ * differ little: 32 vertices a warp in turn and one window, fewer
+ * instructions a level (grid 24 x 24 0.149 -> 0.141 ms, 15 x 8 59 -> 53 us).
+ * What bounds small graphs is the chain of a level, about 2000 cycles. */
 #define WGM_BC_SHARE 4
 #define WGM_BC_K 2 /* 32-edge windows in flight */
-__device__ __forceinline__ int wgm_bc_per(int n, int nw) {
-  return max(1, min(32, (n + WGM_BC_SHARE * nw - 1) / (WGM_BC_SHARE * nw)));
+__device__ __forceinline__ int wgm_bc_per(int n, int nw, int few) {
+  return min(32, max(few, (n + WGM_BC_SHARE * nw - 1) / (WGM_BC_SHARE * nw)));
 }
-__device__ __forceinline__ int wgm_bc_grab(int *counter, int per) {
+/* First vertex of the warp's next share; `turn` counts its shares. */
+__device__ __forceinline__ int wgm_bc_next(int *counter, int n, int per, int warp, int nw,
+                                           int turn) {
+  if (n <= nw * per) return turn ? n : warp * per;
   int b = 0;
   if (wgm_lane() == 0) b = atomicAdd(counter, per);
   return __shfl_sync(WGM_FULL, b, 0);
 }
 
 /* f(valid, target, x of its row's lane) for the edges of the lanes' rows. */
-template <class F>
-__device__ __forceinline__ void wgm_bc_edges(const int *col, int start, int deg, float x, F &&f) {
-  const int lane = wgm_lane(), incl = wgm_warp_incl_scan(deg);
-  const int total = __shfl_sync(WGM_FULL, incl, 31), off = incl - deg;
-  for (int w = 0; w < total; w += 32 * WGM_BC_K) {
-    int j[WGM_BC_K];
-    float xo[WGM_BC_K];
-    bool in[WGM_BC_K];
+template <int K, class F>
+__device__ __forceinline__ void wgm_bc_windows(const int *col, int base, int off, int deg,
+                                               int total, int w, float x, int *tab, F &f) {
+  const int lane = wgm_lane();
+  unsigned mm[K];
+  int j[K], own[K];
+  float xo[K];
+  bool in[K];
 #pragma unroll
-    for (int q = 0; q < WGM_BC_K; q++) {
-      const int sl = w + 32 * q + lane, own = wgm_owner_of(off, min(sl, total - 1));
-      const int e = __shfl_sync(WGM_FULL, start - off, own) + sl;
-      xo[q] = __shfl_sync(WGM_FULL, x, own);
-      in[q] = sl < total;
-      j[q] = in[q] ? __ldg(&col[e]) : 0;
-    }
-#pragma unroll
-    for (int q = 0; q < WGM_BC_K; q++) f(in[q], j[q], xo[q]);
+  for (int q = 0; q < K; q++) {
+    const int w1 = w + 32 * q;
+    const bool mine = deg > 0 && off < w1 + 32 && off + deg > w1;
+    const int pos = mine ? max(off - w1, 0) : 0;
+    mm[q] = __reduce_or_sync(WGM_FULL, mine ? 1u << pos : 0u);
+    if (mine) tab[32 * q + pos] = lane;
   }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    mm[q] &= 0xffffffffu >> (31 - lane);
+    own[q] = tab[32 * q + (mm[q] ? 31 - __clz(mm[q]) : 0)] & 31;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    const int sl = w + 32 * q + lane, e = __shfl_sync(WGM_FULL, base, own[q]) + sl;
+    xo[q] = __shfl_sync(WGM_FULL, x, own[q]);
+    in[q] = sl < total;
+    j[q] = in[q] ? __ldg(&col[e]) : 0;
+  }
+#pragma unroll
+  for (int q = 0; q < K; q++) f(in[q], j[q], xo[q]);
+}
+template <int K, class F>
+__device__ __forceinline__ void wgm_bc_edges(const int *col, int start, int deg, float x, int *tab,
+                                             F &&f) {
+  const int incl = wgm_warp_incl_scan(deg);
+  const int total = __shfl_sync(WGM_FULL, incl, 31), off = incl - deg;
+  int w = 0;
+  if (K > 1)
+    for (; total - w > 32; w += 32 * K)
+      wgm_bc_windows<K>(col, start - off, off, deg, total, w, x, tab, f);
+  for (; w < total; w += 32) wgm_bc_windows<1>(col, start - off, off, deg, total, w, x, tab, f);
 }
 
+template <bool EVEN>
 static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, double *bc64, int src, int *dist,
-                                         float *rho, float *sig, int *order, int *ls, int *s_cnt) {
-  const int V = a.V, lane = wgm_lane(), nw = blockDim.x >> 5;
+                                         float *rho, float *sig, int *order, int *ls, int *s_cnt,
+                                         int *tab, int few) {
+  const int V = a.V, lane = wgm_lane(), warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  tab += warp * 32 * WGM_BC_K;
+  /* by level mod 3: vertices found, shares handed out; by backtrack step mod
+   * 3: shares handed out.  A level clears the next one's, so it ends in one
+   * barrier. */
+  int *found_n = s_cnt, *shares = s_cnt + 3, *back = s_cnt + 6;
   for (int i = threadIdx.x; i < V; i += blockDim.x) {
     dist[i] = i == src ? 0 : -1;
     rho[i] = i == src ? WGM_BC_SCALE : 0.f;
@@ -2882,15 +2923,17 @@ static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, double *bc64, int
     order[0] = src;
     ls[0] = 0;
     ls[1] = 1;
-    s_cnt[0] = 0;
-    s_cnt[1] = 0;
+    for (int k = 0; k < 9; k++) s_cnt[k] = 0;
   }
   __syncthreads();
   int L = 0, S = 0, n = 1;
   for (;;) {
-    const int S1 = S + n, per = wgm_bc_per(n, nw);
-    for (;;) {
-      const int b = wgm_bc_grab(&s_cnt[1], per);
+    const int S1 = S + n, per = EVEN ? 32 : wgm_bc_per(n, nw, few);
+    int *count = &found_n[L % 3];
+    if (threadIdx.x == 0) found_n[(L + 1) % 3] = shares[(L + 1) % 3] = 0;
+    for (int turn = 0;; turn++) {
+      const int b = EVEN ? 32 * (warp + nw * turn)
+                         : wgm_bc_next(&shares[L % 3], n, per, warp, nw, turn);
       if (b >= n) break;
       const int k = b + lane;
       int start = 0, deg = 0;
@@ -2901,7 +2944,7 @@ static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, double *bc64, int
         deg = __ldg(&a.row[v + 1]) - start;
         rv = rho[v];
       }
-      wgm_bc_edges(a.col, start, deg, rv, [&](bool valid, int w, float ro) {
+      wgm_bc_edges<EVEN ? 1 : WGM_BC_K>(a.col, start, deg, rv, tab, [&](bool valid, int w, float ro) {
         bool found = false;
         if (valid) {
           int d = dist[w];
@@ -2912,31 +2955,24 @@ static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, double *bc64, int
           }
           if (d == L + 1) atomicAdd(&rho[w], ro);
         }
-        wgm_warp_push(found, w, &s_cnt[0], order + S1, V - S1, false);
+        wgm_warp_push(found, w, count, order + S1, V - S1, false);
       });
     }
     __syncthreads();
-    const int n2 = s_cnt[0];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      s_cnt[0] = 0;
-      s_cnt[1] = 0;
-      ls[L + 2] = S1 + n2;
-    }
-    __syncthreads();
+    const int n2 = *count;
+    if (threadIdx.x == 0) ls[L + 2] = S1 + n2;
     if (n2 == 0) break;
     S = S1;
     n = n2;
     L++;
   }
+  __syncthreads(); /* the last level's start */
   for (int l = L; l >= 0; l--) {
-    const int B = ls[l], E = ls[l + 1], per = wgm_bc_per(E - B, nw);
-    /* the levels' grab counters take turns: the other one is cleared here,
-     * after its last grab and before its next */
-    int *grab = &s_cnt[1 + ((L - l) & 1)];
-    if (threadIdx.x == 0) s_cnt[1 + ((L - l + 1) & 1)] = 0;
-    for (;;) {
-      const int b = B + wgm_bc_grab(grab, per);
+    const int B = ls[l], E = ls[l + 1], step = (L - l) % 3, per = EVEN ? 32 : wgm_bc_per(E - B, nw, few);
+    if (!EVEN && threadIdx.x == 0) back[(step + 1) % 3] = 0;
+    for (int turn = 0;; turn++) {
+      const int b = B + (EVEN ? 32 * (warp + nw * turn)
+                              : wgm_bc_next(&back[step], E - B, per, warp, nw, turn));
       if (b >= E) break;
       const int k = b + lane;
       const bool have = lane < per && k < E;
@@ -2949,7 +2985,7 @@ static __device__ void wgm_bc_cta_source(const wgm_bc_args &a, double *bc64, int
         sv = sig[v];
         fv = (WGM_BC_SCALE + sv) / rho[v];
       }
-      wgm_bc_edges(a.tcol, start, deg, fv, [&](bool valid, int w, float fo) {
+      wgm_bc_edges<EVEN ? 1 : WGM_BC_K>(a.tcol, start, deg, fv, tab, [&](bool valid, int w, float fo) {
         if (valid && dist[w] == l - 1) atomicAdd(&sig[w], rho[w] * fo);
       });
       if (have && v != src && sv != 0.f) atomicAdd(&bc64[v], (double)(sv / WGM_BC_SCALE));

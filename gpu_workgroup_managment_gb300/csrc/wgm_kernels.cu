@@ -534,33 +534,35 @@ __global__ void __launch_bounds__(1024) wgm_k_bc(wgm_launch L, wgm_bc_args a) {
 }
 
 /* Betweenness centrality, sources spread over CTAs (wgm_bc_cta_source):
- * a plain grid of resident CTAs pulling sources from a queue, no discovery
- * and no grid barrier. */
-__global__ void __launch_bounds__(1024) wgm_k_bc_cta(wgm_bc_args a, double *bc64,
-                                                     int *queue) {
+ * a plain grid of resident CTAs, each with its own first source and the others
+ * from a queue (one word after the sums), no discovery and no grid barrier. */
+template <bool EVEN>
+__global__ void __launch_bounds__(1024, 2) wgm_k_bc_cta(wgm_bc_args a, double *bc64, int few) {
+  int *queue = reinterpret_cast<int *>(bc64 + a.V); /* sources, CTAs done */
   extern __shared__ int wgm_bc_dyn[];
-  __shared__ int s_cnt[3], s_src; /* vertices found; two grab counters */
+  __shared__ int tab[32 * 32 * WGM_BC_K];
+  __shared__ int s_cnt[9], s_src; /* wgm_bc_cta_source's counters */
   int *dist = wgm_bc_dyn;
   float *rho = reinterpret_cast<float *>(dist + a.V);
   float *sig = rho + a.V;
   int *order = reinterpret_cast<int *>(sig + a.V);
   int *ls = order + a.V;
-  for (;;) {
-    if (threadIdx.x == 0) s_src = atomicAdd(queue, 1);
+  for (int src = blockIdx.x; src < a.num_sources;) {
+    wgm_bc_cta_source<EVEN>(a, bc64, src, dist, rho, sig, order, ls, s_cnt, tab, few);
+    if (threadIdx.x == 0) s_src = gridDim.x + atomicAdd(queue, 1);
     __syncthreads();
-    const int src = s_src;
-    __syncthreads();
-    if (src >= a.num_sources) break;
-    wgm_bc_cta_source(a, bc64, src, dist, rho, sig, order, ls, s_cnt);
-    if (threadIdx.x == 0 && a.rounds_out) atomicAdd(a.rounds_out, 1);
+    src = s_src;
   }
-  /* the last CTA to finish rounds the sums */
-  __threadfence();
+  /* the last CTA to finish rounds the sums; the sources are all done then */
   __syncthreads();
-  if (threadIdx.x == 0) s_src = atomicAdd(queue + 1, 1) == (int)gridDim.x - 1;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_src = atomicAdd(queue + 1, 1) == (int)gridDim.x - 1;
+  }
   __syncthreads();
   if (!s_src) return;
   __threadfence();
+  if (threadIdx.x == 0 && a.rounds_out) *a.rounds_out = a.num_sources;
   for (int i = threadIdx.x; i < a.V; i += blockDim.x) a.bc[i] = (float)__ldcg(&bc64[i]);
 }
 
@@ -628,22 +630,23 @@ cudaError_t wgm_launch_bc(const wgm_launch &L, const wgm_bc_args &a, int grid, i
   wgm_k_bc<<<grid, block, 0, s>>>(L, a);
   return cudaGetLastError();
 }
-cudaError_t wgm_launch_bc_cta(const wgm_bc_args &a, double *bc64, int *queue, int block,
+cudaError_t wgm_launch_bc_cta(const wgm_bc_args &a, double *bc64, int edges, bool even, int block,
                               cudaStream_t s) {
   const size_t smem = (size_t)a.V * 20 + 16;
-  cudaError_t e = cudaFuncSetAttribute(wgm_k_bc_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const auto kernel = even ? wgm_k_bc_cta<true> : wgm_k_bc_cta<false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   int per_sm = 0, dev = 0, sms = 0;
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wgm_k_bc_cta, block, smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
   if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  e = cudaMemsetAsync(bc64, 0, (size_t)a.V * 8, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(queue, 0, 8, s);
-  if (e == cudaSuccess && a.rounds_out) e = cudaMemsetAsync(a.rounds_out, 0, 4, s);
+  e = cudaMemsetAsync(bc64, 0, (size_t)a.V * 8 + 8, s);
   if (e != cudaSuccess) return e;
-  wgm_k_bc_cta<<<per_sm * sms, block, smem, s>>>(a, bc64, queue);
+  const int few = (int)min(32LL, max(1LL, 32LL * WGM_BC_K * a.V / max(edges, 1)));
+  const int grid = max(1, min(per_sm * sms, a.num_sources));
+  kernel<<<grid, block, smem, s>>>(a, bc64, few);
   return cudaGetLastError();
 }
 cudaError_t wgm_launch_c4(const wgm_launch &L, const wgm_c4_args &a, int grid, int block,
