@@ -800,13 +800,14 @@ __device__ __forceinline__ void wgm_bfs_cta(const wgm_lonestar_args &a, const in
     wgm_bfs_dyn[in] = a.source;
   }
   __syncthreads();
-  int L = 1, c0 = 1, c1 = 2, c2 = 0; /* L, L + 1, L + 2 mod 3 */
+  int L = 1;
+  wgm_proto_levels w3{1, 2, 0}; /* L, L + 1, L + 2 mod 3 */
   for (;;) {
-    const int n = s_cnt[c0];
+    const int n = s_cnt[w3.now];
     if (n == 0 || L > V + 1) break;
     if (threadIdx.x == 0) {
-      s_cnt[c2] = 0;
-      s_cnt[4 + c2] = 0;
+      s_cnt[w3.size_to_clear()] = 0;
+      s_cnt[4 + w3.flag_to_clear()] = 0; /* not the one that late warps still read below */
     }
     /* Claim N neighbours for level L and queue the new ones: N bit words
      * read together, N claims together, one reservation. */
@@ -828,7 +829,7 @@ __device__ __forceinline__ void wgm_bfs_cta(const wgm_lonestar_args &a, const in
         found += w[q];
       }
       if (found == 0) return;
-      int k = atomicAdd(&s_cnt[c1], found);
+      int k = atomicAdd(&s_cnt[w3.next], found);
 #pragma unroll
       for (int q = 0; q < N; q++) {
         if (!w[q]) continue;
@@ -854,12 +855,12 @@ __device__ __forceinline__ void wgm_bfs_cta(const wgm_lonestar_args &a, const in
           u[4 * q + 2] = r.z;
           u[4 * q + 3] = r.w;
         }
-        if (u[0] != WGM_BFS_PAD) s_cnt[4 + c0] = 1;
+        if (u[0] != WGM_BFS_PAD) s_cnt[4 + w3.now] = 1;
         reach(u);
       } else {
         const int s = __ldg(&a.row[v]);
         const int d = max(__ldg(&a.row[v + 1]) - s, 0);
-        if (d > 0) s_cnt[4 + c0] = 1;
+        if (d > 0) s_cnt[4 + w3.now] = 1;
         for (int j = 0; j < d; j += 4) {
           int u[4];
 #pragma unroll
@@ -871,13 +872,10 @@ __device__ __forceinline__ void wgm_bfs_cta(const wgm_lonestar_args &a, const in
     __syncthreads();
     /* the grid form queues no vertex without edges (it has no pieces): a
      * level that walked no edge is where its frontier was empty */
-    if (!s_cnt[4 + c0]) break;
+    if (!s_cnt[4 + w3.now]) break;
     L++;
-    int t = c0;
-    c0 = c1;
-    c1 = c2;
-    c2 = t;
-    t = in;
+    w3.step();
+    int t = in;
     in = out;
     out = t;
     t = in_sp;

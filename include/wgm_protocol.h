@@ -61,4 +61,24 @@ WGM_PROTO bool wgm_proto_offer_kill(int *num_groups, int *to_kill, int kid) {
   return true;
 }
 
+/* A loop of levels with one barrier a level keeps the words of three levels,
+ * by level mod 3: of the running level (`now`), of the one after it and of
+ * the one before.  Sizes are filled while the level before runs and read at
+ * the top of their own level; flags are raised while their own level runs
+ * and read after its barrier.  A thread still reading those may find the
+ * first one at the top of the next level already, so that one clears, for
+ * each kind, the words that nobody has read since the barrier before and
+ * nobody fills before the next. */
+struct wgm_proto_levels {
+  int now, next, last;
+  WGM_PROTO int size_to_clear() const { return last; } /* read at the top of `last` */
+  WGM_PROTO int flag_to_clear() const { return next; } /* read after the level before `last` */
+  WGM_PROTO void step() {
+    const int t = now;
+    now = next;
+    next = last;
+    last = t;
+  }
+};
+
 #endif
