@@ -2360,7 +2360,9 @@ __device__ __forceinline__ void wgm_rank_pull(const wgm_rank_rows &R, const wgm_
       const int k = part ? __ldg(&R.part_row[unit]) : R.bin_row[0] + unit - R.parts;
       const int r0 = __ldg(&R.prow[k]), n = __ldg(&R.prow[k + 1]) - r0;
       const int off = part ? (unit - __ldg(&R.row_part[k])) * R.part_edges : 0;
-      if (!op.skip(k)) {
+      /* other parts' warps may be lowering the word that skip reads: one answer
+       * for the warp, which works the row together */
+      if (!(op.SKIPS && __any_sync(WGM_FULL, op.skip(k)))) {
         const T x = long_row(r0 + off, part ? min(R.part_edges, n - off) : n);
         if (lane == 0) {
           if (part) op.part(unit, k, x);
@@ -2444,6 +2446,7 @@ struct wgm_psssp_op {
   int *xr;
   int bound;           /* costs up to here cannot fall in this pass */
   int least = INT_MAX; /* least cost that this thread lowered */
+  static constexpr bool SKIPS = true;
   __device__ __forceinline__ bool skip(int k) const { return __ldcg(&xr[k]) <= bound; }
   __device__ __forceinline__ int none() const { return INT_MAX; }
   __device__ __forceinline__ int edge(int u, int w) const {
@@ -2562,6 +2565,7 @@ struct wgm_pr_op {
   float *cout;
   float base;
   bool last;
+  static constexpr bool SKIPS = false;
   __device__ __forceinline__ bool skip(int) const { return false; }
   __device__ __forceinline__ float none() const { return 0.f; }
   __device__ __forceinline__ float edge(int u, int) const {
