@@ -1042,7 +1042,9 @@ __device__ __forceinline__ void wgm_bfs_up_level(const wgm_cta *c, const wgm_lon
       bool f = false;
       for (long long x = (long long)__ldg(&b.trow[v]) + WGM_BFS_UP_SCAN + 128LL * sub;
            x < end && !f; x += 128LL * S) {
-        if (__ldcg(&nxt[v >> 5]) >> (v & 31) & 1u) break; /* another warp has it */
+        /* another warp has it: it may be setting the bit now, so one answer for
+         * the warp, which looks together */
+        if (__any_sync(WGM_FULL, __ldcg(&nxt[v >> 5]) >> (v & 31) & 1u)) break;
         int j[4];
         bool h4 = false;
 #pragma unroll
