@@ -476,10 +476,11 @@ static int wgm_bfs_up_layout(wgm_app *a, const int32_t *row_ptr) {
     if (e == cudaSuccess) e = wgm_dmalloc(&a->d_up_cnt, 3 * (size_t)WGM_LINE);
     if (e == cudaSuccess) e = wgm_dmalloc(&a->d_up_wide, (size_t)(a->E / WGM_BFS_UP_SCAN) + 2);
   }
-  /* dist is free before a run: the in-degrees pass through it */
+  /* the worklist is free before a run: the in-degrees pass through it (the
+   * result stays the last run's) */
   if (e == cudaSuccess)
     e = wgm_launch_in_edges(V, used, a->d_row, a->d_col, a->d_trow, a->d_tcol, a->d_up_wide,
-                            (int *)a->d_out, st);
+                            a->d_wl_start, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&a->up_nwide, a->d_up_wide, 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -566,10 +567,11 @@ static int wgm_rank_layout(wgm_app *a, const int32_t *row_ptr) {
     const int none = INT32_MAX;
     e = cudaMemcpyAsync(a->d_cnt, &none, 4, cudaMemcpyHostToDevice, st);
   }
-  /* PageRank's ranks only pass through: its result buffer holds them */
+  /* PageRank's ranks only pass through: its contributions, free before a run,
+   * hold them (the result stays the last run's) */
   if (e == cudaSuccess)
     e = wgm_launch_rank_layout(V, wgm_rank_view(a), a->d_row, a->d_col, (const int *)a->d_wt,
-                               a->d_rk_of ? a->d_rk_of : (int *)a->d_out, a->d_rk_col, a->d_rk_wt,
+                               a->d_rk_of ? a->d_rk_of : (int *)a->d_contrib, a->d_rk_col, a->d_rk_wt,
                                a->d_cnt, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e == cudaSuccess ? WGM_OK : wgm_cuda_fail(a->rt, e);

@@ -163,7 +163,8 @@ const char *wgm_persistent_kernel_name(int app_kind);
  * allocates device buffers and uploads the graph. */
 int wgm_app_create(wgm_runtime *rt, int app_kind, const wgm_graph_desc *g, wgm_app **out);
 /* Re-upload a graph with the same node and edge counts (reset_persistent_task
- * re-writes the graph buffers, bfs.h:284-313). */
+ * re-writes the graph buffers, bfs.h:284-313).  The result stays the last
+ * run's until the next run. */
 int wgm_app_upload(wgm_app *app, const wgm_graph_desc *g);
 /* Source vertex (the reference hard-wires 0: bfs.cl:236-240, pannotia sssp.h:21). */
 int wgm_app_set_source(wgm_app *app, int32_t source);
