@@ -586,20 +586,29 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
   if (g->num_nodes != a->V || g->num_edges != a->E) return WGM_ERR_INVALID;
   cudaSetDevice(a->rt->device);
   cudaStream_t st = a->rt->stream;
+  /* The quirk again: where the last vertex has no edges of its own, the row
+   * before it can end one past the columns given.  It ends with them here. */
+  const int32_t *row_ptr = g->row_ptr;
+  std::vector<int32_t> cut;
+  if (row_ptr[a->V - 1] > g->num_edges) {
+    cut.assign(row_ptr, row_ptr + a->V + 1);
+    for (int v = a->V - 1; cut[v] > g->num_edges; v--) cut[v] = (int32_t)g->num_edges;
+    row_ptr = cut.data();
+  }
   cudaError_t e =
-      cudaMemcpyAsync(a->d_row, g->row_ptr, (size_t)(a->V + 1) * 4, cudaMemcpyHostToDevice, st);
+      cudaMemcpyAsync(a->d_row, row_ptr, (size_t)(a->V + 1) * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && a->E > 0)
     e = cudaMemcpyAsync(a->d_col, g->col, (size_t)a->E * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && wgm_needs_weights(a->kind) && a->E > 0)
     e = cudaMemcpyAsync(a->d_wt, g->weights, (size_t)a->E * 4, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
   if (a->kind == WGM_APP_LONESTAR_BFS) {
-    s = wgm_bfs_ell_layout(a, g->row_ptr);
-    if (s == WGM_OK) s = wgm_bfs_up_layout(a, g->row_ptr);
+    s = wgm_bfs_ell_layout(a, row_ptr);
+    if (s == WGM_OK) s = wgm_bfs_up_layout(a, row_ptr);
     if (s) return s;
   }
   if (a->kind == WGM_APP_PANNOTIA_COLOR) {
-    a->h_row.assign(g->row_ptr, g->row_ptr + a->V + 1);
+    a->h_row.assign(row_ptr, row_ptr + a->V + 1);
     s = wgm_color_layout(a); /* nothing to do before the first priorities */
     if (s) return s;
   }
@@ -608,7 +617,7 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
     if (s) return s;
   }
   if (a->kind == WGM_APP_PAGERANK || a->kind == WGM_APP_PANNOTIA_SSSP)
-    return wgm_rank_layout(a, g->row_ptr);
+    return wgm_rank_layout(a, row_ptr);
   return WGM_OK;
 }
 
