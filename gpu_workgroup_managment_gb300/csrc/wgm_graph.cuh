@@ -1498,7 +1498,10 @@ struct wgm_color_blocks_args {
   int NB, B;
 };
 
-extern __shared__ int wgm_cb_dyn[]; /* group 0: the colours of two blocks, 2 x B; a 0 */
+/* Group 0: the colours of two blocks, 2 x B, then a 0; read and written in
+ * words of 16 bytes (B is a multiple of 4). */
+extern __shared__ __align__(16) int wgm_cb_dyn[];
+static_assert(__alignof__(wgm_cb_dyn) >= 16, "wgm_cb_finish moves int4 words");
 
 /* Append the lanes' edges of four windows to the block's lists: target k,
  * source rank j; late when lo2 <= j < lo, inner when lo <= j < lo + k. */
@@ -2558,7 +2561,8 @@ struct wgm_pr_args {
   float dangling;    /* vertices without edges */
 };
 
-extern __shared__ float wgm_pr_cache[];
+extern __shared__ __align__(16) float wgm_pr_cache[]; /* filled in float4 words */
+static_assert(__alignof__(wgm_pr_cache) >= 16, "wgm_phase_pagerank moves float4 words");
 
 /* One iteration over the rows (wgm_rank_pull). */
 struct wgm_pr_op {
