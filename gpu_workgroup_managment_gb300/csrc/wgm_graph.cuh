@@ -1652,7 +1652,8 @@ __device__ __forceinline__ bool wgm_cb_look(const wgm_color_args &a,
 }
 
 /* Stage B of block b on this CTA (every thread): returns the thread's
- * largest colour.  A function of its own: its registers and those of the
+ * largest colour, or -1 to every thread when the block did not settle (a
+ * broken layout only).  A function of its own: its registers and those of the
  * prefetched step of stage A never live at once. */
 static __device__ __noinline__ int wgm_cb_finish(int V, int B, int b, int *colour,
                                                  const unsigned *lists, int *cnts,
@@ -1712,12 +1713,12 @@ static __device__ __noinline__ int wgm_cb_finish(int V, int B, int b, int *colou
       if (c[p] >= d[p]) atomicMax(&cur[late[p] >> 16], c[p] + 1);
   }
   __syncthreads();
-  /* Inner edges, all at once until a sweep changes nothing.  A look at four edges takes about 200 cycles and a CTA
-   * barrier with its vote 260, so a sweep looks three times (13 links: 4600
-   * cycles, against 6750 with one look).  A chain inside the block has fewer
-   * than nv links; an absent edge reads a word that stays 0.  Plain stores
-   * do: of two that meet, the smaller may stay, but its loser is still
-   * violated at the next look, and no value ever passes the true colour. */
+  /* Inner edges, all at once until a sweep changes nothing.  A look at four
+   * edges takes about 200 cycles and a CTA barrier with its vote 260, so a
+   * sweep looks three times (13 links: 4600 cycles, against 6750 with one
+   * look).  An absent edge reads a word that stays 0.  Plain stores do: of
+   * two that meet, the smaller may stay, but its loser is still violated at
+   * the next look, and no value ever passes the true colour. */
   volatile int *col = cur;
   int src[KI], dst[KI];
 #pragma unroll
@@ -1726,8 +1727,9 @@ static __device__ __noinline__ int wgm_cb_finish(int V, int B, int b, int *colou
     src[p] = have ? (int)(in[p] & 0xffffu) : (2 - (b & 1)) * B;
     dst[p] = have ? (int)(in[p] >> 16) : 0;
   }
-  for (int sweep = 0; sweep <= nv; sweep++) {
-    bool changed = false;
+  bool changed = true;
+  for (int sweep = wgm_proto_chain_sweeps(ni); sweep > 0 && changed; sweep--) {
+    changed = false;
 #pragma unroll 1
     for (int look = 0; look < 3; look++) {
       int c[KI], d[KI];
@@ -1751,10 +1753,10 @@ static __device__ __noinline__ int wgm_cb_finish(int V, int B, int b, int *colou
         changed = true;
       }
     }
-    if (!__syncthreads_or(changed)) break;
+    changed = __syncthreads_or(changed);
   }
-  int m = 0;
-  for (int k = 4 * threadIdx.x; k < nv; k += 4 * T) {
+  int m = changed ? -1 : 0;
+  for (int k = 4 * threadIdx.x; k < nv && !changed; k += 4 * T) {
     const int4 c = *reinterpret_cast<const int4 *>(&cur[k]);
     *reinterpret_cast<int4 *>(&colour[lo + k]) = c;
     m = max(m, c.x);

@@ -201,9 +201,12 @@ __global__ void __launch_bounds__(1024) wgm_k_color_blocks(wgm_launch L, wgm_col
     if (look) F = wgm_cb_prefetch(a, q, b, gw, NW);
     live = wgm_barrier(L, &c);
     if (!live) break;
-    if (b > 0 && c.id == 0)
-      mx = max(mx, wgm_cb_finish(a.V, q.B, b - 1, q.colour, q.list, q.cnt, q.blk_hub, q.hub_rank,
-                                 q.hub_max));
+    if (b > 0 && c.id == 0) {
+      const int m = wgm_cb_finish(a.V, q.B, b - 1, q.colour, q.list, q.cnt, q.blk_hub, q.hub_rank,
+                                  q.hub_max);
+      if (m < 0 && threadIdx.x == 0) wgm_fail(L, WGM_DEV_BAD_INPUT, WGM_SITE_QUEUE, b - 1);
+      mx = max(mx, m);
+    }
     if (look) ok &= wgm_cb_look(a, q, b, gw, NW, F, &sm);
   }
   /* the largest colour is the reference's round count */

@@ -81,4 +81,13 @@ struct wgm_proto_levels {
   }
 };
 
+/* Raising targets to one more than their sources, every edge of an acyclic
+ * list at once, sweep after sweep with plain stores, until one changes
+ * nothing (the inner edges of a colour block).  A target never falls below
+ * what it was at the sweep's start, so once its sources are final every sweep
+ * that leaves it short - a smaller store came last - is the last store of
+ * one more of its edges.  Along a chain those edges are different ones:
+ * `edges` sweeps settle everything, and one more finds nothing to do. */
+WGM_PROTO int wgm_proto_chain_sweeps(int edges) { return edges + 1; }
+
 #endif
