@@ -12,6 +12,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <new>
 #include <vector>
 
@@ -184,21 +185,46 @@ static cudaError_t wgm_dmalloc(T **p, size_t count) {
   return cudaMalloc((void **)p, std::max<size_t>(count, 1) * sizeof(T));
 }
 
+/* Every buffer of the list, or none of them. */
+struct wgm_want {
+  void **p;
+  size_t bytes;
+};
+static void wgm_dfree_all(std::initializer_list<void **> list) {
+  for (void **p : list) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+}
+static cudaError_t wgm_dmalloc_all(std::initializer_list<wgm_want> want) {
+  cudaError_t e = cudaSuccess;
+  for (const wgm_want &w : want)
+    if (e == cudaSuccess) e = cudaMalloc(w.p, std::max<size_t>(w.bytes, 4));
+  if (e != cudaSuccess) {
+    for (const wgm_want &w : want) wgm_dfree_all({w.p});
+    cudaGetLastError();
+  }
+  return e;
+}
+/* How a layout that an app can do without ends: short of memory (its kernels
+ * need some too), the app runs without it. */
+static int wgm_extra_layout(wgm_app *a, cudaError_t e) {
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return WGM_OK;
+  }
+  return e == cudaSuccess ? WGM_OK : wgm_cuda_fail(a->rt, e);
+}
+
+/* Hubs that a graph of E edges can have at most. */
+static size_t wgm_most_hubs(const wgm_app *a) { return (size_t)(a->E / (a->hub_threshold + 1)); }
+
 static int wgm_upload_hubs(wgm_app *a, const int32_t *row_ptr, const int *order) {
   std::vector<int> ids, prefix, wmap;
   wgm_build_hubs(a->V, row_ptr, order, a->hub_threshold, ids, prefix, wmap);
   cudaStream_t s = a->rt->stream;
   cudaError_t e = cudaSuccess;
-  if (a->hubs.ids) {
-    cudaFree(a->hubs.ids);
-    cudaFree(a->hubs.prefix);
-    cudaFree(a->hubs.wmap);
-    a->hubs = wgm_dev_hubs();
-  }
-  if (e == cudaSuccess) e = wgm_dmalloc(&a->hubs.ids, ids.size());
-  if (e == cudaSuccess) e = wgm_dmalloc(&a->hubs.prefix, prefix.size());
-  if (e == cudaSuccess) e = wgm_dmalloc(&a->hubs.wmap, wmap.size());
-  if (e == cudaSuccess && !ids.empty())
+  if (!ids.empty())
     e = cudaMemcpyAsync(a->hubs.ids, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(a->hubs.prefix, prefix.data(), prefix.size() * 4,
@@ -318,12 +344,58 @@ static double wgm_color_estimate(const std::vector<int> &row, const unsigned lon
  *     costs about 6 us, a round about 5 us, so grids of random priorities
  *     (a dozen rounds) stay with the rounds once they have 8 blocks. */
 #define WGM_CB_TARGET 1933.0
+
+/* Blocks to begin with, and the most vertices of one; false: none fit. */
+static bool wgm_color_plan(const wgm_app *a, int *NB, int *maxB) {
+  const int ctas = std::max(1, 512 / wgm_block_size(a->rt));
+  /* 1 KB reserved and 9 KB static per CTA */
+  const long long room =
+      ((long long)a->rt->prop.sharedMemPerMultiprocessor / ctas - 10 * 1024) / 4;
+  *maxB = (int)std::min<long long>(WGM_CB_MAX_B, room / 2) & ~3;
+  if (*maxB < 256) return false;
+  const int n = std::max((int)std::ceil(std::sqrt((double)a->E / WGM_CB_TARGET)),
+                         (a->V + *maxB - 1) / *maxB);
+  *NB = std::min(std::max(n, 1), a->V);
+  return true;
+}
+static size_t wgm_most_blocks(const wgm_app *a, int NB) {
+  return (size_t)std::min<long long>(2LL * NB, a->V) + 1;
+}
+
+/* The layout's buffers, at the sizes that V and E allow, so that new
+ * priorities and graphs only fill them. */
+static cudaError_t wgm_color_alloc_hubs(wgm_app *a) {
+  const size_t H = wgm_most_hubs(a);
+  return wgm_dmalloc_all({{(void **)&a->hubs.ids, H * 4},
+                          {(void **)&a->hubs.prefix, (H + 1) * 4},
+                          {(void **)&a->hubs.wmap, ((size_t)a->E + 31) / 32 * 16}});
+}
+static cudaError_t wgm_color_alloc_blocks(wgm_app *a, size_t max_blocks) {
+  const size_t V = (size_t)a->V, H = wgm_most_hubs(a);
+  return wgm_dmalloc_all({{(void **)&a->d_cb_ord, V * sizeof(int4)},
+                          {(void **)&a->d_cb_colour, (V + 4) * 4},
+                          {(void **)&a->d_cb_crank, (size_t)a->E * 4},
+                          {(void **)&a->d_cb_list, 2 * (size_t)WGM_CB_LISTS * 4},
+                          {(void **)&a->d_cb_cnt, 3 * (size_t)WGM_LINE * 4},
+                          {(void **)&a->d_cb_hub, max_blocks * 4},
+                          {(void **)&a->d_hub_rank, H * 4},
+                          {(void **)&a->d_hub_max, H * 4}});
+}
+
+static void wgm_color_free_blocks(wgm_app *a) {
+  wgm_dfree_all({(void **)&a->d_cb_ord, (void **)&a->d_cb_colour, (void **)&a->d_cb_crank,
+                 (void **)&a->d_cb_list, (void **)&a->d_cb_cnt, (void **)&a->d_cb_hub,
+                 (void **)&a->d_hub_rank, (void **)&a->d_hub_max});
+}
+
 static int wgm_color_layout(wgm_app *a) {
   const int V = a->V;
   a->cb_blocks = 0;
   if ((int)a->order.size() != V || (int)a->h_row.size() != V + 1) return WGM_OK;
   int s = wgm_upload_hubs(a, a->h_row.data(), a->order.data());
   if (s) return s;
+  int NB = 0, maxB = 0;
+  if (!wgm_color_plan(a, &NB, &maxB)) return WGM_OK;
   std::vector<int> hub_of((size_t)V, -1), hub_rank;
   for (int k = 0; k < V; k++)
     if (a->h_row[a->order[k] + 1] - a->h_row[a->order[k]] > a->hub_threshold) {
@@ -331,39 +403,19 @@ static int wgm_color_layout(wgm_app *a) {
       hub_rank.push_back(k);
     }
   const double E = (double)a->E;
-  const int ctas = std::max(1, 512 / wgm_block_size(a->rt));
-  /* 1 KB reserved and 9 KB static per CTA */
-  const long long room =
-      ((long long)a->rt->prop.sharedMemPerMultiprocessor / ctas - 10 * 1024) / 4;
-  const int maxB = (int)std::min<long long>(WGM_CB_MAX_B, room / 2) & ~3;
-  if (maxB < 256) return WGM_OK;
-  int NB = std::max((int)std::ceil(std::sqrt(E / WGM_CB_TARGET)), (V + maxB - 1) / maxB);
-  NB = std::min(std::max(NB, 1), V);
-  const size_t max_blocks = (size_t)std::min<long long>(2LL * NB, V) + 1;
+  const size_t max_blocks = wgm_most_blocks(a, NB);
   cudaStream_t st = a->rt->stream;
+  int *tmp = nullptr, *cnt = nullptr; /* order, hub_of, rank; the counts */
+  unsigned long long *hist = nullptr, edges[WGM_DEGREE_BUCKETS] = {};
   cudaError_t e = cudaSuccess;
-  for (int **p : {&a->d_cb_hub, &a->d_hub_rank, &a->d_hub_max}) {
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-  }
-  e = wgm_dmalloc(&a->d_cb_hub, max_blocks);
-  if (e == cudaSuccess) e = wgm_dmalloc(&a->d_hub_rank, hub_rank.size());
-  if (e == cudaSuccess) e = wgm_dmalloc(&a->d_hub_max, hub_rank.size());
-  if (e == cudaSuccess && !a->d_cb_ord) {
-    e = wgm_dmalloc(&a->d_cb_ord, (size_t)V);
-    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cb_colour, (size_t)V + 4);
-    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cb_crank, (size_t)a->E);
-    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cb_list, 2 * (size_t)WGM_CB_LISTS);
-    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cb_cnt, 3 * (size_t)WGM_LINE);
-  }
+  if (!a->d_cb_ord) e = wgm_color_alloc_blocks(a, max_blocks);
+  if (e == cudaSuccess)
+    e = wgm_dmalloc_all({{(void **)&tmp, 3 * (size_t)V * 4},
+                         {(void **)&cnt, 2 * max_blocks * 4},
+                         {(void **)&hist, sizeof(edges)}});
   if (e == cudaSuccess && !hub_rank.empty())
     e = cudaMemcpyAsync(a->d_hub_rank, hub_rank.data(), hub_rank.size() * 4,
                         cudaMemcpyHostToDevice, st);
-  int *tmp = nullptr, *cnt = nullptr; /* order, hub_of, rank; the counts */
-  unsigned long long *hist = nullptr, edges[WGM_DEGREE_BUCKETS] = {};
-  if (e == cudaSuccess) e = wgm_dmalloc(&tmp, 3 * (size_t)V);
-  if (e == cudaSuccess) e = wgm_dmalloc(&cnt, 2 * max_blocks);
-  if (e == cudaSuccess) e = wgm_dmalloc(&hist, WGM_DEGREE_BUCKETS);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(tmp, a->order.data(), (size_t)V * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess)
@@ -415,14 +467,12 @@ static int wgm_color_layout(wgm_app *a) {
   }
   const cudaError_t e2 = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = e2;
-  if (tmp) cudaFree(tmp);
-  if (cnt) cudaFree(cnt);
-  if (hist) cudaFree(hist);
+  wgm_dfree_all({(void **)&tmp, (void **)&cnt, (void **)&hist});
   if (e != cudaSuccess) {
-    a->cb_blocks = 0;
-    return wgm_cuda_fail(a->rt, e);
+    a->cb_blocks = 0; /* the rounds need none of it */
+    wgm_color_free_blocks(a);
   }
-  return WGM_OK;
+  return wgm_extra_layout(a, e);
 }
 
 /* Lonestar BFS on one CTA (wgm_bfs_cta): chosen by default for graphs of
@@ -448,15 +498,13 @@ static int wgm_bfs_ell_layout(wgm_app *a, const int32_t *row_ptr) {
   for (int v = 0; v < a->V; v++) most = std::max(most, row_ptr[v + 1] - row_ptr[v]);
   if (most > 8) return WGM_OK;
   const int W = most > 4 ? 8 : 4;
-  if (!a->d_ell) {
-    cudaError_t e = wgm_dmalloc(&a->d_ell, 8 * (size_t)a->V);
-    if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
-  }
-  cudaError_t e = wgm_launch_bfs_ell(W, a->V, a->d_row, a->d_col, a->d_ell, a->rt->stream);
+  cudaError_t e = cudaSuccess;
+  if (!a->d_ell) e = wgm_dmalloc_all({{(void **)&a->d_ell, 8 * (size_t)a->V * 4}});
+  if (e == cudaSuccess) e = wgm_launch_bfs_ell(W, a->V, a->d_row, a->d_col, a->d_ell, a->rt->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(a->rt->stream); /* runs may use another stream */
-  if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
-  a->ell_w = W;
-  return WGM_OK;
+  if (e == cudaSuccess) a->ell_w = W;
+  else wgm_dfree_all({(void **)&a->d_ell}); /* the rows are there */
+  return wgm_extra_layout(a, e);
 }
 
 /* In-edges of a large graph, for BFS from both sides (wgm_phase_bfs): where
@@ -469,13 +517,12 @@ static int wgm_bfs_up_layout(wgm_app *a, const int32_t *row_ptr) {
   const int64_t used = std::max(row_ptr[V - 1], row_ptr[V]);
   cudaStream_t st = a->rt->stream;
   cudaError_t e = cudaSuccess;
-  if (!a->d_trow) {
-    e = wgm_dmalloc(&a->d_trow, (size_t)V + 1);
-    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_tcol, (size_t)a->E);
-    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_up_bits, 3 * (((size_t)V + 31) / 32));
-    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_up_cnt, 3 * (size_t)WGM_LINE);
-    if (e == cudaSuccess) e = wgm_dmalloc(&a->d_up_wide, (size_t)(a->E / WGM_BFS_UP_SCAN) + 2);
-  }
+  if (!a->d_trow)
+    e = wgm_dmalloc_all({{(void **)&a->d_trow, ((size_t)V + 1) * 4},
+                         {(void **)&a->d_tcol, (size_t)a->E * 4},
+                         {(void **)&a->d_up_bits, 3 * (((size_t)V + 31) / 32) * 4},
+                         {(void **)&a->d_up_cnt, 3 * (size_t)WGM_LINE * 4},
+                         {(void **)&a->d_up_wide, ((size_t)(a->E / WGM_BFS_UP_SCAN) + 2) * 4}});
   /* the worklist is free before a run: the in-degrees pass through it (the
    * result stays the last run's) */
   if (e == cudaSuccess)
@@ -484,9 +531,11 @@ static int wgm_bfs_up_layout(wgm_app *a, const int32_t *row_ptr) {
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&a->up_nwide, a->d_up_wide, 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
-  a->bfs_up = true;
-  return WGM_OK;
+  a->bfs_up = e == cudaSuccess;
+  if (!a->bfs_up) /* the worklist needs no in-edges */
+    wgm_dfree_all({(void **)&a->d_trow, (void **)&a->d_tcol, (void **)&a->d_up_bits,
+                   (void **)&a->d_up_cnt, (void **)&a->d_up_wide});
+  return wgm_extra_layout(a, e);
 }
 
 /* Edges a group at least (RMAT-14: 0.152 ms with 2048 to 8192, 0.28 with
@@ -700,6 +749,7 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
         if (e == cudaSuccess) e = wgm_dmalloc(&a->d_stamp, V); /* pending */
         if (e == cudaSuccess) e = wgm_dmalloc(&a->d_cnt, 3 * WGM_LINE);
         if (e == cudaSuccess) e = wgm_dmalloc(&a->d_tcv, E); /* in-edges with values */
+        if (e == cudaSuccess) e = wgm_color_alloc_hubs(a);
       }
       if (kind == WGM_APP_PANNOTIA_MIS) {
         if (e == cudaSuccess) e = wgm_dmalloc(&a->d_mis_word, V);
