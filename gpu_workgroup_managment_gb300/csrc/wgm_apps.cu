@@ -150,11 +150,6 @@ static void wgm_rounds_take(wgm_app *a) {
 }
 
 static void wgm_app_free_buffers(wgm_app *a) {
-  if (a->rounds_slot >= 0) {
-    std::lock_guard<std::mutex> hold(a->rt->rounds_mutex);
-    a->rt->rounds_used[a->rounds_slot] = false;
-    a->rounds_slot = -1;
-  }
   void *ptrs[] = {a->d_row,     a->d_col,       a->d_wt,      a->d_node_value, a->d_out,
                   a->d_wl_start, a->d_wl_cnt,   a->d_wl_u,
                   a->d_cnt,       a->d_stamp,   a->d_stop,
@@ -169,6 +164,12 @@ static void wgm_app_free_buffers(wgm_app *a) {
   for (void *p : ptrs)
     if (p) cudaFree(p);
   a->hubs = wgm_dev_hubs();
+  /* last: cudaFree has waited for a run on a caller's stream, which writes it */
+  if (a->rounds_slot >= 0) {
+    std::lock_guard<std::mutex> hold(a->rt->rounds_mutex);
+    a->rt->rounds_used[a->rounds_slot] = false;
+    a->rounds_slot = -1;
+  }
 }
 
 /* Independent set: the edges of one vertex that a single warp looks at, and
