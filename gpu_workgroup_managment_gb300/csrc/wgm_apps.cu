@@ -1257,13 +1257,14 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
     const long long want = ((long long)a->V / b + sms - 1) / sms * sms;
     *grid = (int)std::min<long long>(hw, std::max(sms, want));
   }
-  /* PageRank by default (block: wgm_app_block): one group per SM, whose
-   * shared memory holds the contributions read most often; fewer for small
-   * graphs, WGM_PR_EDGES edges each, since an iteration ends in a barrier. */
+  /* PageRank by default (block: wgm_app_block): 1024 threads per SM, one group
+   * whose shared memory holds the contributions read most often; fewer for
+   * small graphs, WGM_PR_EDGES edges per 1024 threads, since an iteration ends
+   * in a barrier. */
   if (num_wgs <= 0 && a->kind == WGM_APP_PAGERANK) {
-    const long long sms = a->rt->prop.multiProcessorCount;
-    *grid = (int)std::min<long long>(std::min<long long>(hw, sms),
-                                     std::max<long long>(1, a->E / WGM_PR_EDGES));
+    const long long sms = a->rt->prop.multiProcessorCount, b = std::max(block, 1);
+    *grid = (int)std::min({(long long)hw, sms * std::max(1LL, 1024 / b),
+                           std::max(1LL, (long long)a->E * 1024 / (WGM_PR_EDGES * b))});
   }
   /* Pannotia SSSP by default: 1024 threads per SM (four 256-thread CTAs of
    * the six that fit), more only for graphs of more than one 256-thread CTA
@@ -1278,11 +1279,12 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
   return WGM_OK;
 }
 
-/* Threads per group of a standalone run: the runtime's, but PageRank on its
- * default group count runs one group of 1024 per SM (its shared memory serves
- * them all). */
+/* Threads per group of a standalone run: the runtime's, but where that is left
+ * at its default, PageRank on its default group count runs one group of 1024
+ * per SM (its shared memory serves them all). */
 static int wgm_app_block(const wgm_app *a, int num_wgs) {
-  return a->kind == WGM_APP_PAGERANK && num_wgs <= 0 ? 1024 : wgm_block_size(a->rt);
+  const int b = wgm_block_size(a->rt);
+  return a->kind == WGM_APP_PAGERANK && num_wgs <= 0 && b == 256 ? 1024 : b;
 }
 
 extern "C" int wgm_launch_persistent(wgm_runtime *rt, wgm_app *a, int num_wgs, void *stream) {

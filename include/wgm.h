@@ -75,7 +75,8 @@ typedef struct wgm_host_graph wgm_host_graph;
  * to the persistent path, plus the GB300 knobs. */
 typedef struct wgm_config {
   int device;
-  int threads_per_wg;          /* skel.cpp:39 */
+  int threads_per_wg;          /* skel.cpp:39; at 256, the default, a standalone PageRank
+                                  with num_wgs <= 0 runs groups of 1024 instead */
   int num_wgs;                 /* skel.cpp:40; <=0: every co-resident CTA */
   int use_query_barrier;       /* skel.cpp:34 */
   int non_persistent_wgs;      /* skel.cpp:30 */
