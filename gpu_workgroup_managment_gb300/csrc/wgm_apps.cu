@@ -909,6 +909,12 @@ extern "C" int wgm_app_set_color_mode(wgm_app *a, int32_t mode) {
   return WGM_OK;
 }
 
+extern "C" int wgm_app_color_blocks(wgm_app *a, int32_t *blocks) {
+  if (!a || !blocks || a->kind != WGM_APP_PANNOTIA_COLOR) return WGM_ERR_INVALID;
+  *blocks = a->cb_blocks;
+  return WGM_OK;
+}
+
 extern "C" int wgm_app_set_pagerank(wgm_app *a, float damping, int iterations) {
   if (!a || a->kind != WGM_APP_PAGERANK || iterations < 0 || !(damping >= 0.f && damping <= 1.f))
     return WGM_ERR_INVALID;

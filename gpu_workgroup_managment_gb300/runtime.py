@@ -227,6 +227,12 @@ class PersistentApp:
         d, _keep = _desc(g)
         check(lib.wgm_app_upload(self._h, C.byref(d)), "wgm_app_upload")
 
+    def color_blocks(self) -> int:
+        """Blocks of priorities that a standalone colour run takes; 0: rounds."""
+        n = C.c_int32()
+        check(lib.wgm_app_color_blocks(self._h, C.byref(n)), "color_blocks")
+        return n.value
+
     def run(self, num_wgs: int = 0) -> RunStats:
         """One iteration of run_persistent (skel.cpp:316-355)."""
         st = WgmRunStats()

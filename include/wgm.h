@@ -173,15 +173,22 @@ int wgm_app_set_source(wgm_app *app, int32_t source);
 int wgm_app_set_node_values(wgm_app *app, const float *node_value);
 int wgm_app_set_pagerank(wgm_app *app, float damping, int iterations);
 /* How a standalone Pannotia colour run proceeds (no reference counterpart):
- * 0 (the default) a grid barrier per round (color.cl's structure; the
- * megakernel and the served form always run rounds, where they resize);
- * 1 without rounds - a vertex is coloured as soon as its last larger
- * out-neighbour is, the warp that colours it releasing its smaller
- * neighbours next (slower on RMAT graphs: 16 ms against 8.3 ms at scale
- * 20).  Same colours, same round count (the largest colour). */
+ * 0 (the default) in blocks of priorities, a grid barrier per block, where
+ * the graph and its priorities allow it (wgm_app_color_blocks), else a grid
+ * barrier per round (color.cl's structure; the megakernel and the served
+ * form always run rounds, where they resize); 1 without rounds - a vertex is
+ * coloured as soon as its last larger out-neighbour is, the warp that
+ * colours it releasing its smaller neighbours next (slower on RMAT graphs:
+ * 16 ms at scale 20, against 8.3 ms in rounds and 1.7 ms in blocks).  Same
+ * colours, same round count (the largest colour). */
 int wgm_app_set_color_mode(wgm_app *app, int32_t mode);
+/* Blocks of priorities that a standalone run of mode 0 takes with the graph
+ * and the priorities that the app has now; 0: it runs in rounds. */
+int wgm_app_color_blocks(wgm_app *app, int32_t *blocks);
 /* How a standalone Lonestar BFS run proceeds (no reference counterpart):
- * 0 the reference's shape - discovered groups, a grid barrier per level;
+ * 0 the reference's shape - discovered groups, a grid barrier per level
+ * (wide levels of a graph of two million edges or more run over the
+ * unreached vertices' in-edges instead of the reached ones' edges);
  * 1 one CTA, the visited set and the frontier in shared memory and
  * __syncthreads as the level barrier (graphs of at most 2^20 vertices);
  * -1 (the default) 1 for graphs of at most 65,536 vertices and average
