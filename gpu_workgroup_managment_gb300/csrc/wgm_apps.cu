@@ -769,7 +769,7 @@ extern "C" int wgm_app_create(wgm_runtime *rt, int kind, const wgm_graph_desc *g
     case WGM_APP_PAGERANK:
       a->out_bytes = V * 4;
       if (e == cudaSuccess) e = cudaMalloc(&a->d_out, a->out_bytes);
-      /* contrib: two rows of V rounded up to whole 16-byte words, and one more */
+      /* contrib: two rows of V rounded up to whole 16-byte words */
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_contrib, 2 * wgm_pr_stride(a->V));
       if (e == cudaSuccess) e = wgm_dmalloc(&a->d_dang, 3 * WGM_LINE);
       if (e == cudaSuccess) e = wgm_rank_alloc(a, false);
@@ -1235,6 +1235,8 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
   }
   if (s) return s;
   if (hw < 1) return WGM_ERR_INVALID;
+  /* (all that fit, by default, is also what Pannotia SSSP takes: 1024 threads
+   * per SM at its 64 registers) */
   *grid = (num_wgs > 0) ? std::min(num_wgs, hw) : hw;
   /* Pannotia colour by default: 512 threads per SM.  Its rounds (~1600 on
    * RMAT-20) carry little work each and end in a grid barrier, so fewer
@@ -1271,16 +1273,6 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
     const long long sms = a->rt->prop.multiProcessorCount, b = std::max(block, 1);
     *grid = (int)std::min({(long long)hw, sms * std::max(1LL, 1024 / b),
                            std::max(1LL, (long long)a->E * 1024 / (WGM_PR_EDGES * b))});
-  }
-  /* Pannotia SSSP by default: 1024 threads per SM (four 256-thread CTAs of
-   * the six that fit), more only for graphs of more than one 256-thread CTA
-   * per 32768 edges: on grids and RMAT graphs up to 7.6M edges four CTAs
-   * per SM ran 9-15 % faster than six, on RMAT-20 (33M edges) six won. */
-  if (num_wgs <= 0 && a->kind == WGM_APP_PANNOTIA_SSSP) {
-    const long long sms = a->rt->prop.multiProcessorCount, b = std::max(block, 1);
-    const long long base = sms * std::max(1LL, 1024 / b);
-    const long long byE = ((long long)a->E / 128 / b + sms - 1) / sms * sms;
-    *grid = (int)std::min<long long>(hw, std::max(base, byE));
   }
   return WGM_OK;
 }

@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(1024) wgm_k_color(wgm_launch L, wgm_color_args
   WGM_PERSISTENT_EPILOGUE
 }
 
-/* 48 registers (six spilled words): five 256-thread CTAs per SM.  RMAT-20: 0.228 ms,
+/* 48 registers (eight spilled words): five 256-thread CTAs per SM.  RMAT-20: 0.228 ms,
  * against 0.235 with 64, 0.246 with 40 and 0.292 with 32 (more CTAs only
  * make the barrier dearer). */
 __global__ void __maxnreg__(48) wgm_k_mis(wgm_launch L, wgm_mis_args a) {
