@@ -652,6 +652,11 @@ extern "C" int wgm_app_upload(wgm_app *a, const wgm_graph_desc *g) {
   if (e == cudaSuccess && wgm_needs_weights(a->kind) && a->E > 0)
     e = cudaMemcpyAsync(a->d_wt, g->weights, (size_t)a->E * 4, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return wgm_cuda_fail(a->rt, e);
+  if (a->kind == WGM_APP_LONESTAR_SSSP) {
+    a->most_edges = 0;
+    for (int v = 0; v < a->V; v++)
+      a->most_edges = std::max(a->most_edges, row_ptr[v + 1] - row_ptr[v]);
+  }
   if (a->kind == WGM_APP_LONESTAR_BFS) {
     s = wgm_bfs_ell_layout(a, row_ptr);
     if (s == WGM_OK) s = wgm_bfs_up_layout(a, row_ptr);
@@ -1017,7 +1022,7 @@ int wgm_app_fill_mega(wgm_app *a, wgm_mega_args *A) {
       x.source = a->source;
       x.levels_out = wgm_rounds_out(a);
       x.packed = a->kind == WGM_APP_LONESTAR_SSSP ? 1 : 0;
-      x.low_degree = x.packed && a->E <= 8LL * a->V ? 1 : 0;
+      x.low_degree = x.packed && a->E <= 8LL * a->V && a->most_edges <= WGM_LS_NARROW_MOST ? 1 : 0;
       return WGM_OK;
     }
     case WGM_APP_PANNOTIA_COLOR: {

@@ -202,7 +202,7 @@ struct wgm_lonestar_args {
   int source;
   int *levels_out; /* number of levels run (written by group 0) */
   int packed = 0;  /* SSSP relaxes packed words (wgm_ls_chunk PACK) */
-  int low_degree = 0; /* SSSP: average degree at most 8 (wgm_ls_narrow) */
+  int low_degree = 0; /* SSSP: average degree at most 8, no hubs (wgm_ls_narrow) */
   int *grab = nullptr; /* [3 lines] chunks of a wide level handed out, by level mod 3 */
 };
 
@@ -599,8 +599,16 @@ __device__ __forceinline__ unsigned wgm_ls_relax32(const wgm_lonestar_args &a, i
  * followed by a relaxation that reads it.  509x517 grid: 759 levels, 3.95 ms
  * without hops; 581 and 3.45 with one, 514 and 3.39 with two, 481 and 3.16
  * with three, 455 and 3.33 with five (more hops relax distances that are not
- * final yet). */
+ * final yet).
+ * For graphs without hubs: there is no look at a word before its atomic, and
+ * a lane writes its vertex's pieces alone.  A hub's word takes an atomic of
+ * every leaf, and its pieces keep one lane long; star of 300,000 from a leaf
+ * 0.172 ms this way and 0.057 by wgm_ls_piece, of 30,000 0.049 and 0.022, and
+ * RMAT graphs of low degree are faster without it too (2^12 vertices of
+ * factor 2: 0.067 and 0.052).  Doing both here for all graphs (a look where
+ * every vertex has one edge, a warp's writes) cost grids 8 and 13 %. */
 #define WGM_LS_HOPS 3
+#define WGM_LS_NARROW_MOST 128 /* edges of any vertex */
 __device__ __forceinline__ bool wgm_ls_narrow(const wgm_lonestar_args &a, int L, int start, int deg,
                                               int src, const wgm_ls_out &o) {
   const int lane = wgm_lane(), P = a.piece;

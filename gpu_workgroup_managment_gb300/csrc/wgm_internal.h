@@ -93,6 +93,7 @@ struct wgm_app {
   int4 *d_tcv4 = nullptr;
   int *d_cmax = nullptr, *d_cq = nullptr, *d_cqctl = nullptr;
   int cq_cap = 0;
+  int most_edges = 0; /* Lonestar SSSP: of any vertex (wgm_ls_narrow) */
   int source = 0;
   float damping = 0.85f;
   /* PageRank, Pannotia SSSP: rows, columns and weights by falling degree
