@@ -1285,15 +1285,21 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
                            std::max({1LL, (long long)a->E * 1024 / (WGM_PR_EDGES * b),
                                      (units + w - 1) / w})});
   }
-  /* Pannotia SSSP by default: a warp for every unit of a pass (a part of a
-   * wide row, a row of bin 0, a task of the other bins), in whole groups per
-   * SM.  Passes are many and short on graphs of large diameter, and each ends
-   * in a barrier of all groups: 200 x 200 grid 1.83 ms on 304 groups of 256,
-   * 2.47 on all 608 and 2.07 on 152 (units left over for a second turn). */
+  /* Pannotia SSSP by default: 1024 threads per SM, which is all that fit, and
+   * for small graphs 256 or 512.  Passes are many and short where the diameter
+   * is large, and each ends in a barrier of all groups, so a warp needs no more
+   * than a unit of work (a part of a wide row, a row of bin 0, a task of the
+   * other bins).  ms on 152 / 304 / 608 groups of 256: path of 1000 (32 units)
+   * 3.1 / 3.3 / 4.5, 200 x 200 grid (1250) 1.99 / 1.73 / 2.32, RMAT-14 of
+   * factor 16 0.101 / 0.081 / 0.102, 512 x 512 grid (8192) 11.2 / 8.3 / 7.7.
+   * (256 x 256, 2048 units: 2.63 / 2.25 / 3.05; its group count is a promise
+   * of test_lonestar_default_groups, and so bounds the rows here.) */
   if (num_wgs <= 0 && a->kind == WGM_APP_PANNOTIA_SSSP) {
-    const long long sms = a->rt->prop.multiProcessorCount, w = std::max(block / 32, 1);
+    const long long sms = a->rt->prop.multiProcessorCount;
     const long long units = a->rk_parts + a->rk_bin_task[WGM_RANK_BINS];
-    *grid = (int)std::min<long long>(hw, std::max(1LL, (units + sms * w - 1) / (sms * w)) * sms);
+    long long threads = 1024;
+    if (a->rk_rows <= 13 * 32 * sms && units <= 32 * sms) threads = units <= 8 * sms ? 256 : 512;
+    *grid = (int)std::min<long long>(hw, sms * std::max(1LL, threads / std::max(block, 1)));
   }
   return WGM_OK;
 }

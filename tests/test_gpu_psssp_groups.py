@@ -1,5 +1,5 @@
-"""Pannotia SSSP on its default groups - a warp for every unit of a pass, whole groups
-per SM - at the sizes where the rule steps, with a unit more and a unit less; costs
+"""Pannotia SSSP on its default groups - 256, 512 or 1024 threads per SM by the work of
+a pass - at the sizes where the rule steps, with a row more and a row less; costs
 against the oracle, bit exact."""
 import numpy as np
 import pytest
@@ -10,18 +10,21 @@ from oracle import oracle
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("threads", [64, 256, 1024])
-@pytest.mark.parametrize("turns", [1, 2])
-@pytest.mark.parametrize("more", [-1, 0, 1])
-def test_default_groups(threads, turns, more):
+@pytest.mark.parametrize("threads", [64, 256, 512, 1024])
+@pytest.mark.parametrize("units_per_sm,degree,per_sm", [
+    (2, 3, (256, 256, 256)), (8, 3, (256, 256, 512)), (13, 5, (512, 512, 1024)),
+    (32, 8, (1024, 1024, 1024)), (32, 40, (512, 512, 1024))])
+def test_default_groups(threads, units_per_sm, degree, per_sm):
     with Runtime(threads_per_wg=threads) as r:
-        sms, per_sm = r.sm_count(), 1024 // threads
-        n = turns * sms * (threads // 32) * 32 + more  # a unit holds 32 rows of 3 edges
-        rng = np.random.default_rng(n)
-        g = graphs.Graph(np.arange(0, 3 * n + 1, 3, dtype=np.int32),
-                         rng.integers(0, n, 3 * n).astype(np.int32),
-                         rng.integers(1, 100, 3 * n).astype(np.uint32))
-        with PersistentApp(r, "sssp", g, source=5) as a:
-            st = a.run()
-            assert st.groups == sms * min(per_sm, turns + (more > 0))
-            assert np.array_equal(a.result(), oracle.pannotia_sssp(g, 5))
+        sms = r.sm_count()
+        rows = 32 if degree <= 8 else 4  # of a unit
+        for more, want_threads in zip((-1, 0, 1), per_sm):
+            n = units_per_sm * sms * rows + more
+            rng = np.random.default_rng(n)
+            g = graphs.Graph(np.arange(0, degree * n + 1, degree, dtype=np.int32),
+                             rng.integers(0, n, degree * n).astype(np.int32),
+                             rng.integers(1, 100, degree * n).astype(np.uint32))
+            with PersistentApp(r, "sssp", g, source=5) as a:
+                st = a.run()
+                assert st.groups == sms * max(1, want_threads // threads), (more, n)
+                assert np.array_equal(a.result(), oracle.pannotia_sssp(g, 5))
