@@ -640,7 +640,11 @@ __device__ __forceinline__ bool wgm_ls_narrow(const wgm_lonestar_args &a, int L,
  * search, no scans, and the pushes are counted by ballots unless a vertex
  * has several pieces.  A piece of more than 8 edges keeps the pre-check: on
  * a dense graph most of its atomics would fail, thousands of them on a hub's
- * word.  (SSSP of low average degree goes by wgm_ls_narrow.) */
+ * word.  (SSSP of low average degree goes by wgm_ls_narrow.)  Pieces of more
+ * than two windows (they are as long as the average row) go by wgm_ls_chunk,
+ * which has four in flight: clique of 1000, BFS 0.069 ms here and 0.049
+ * there, SSSP 0.222 and 0.180; average degree 40, SSSP 0.226 and 0.238. */
+#define WGM_LS_PIECE_MOST 64
 template <bool SSSP>
 __device__ __forceinline__ bool wgm_ls_piece(const wgm_lonestar_args &a, int L, int start, int deg,
                                              int src, const wgm_ls_out &o) {
@@ -727,7 +731,7 @@ __device__ __forceinline__ bool wgm_ls_level(const wgm_launch &Lc, wgm_cta *c,
   o.cap = a.cap;
   bool ok = true;
   const bool narrow = SSSP && a.packed && a.low_degree && n <= 8 * NW;
-  if (n <= NW && (!SSSP || a.packed) && !narrow)
+  if (n <= NW && (!SSSP || a.packed) && !narrow && a.piece <= WGM_LS_PIECE_MOST)
     return gw >= n || wgm_ls_piece<SSSP>(a, L, first.x, first.y, first.z, o);
   /* pieces per warp: 32, or fewer when the list is short, so a small
    * frontier spreads over every warp instead of queueing on a few */
