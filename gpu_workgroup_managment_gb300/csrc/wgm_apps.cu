@@ -856,10 +856,10 @@ extern "C" int wgm_app_set_bc_mode(wgm_app *a, int32_t mode) {
 
 /* Threads a source: small graphs fill the SM with more CTAs, each with a
  * cheaper barrier; once shared memory (20 bytes a vertex) holds only two CTAs,
- * 1024 threads fill it.  256 / 512 / 1024 threads, ms: RMAT 500 0.062 / 0.066
- * / 0.086, 1000 0.113 / 0.130 / 0.174, 2000 0.549 / 0.493 / 0.631, 3000 0.716
- * / 0.548 / 0.647, 4096 3.71 / 2.35 / 2.12; grid 24 x 24 0.141 / 0.145 /
- * 0.272. */
+ * 1024 threads fill it.  256 / 512 / 1024 threads, ms: RMAT of factor 16 with
+ * 500 vertices 0.066 / 0.071 / 0.089, 1000 0.152 / 0.160 / 0.215, 2000 0.545 /
+ * 0.496 / 0.648, 3000 1.155 / 0.840 / 1.025, 4096 3.65 / 2.32 / 2.10; grid 24 x
+ * 24 0.128 / 0.132 / 0.252. */
 static int wgm_bc_cta_threads(int V) { return V <= 1024 ? 256 : V <= 3584 ? 512 : 1024; }
 /* Sources spread over CTAs (bc_mode 1): a plain launch of resident CTAs, no
  * discovery and no host handshake, so the launch generation is untouched. */

@@ -2900,7 +2900,7 @@ static __device__ int wgm_phase_bc(const wgm_launch &Lc, wgm_cta *c, const wgm_b
  * from a table of the window's row starts (five dependent shuffles: 2.25,
  * the table 2.12).  EVEN, for graphs of degree up to 4 on average, whose rows
  * differ little: 32 vertices a warp in turn and one window, fewer
- * instructions a level (grid 24 x 24 0.149 -> 0.141 ms, 15 x 8 59 -> 53 us).
+ * instructions a level (grid 24 x 24 0.137 -> 0.128 ms, 15 x 8 53 -> 45 us).
  * What bounds small graphs is the chain of a level, about 2000 cycles. */
 #define WGM_BC_SHARE 4
 #define WGM_BC_K 2 /* 32-edge windows in flight */
