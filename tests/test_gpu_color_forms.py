@@ -20,7 +20,7 @@ def _band(n, half):
 
 
 GRAPHS = {"clique": lambda: _band(150, 150), "rmat10": lambda: graphs.rmat(10, 8, seed=2),
-          "rmat15": lambda: graphs.rmat(15, 16, seed=4), "band": lambda: _band(30000, 16),
+          "rmat15": lambda: graphs.rmat(15, 16, seed=4), "band": lambda: _band(16000, 16),
           "grid": lambda: graphs.grid(300, 300)}
 # (seeded priorities, priorities by vertex number)
 BLOCKS = {"clique": (True, True), "rmat10": (True, True), "rmat15": (True, True),
