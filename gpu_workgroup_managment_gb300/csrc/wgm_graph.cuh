@@ -1739,9 +1739,8 @@ static __device__ __noinline__ int wgm_cb_finish(int V, int B, int b, int *colou
     src[p] = have ? (int)(in[p] & 0xffffu) : (2 - (b & 1)) * B;
     dst[p] = have ? (int)(in[p] >> 16) : 0;
   }
-  bool changed = true;
-  for (int sweep = wgm_proto_chain_sweeps(ni); sweep > 0 && changed; sweep--) {
-    changed = false;
+  for (int sweeps = wgm_proto_chain_sweeps(ni);;) {
+    bool changed = false;
 #pragma unroll 1
     for (int look = 0; look < 3; look++) {
       int c[KI], d[KI];
@@ -1765,10 +1764,11 @@ static __device__ __noinline__ int wgm_cb_finish(int V, int B, int b, int *colou
         changed = true;
       }
     }
-    changed = __syncthreads_or(changed);
+    if (!__syncthreads_or(changed)) break;
+    if (--sweeps == 0) return -1;
   }
-  int m = changed ? -1 : 0;
-  for (int k = 4 * threadIdx.x; k < nv && !changed; k += 4 * T) {
+  int m = 0;
+  for (int k = 4 * threadIdx.x; k < nv; k += 4 * T) {
     const int4 c = *reinterpret_cast<const int4 *>(&cur[k]);
     *reinterpret_cast<int4 *>(&colour[lo + k]) = c;
     m = max(m, c.x);
