@@ -548,6 +548,7 @@ static int wgm_bfs_up_layout(wgm_app *a, const int32_t *row_ptr) {
 static wgm_rank_rows wgm_rank_view(const wgm_app *a) {
   wgm_rank_rows r;
   r.rows = a->rk_rows;
+  r.short_rows = a->E <= 32LL * a->rk_rows;
   r.prow = a->d_rk_row;
   r.pcol = a->d_rk_col;
   r.pwt = a->d_rk_wt;
@@ -1290,9 +1291,9 @@ static int wgm_pick_grid(wgm_app *a, int num_wgs, int block, int *grid) {
    * is large, and each ends in a barrier of all groups, so a warp needs no more
    * than a unit of work (a part of a wide row, a row of bin 0, a task of the
    * other bins).  ms on 152 / 304 / 608 groups of 256: path of 1000 (32 units)
-   * 3.1 / 3.3 / 4.5, 200 x 200 grid (1250) 1.99 / 1.73 / 2.32, RMAT-14 of
-   * factor 16 0.101 / 0.081 / 0.102, 512 x 512 grid (8192) 11.2 / 8.3 / 7.7.
-   * (256 x 256, 2048 units: 2.63 / 2.25 / 3.05; its group count is a promise
+   * 3.1 / 3.2 / 4.3, 200 x 200 grid (1250) 1.90 / 1.66 / 2.13, RMAT-14 of
+   * factor 16 0.098 / 0.081 / 0.106, 512 x 512 grid (8192) 9.9 / 7.4 / 6.9.
+   * (256 x 256, 2048 units: 2.44 / 2.11 / 2.80; its group count is a promise
    * of test_lonestar_default_groups, and so bounds the rows here.) */
   if (num_wgs <= 0 && a->kind == WGM_APP_PANNOTIA_SSSP) {
     const long long sms = a->rt->prop.multiProcessorCount;

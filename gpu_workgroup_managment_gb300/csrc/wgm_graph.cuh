@@ -2310,6 +2310,7 @@ struct wgm_rank_rows {
   int part_edges;
   const int *part_row; /* [parts] rank of a part's row */
   const int *row_part; /* [wide+1] first part of a row */
+  int short_rows;      /* few edges a row on average (wgm_rank_pull) */
   int bin_row[WGM_RANK_BINS + 1];  /* first rank of each bin, then `rows` */
   int bin_task[WGM_RANK_BINS + 1]; /* first warp task of each bin, then their count */
 };
@@ -2420,55 +2421,55 @@ __device__ __forceinline__ void wgm_rank_pull(const wgm_rank_rows &R, const wgm_
           n = skip ? 0 : __ldg(&R.prow[k + 1]) - r0;
         }
       };
-      /* Where passes leave rows out, most of a task's instructions can be for
-       * nothing: those of rows that are all left out, of slots past four edges a
-       * lane where no row has them (more than one lane a row: always more than
-       * four each), of the look ahead past the last task.  They are not run
-       * then: Pannotia SSSP on a 512 x 512 grid 9.5 -> 7.6 ms.  PageRank takes
-       * every row, and its large graphs were 0.7 % slower for it. */
-      auto some = [&](int n, int g, bool &more) {
-        more = !op.SKIPS || g > 1 || __any_sync(WGM_FULL, n > 4);
-        return !op.SKIPS || __any_sync(WGM_FULL, n > 0);
-      };
-      int k0, g0, r0, n0, k1 = 0, g1 = 1, r1 = 0, n1 = 0, u[8], w[8];
-      bool live0, more0;
-      locate(x0, k0, g0, r0, n0);
-      if (!op.SKIPS || x0 + 1 < x1) locate(x0 + 1, k1, g1, r1, n1);
-      live0 = some(n0, g0, more0);
-      if (live0) columns(r0, n0, lane & (g0 - 1), g0, more0, u, w);
-      for (int x = x0; x < x1; x++) {
-        T v[8];
-        if (live0) {
-#pragma unroll
-          for (int q = 0; q < 4; q++) v[q] = op.edge(u[q], w[q]);
-          if (more0) {
-#pragma unroll
-            for (int q = 4; q < 8; q++) v[q] = op.edge(u[q], w[q]);
-          }
-        }
-        bool live1 = false, more1 = false;
-        int k2 = 0, g2 = 1, r2 = 0, n2 = 0;
-        if (!op.SKIPS || x + 1 < x1) {
-          live1 = some(n1, g1, more1);
-          if (live1) columns(r1, n1, lane & (g1 - 1), g1, more1, u, w);
-          if (!op.SKIPS || x + 2 < x1) locate(x + 2, k2, g2, r2, n2);
-        }
-        if (live0) {
+      /* Where passes leave rows out and rows are short, a task is mostly
+       * instructions for nothing: of rows that are all left out, of slots past
+       * four edges a lane where no row has them (more than one lane a row:
+       * always more than four each), of the look ahead below.  One task after
+       * the other then, without them: Pannotia SSSP on a 512 x 512 grid 9.5 ->
+       * 6.9 ms, RMAT of 800,000 vertices and factor 4 0.525 -> 0.455; of 900,000
+       * and factor 14, 0.99 in the pipeline and 1.06 with these tests in it. */
+      if (op.SKIPS && R.short_rows) {
+        for (int x = x0; x < x1; x++) {
+          int k0, g0, r0, n0, u[8], w[8];
+          locate(x, k0, g0, r0, n0);
+          if (!__any_sync(WGM_FULL, n0 > 0)) continue;
+          const bool more = g0 > 1 || __any_sync(WGM_FULL, n0 > 4);
+          columns(r0, n0, lane & (g0 - 1), g0, more, u, w);
           T sum = op.none();
 #pragma unroll
-          for (int q = 0; q < 4; q++) sum = op.join(sum, v[q]);
-          if (more0) {
+          for (int q = 0; q < 4; q++) sum = op.join(sum, op.edge(u[q], w[q]));
+          if (more) {
 #pragma unroll
-            for (int q = 4; q < 8; q++) sum = op.join(sum, v[q]);
+            for (int q = 4; q < 8; q++) sum = op.join(sum, op.edge(u[q], w[q]));
           }
           sum = reduce(sum, g0);
           if (n0 > 0 && (lane & (g0 - 1)) == 0) op.row(k0, n0, sum);
         }
+        unit = next;
+        continue;
+      }
+      /* rows of at most 8 edges a lane, in a pipeline over the tasks: the row
+       * bounds of task x + 2 and the columns of task x + 1 are read beside
+       * the terms of task x */
+      int k0, g0, r0, n0, k1, g1, r1, n1, u[8], w[8];
+      locate(x0, k0, g0, r0, n0);
+      locate(x0 + 1, k1, g1, r1, n1);
+      columns(r0, n0, lane & (g0 - 1), g0, true, u, w);
+      for (int x = x0; x < x1; x++) {
+        T v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[q] = op.edge(u[q], w[q]);
+        columns(r1, n1, lane & (g1 - 1), g1, true, u, w);
+        int k2, g2, r2, n2;
+        locate(x + 2, k2, g2, r2, n2);
+        T sum = op.none();
+#pragma unroll
+        for (int q = 0; q < 8; q++) sum = op.join(sum, v[q]);
+        sum = reduce(sum, g0);
+        if (n0 > 0 && (lane & (g0 - 1)) == 0) op.row(k0, n0, sum);
         k0 = k1;
         g0 = g1;
         n0 = n1;
-        live0 = live1;
-        more0 = more1;
         k1 = k2;
         g1 = g2;
         r1 = r2;
